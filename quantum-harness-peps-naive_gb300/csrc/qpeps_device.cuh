@@ -285,7 +285,38 @@ enum ErrorBits : u32 {
   kErrOverflow = 2u,    // a bounded structure overflowed its capacity
   kErrWaitLimit = 4u,   // a bounded spin-wait gave up
   kErrBounds = 8u,      // an index fell outside its buffer; the access was skipped
+  kErrSkipped = 16u,    // queued step: an earlier step of the chain failed
+  kErrCapacity = 32u,   // queued step: its terms do not fit the buffers
 };
+
+#if defined(__CUDACC__)
+__device__ __forceinline__ u64 global_ns() {
+  u64 t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// A step's input entries and partition count (StepSource); false when a queued
+// step must not run. `cap`: entries the boundary holds. One answer for the
+// whole grid: it depends only on the finished step before.
+template <typename Source, typename Scalars>
+__device__ __forceinline__ bool step_sizes(const Source& q, Scalars* sc, u64 cap, u64& n_in, u32& parts) {
+  if (!q.prev) return true;
+  if (q.prev->error) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->error, (u32)kErrSkipped);
+    return false;
+  }
+  const u64 terms = q.prev->next_terms;
+  const u64 p = (u64)((double)terms / q.mean) + 1;
+  if (p > q.parts_cap || terms > cap) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->error, (u32)kErrCapacity);
+    return false;
+  }
+  n_in = terms ? q.prev->out_count : 0;
+  parts = (u32)p;
+  return true;
+}
+#endif
 
 // Insert one contribution into the global table with linear probing.
 // Returns false (and sets kErrProbeLimit) if `max_probe` slots were visited.

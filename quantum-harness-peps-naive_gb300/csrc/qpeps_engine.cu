@@ -302,6 +302,9 @@ struct Ctx {
   } tune;
   DevBuf tail;                   // TailControl + overflow list
   DevBuf plan;                   // class-grouped partitions: histogram, bucket table, scan partials
+  DevBuf queue;                  // queued steps: their scalars
+  StepScalars* h_queue = nullptr;  // pinned: the scalars as uploaded, then as read back
+  size_t h_queue_steps = 0;
   uint64_t pool_gen = 0;         // bumped whenever a pool buffer is allocated or freed
   GraphRecorder* rec = nullptr;  // row steps of the running contraction (use_graph)
   GraphPlan* graph = nullptr;    // captured contraction (use_graph)
@@ -346,6 +349,8 @@ static void ctx_free(Ctx* ctx) {
   buf_release(*ctx, ctx->table);
   buf_release(*ctx, ctx->tail);
   buf_release(*ctx, ctx->plan);
+  buf_release(*ctx, ctx->queue);
+  if (ctx->h_queue) cudaFreeHost(ctx->h_queue);
   if (ctx->d_sc) cudaFree(ctx->d_sc);
   if (ctx->h_sc) cudaFreeHost(ctx->h_sc);
   for (auto& e : ctx->ev)
@@ -418,6 +423,7 @@ struct Plan {
   size_t budget;
   int threads;
   unsigned tail_row;  // rows >= tail_row go to the slice-tail kernel (n = none)
+  double batch_states = 0;  // expected largest boundary of one device batch (0: unknown)
   bool w64 = false;   // residue planes 0/1 hold the low/high words of exact weights (partitioned row merge)
   int Rc = 0;         // residues of the CRT bookkeeping (= R except with w64, where R = 2 planes)
 };
@@ -972,6 +978,214 @@ static void run_tail(Ctx& ctx, const Plan& p, DevFrontier& f, unsigned row0, std
   f.count = 0;
 }
 
+// ---- queued rows ------------------------------------------------------------
+//
+// A small row's kernels take a few microseconds, the host's wait for its sizes
+// several times that. While a boundary is expected to stay within kQueueTerms
+// successor terms, its rows are queued as one chain: each row's kernels read
+// the entry and term counts the row before left on the device (StepSource),
+// the merges clear the partition cursors they read, and the host waits once
+// for all of them. A row that does not fit the chain's buffers stops it with
+// its input intact, and the host goes on from that row as before.
+// Above kQueueTerms a row runs for 0.1 ms and more, and its exact sizes save
+// more memory than the wait costs.
+constexpr u64 kQueueTerms = 4u << 20;
+
+// Scalars of `steps` queued steps and of the state before them ([0], which the
+// caller fills), pinned and on the device.
+static StepScalars* queue_scalars(Ctx& ctx, const Plan& p, size_t steps) {
+  const size_t n = steps + 1;
+  if (ctx.h_queue_steps < n) {
+    if (ctx.h_queue) cudaFreeHost(ctx.h_queue);
+    ctx.h_queue = nullptr;
+    ctx.h_queue_steps = 0;
+    cuda_check(cudaMallocHost(&ctx.h_queue, n * sizeof(StepScalars)), "pinned step scalars");
+    ctx.h_queue_steps = n;
+  }
+  buf_reserve(ctx, ctx.queue, n * sizeof(StepScalars), p.budget, "queued step scalars");
+  std::memset(ctx.h_queue, 0, n * sizeof(StepScalars));
+  return static_cast<StepScalars*>(ctx.queue.ptr);
+}
+
+// Device times of a finished chain's kernels from their start stamps; `total`
+// (ms, CUDA events) bounds the last one.
+struct QueueTimes {
+  std::vector<double> scatter, merge;  // ms per step
+};
+static QueueTimes queue_times(const StepScalars* h, size_t steps, double total) {
+  QueueTimes t;
+  double sum = 0;
+  for (size_t i = 1; i <= steps; ++i) {
+    const StepScalars& a = h[i];
+    const bool more = i < steps && h[i + 1].t_scatter > a.t_merge;
+    t.scatter.push_back(a.t_merge > a.t_scatter ? (double)(a.t_merge - a.t_scatter) * 1e-6 : 0.0);
+    t.merge.push_back(more ? (double)(h[i + 1].t_scatter - a.t_merge) * 1e-6 : 0.0);
+    sum += t.scatter.back() + t.merge.back();
+  }
+  if (steps) t.merge.back() += std::max(0.0, total - sum);
+  return t;
+}
+
+// Rows [row, stop) of the live boundary as a chain; returns how many were
+// contracted (0: none, the boundary and the metrics are unchanged).
+static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigned row, unsigned stop, u64& known_terms,
+                                std::vector<RowAcc>& rows, RunStats& rs) {
+  const bool wkeys = p.key_bits == 128;
+  const u32 kind = ctx.tune.scatter_kind;
+  if (p.grain != QPEPS_GRAIN_ROW || p.merge != QPEPS_MERGE_PARTITION || p.batch_states <= 0 || f.count == 0 ||
+      row >= stop || ctx.tune.merge_kind != 1)
+    return 0;
+  if (!wkeys && ((kind != 0 && kind != 1 && kind != 4) || (ctx.tune.wide_merge & 1u))) return 0;
+  const u64 most = (u64)std::min((double)kQueueTerms, std::max(65536.0, 1.6 * p.batch_states));  // terms of a row
+  if (f.count > most || (known_terms != kTermsUnknown && known_terms > most)) return 0;
+  // Rows expected to stay below that: a row of n columns with r queens on the
+  // board leaves about n - 2.2 r free ones (fewer, and no more growth, from
+  // the middle of the board on).
+  unsigned count = 0;
+  double expect = known_terms != kTermsUnknown ? (double)known_terms
+                                               : (double)f.count * std::max(1.0, (double)p.n - 2.2 * row);
+  while (row + count < stop && (1.6 * p.batch_states <= (double)most || 2 * row > p.n || expect <= (double)most)) {
+    ++count;
+    expect *= std::max(1.5, (double)p.n - 2.2 * (row + count));
+  }
+  if (count < 2) return 0;
+  const size_t eb = entry_bytes(p);
+  const u32 pcap = wkeys ? wide_key_partition_capacity() : partition_capacity(0);
+  const double mean = ctx.partition_fill * pcap;
+  const u32 parts_cap = (u32)((double)most / mean) + 1;
+  const u32 cstride = (parts_cap <= ctx.tune.spread_cursors_below) ? 8u : 1u;
+  const size_t region_bytes = (size_t)parts_cap * pcap * cand_bytes(p);
+  const size_t cursor_bytes = (size_t)parts_cap * 4 * cstride;
+  const size_t table_bytes = region_bytes + (cursor_bytes + 255) / 256 * 256;
+  if (std::max<u64>(f.cap, most) * eb + table_bytes + (1u << 20) > p.budget) return 0;
+  if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
+  if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes)) return 0;
+  if (ctx.pool_bytes - ctx.table.bytes + table_bytes > p.budget) return 0;
+  buf_reserve(ctx, ctx.table, table_bytes, p.budget, "partition regions");
+  StepScalars* d = queue_scalars(ctx, p, count);
+  StepScalars* h = ctx.h_queue;
+  const auto t0 = std::chrono::steady_clock::now();
+  h[0].out_count = f.count;
+  if (known_terms != kTermsUnknown) h[0].next_terms = known_terms;
+  void* regions = ctx.table.ptr;
+  u32* cursors = reinterpret_cast<u32*>(static_cast<char*>(ctx.table.ptr) + region_bytes);
+  const FrontierView view = view_of(p, ctx.front[0], f.cap);
+  PartitionCfg pc{p.R, ctx.sms, parts_cap, pcap, p.R == 1 ? 3 : p.R == 2 ? 2 : 1, cstride, ctx.tune.parents_per_lane,
+                  0, kind, ctx.tune.merge_kind,
+                  p.w64 ? 2u : (ctx.tune.fold_weights && p.R == 2 && p.free_rows <= 20) ? 1u : 0u};
+  pc.merge_regs = ctx.tune.merge_compact;
+  pc.scatter_block = ctx.tune.scatter_block;
+  pc.key_bits = (uint32_t)p.key_bits;
+  cuda_check(cudaMemcpyAsync(d, h, (count + 1) * sizeof(StepScalars), cudaMemcpyHostToDevice, ctx.stream),
+             "queued step scalars");
+  cuda_check(cudaMemsetAsync(cursors, 0, cursor_bytes, ctx.stream), "clear partition cursors");
+  u64 launches = 0;
+  if (known_terms == kTermsUnknown) {
+    cuda_check(launch_row_count(LaunchCfg{p.key_bits, p.R, p.threads, ctx.sms}, view, f.count, p.n, d, ctx.stream),
+               "row count kernel");
+    launches += 1;
+  }
+  cuda_check(cudaEventRecord(ctx.ev[0], ctx.stream), "event");
+  // Grid bounds: a row's entries are at most the terms of the row before.
+  u64 entries = f.count;
+  double terms = known_terms != kTermsUnknown ? (double)known_terms : (double)f.count * p.n;
+  for (unsigned i = 0; i < count; ++i) {
+    const double fits = std::min((double)most, terms);
+    pc.queued = StepSource{d + i, mean, parts_cap};
+    pc.parts = std::min<u32>(parts_cap, (u32)(fits / mean) + 1);
+    cuda_check(launch_partition_scatter(pc, view, entries, p.n, regions, cursors, d + i + 1, ctx.stream),
+               "partition scatter kernel");
+    cuda_check(launch_partition_merge(pc, regions, cursors, view, p.n, row + i + 1 < p.n, d + i + 1, ctx.stream),
+               "partition merge kernel");
+    launches += 2;
+    entries = (u64)fits;
+    terms = fits * (p.n - (row + i + 1));
+  }
+  cuda_check(cudaEventRecord(ctx.ev[1], ctx.stream), "event");
+  cuda_check(cudaMemcpyAsync(h, d, (count + 1) * sizeof(StepScalars), cudaMemcpyDeviceToHost, ctx.stream),
+             "read step scalars");
+  cuda_check(cudaStreamSynchronize(ctx.stream), "queued rows");
+  ctx.h2d_bytes += (count + 1) * sizeof(StepScalars);
+  ctx.d2h_bytes += (count + 1) * sizeof(StepScalars);
+  rs.launches += launches;
+  float ms = 0;
+  cudaEventElapsedTime(&ms, ctx.ev[0], ctx.ev[1]);
+  rs.device_ms += ms;
+  unsigned done = 0;
+  while (done < count && !h[done + 1].error) ++done;
+  if (done < count && (h[done + 1].error & kErrBounds))
+    fail(QPEPS_ERR_CUDA, row_msg("a kernel's bounds check failed (access skipped) at row", row + done + 1));
+  const QueueTimes times = queue_times(h, done, ms);
+  const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+  for (unsigned i = 0; i < done; ++i) {
+    const StepScalars& r = h[i + 1];
+    const u64 in = i ? h[i].out_count : f.count, tm = h[i].next_terms;
+    const bool last = row + i + 1 == p.n;
+    if (p.w64) {
+      // The certificate of the row, as before a row that runs by itself.
+      const u128 bound = f.weight_bound * (u128)(p.n - (row + i));
+      if (bound >> 63) fail(QPEPS_ERR_OVERFLOW, row_msg("exact 64-bit weights are not certified at row", row + i + 1));
+      f.weight_bound = r.weight_sum[0];
+    }
+    RowAcc& acc = rows[row + i];
+    acc.used = true;
+    acc.device_row = true;
+    acc.input_states += in;
+    acc.candidates += (u128)in * p.n;
+    acc.matched += tm;
+    acc.completed += tm;
+    acc.output_states += r.out_count;
+    for (int q = 0; q < p.Rc; ++q) {
+      acc.weight_res[q] = (acc.weight_res[q] + r.weight_sum[p.w64 ? 0 : q] % kPrimes[q]) % kPrimes[q];
+      if (last) rs.final_res[q] = (rs.final_res[q] + r.final_sum[p.w64 ? 0 : q] % kPrimes[q]) % kPrimes[q];
+    }
+    acc.elapsed += ms > 0 ? wall * (times.scatter[i] + times.merge[i]) / ms : 0.0;
+    rs.peak_states = std::max<u64>(rs.peak_states, r.out_count);
+    if (tm) {
+      rs.scatter_ms += times.scatter[i];
+      rs.merge_ms += times.merge[i];
+      rs.merge_launches += 1;
+      rs.merge_bytes += (in + r.out_count) * eb;
+      rs.entries_in += in;
+      rs.entries_out += r.out_count;
+      rs.candidates += tm;
+    }
+    if (ctx.rec) {
+      // What the row would have recorded by itself.
+      GraphStepRec g;
+      if (tm) {
+        g.pc = pc;
+        g.pc.queued = StepSource{};
+        g.pc.parts = (u32)((double)tm / mean) + 1;
+        g.pc.cursor_stride = (g.pc.parts <= ctx.tune.spread_cursors_below) ? 8u : 1u;
+        g.n_in = in;
+        g.terms = tm;
+        g.out = r.out_count;
+        g.need_cap = last ? in : std::max(in, tm);
+        g.region_bytes = (size_t)g.pc.parts * pcap * cand_bytes(p);
+        g.table_bytes = g.region_bytes + ((size_t)g.pc.parts * 4 * g.pc.cursor_stride + 255) / 256 * 256;
+        g.final_step = last;
+        for (int q = 0; q < p.R; ++q) {
+          g.weight_sum[q] = r.weight_sum[q];
+          g.final_sum[q] = r.final_sum[q];
+        }
+      }
+      if (ctx.rec->chunks.empty())
+        ctx.rec->ok = false;
+      else
+        ctx.rec->chunks.back().steps.push_back(g);
+    }
+  }
+  if (done) {
+    const bool ended = row + done == p.n;
+    f.count = ended ? 0 : h[done].out_count;
+    known_terms = h[done].next_terms;
+  } else if (known_terms == kTermsUnknown) {
+    known_terms = h[0].next_terms;
+  }
+  return done;
+}
+
 // Contract every pending chunk to the last row. Each chunk is one merged
 // device boundary; under memory pressure a boundary is halved and the upper
 // half parked on the host (exact: the contraction is linear in the boundary).
@@ -993,6 +1207,10 @@ static void run_chunks(Ctx& ctx, const Plan& p, std::vector<HostChunk> pending, 
     u64 known_terms = kTermsUnknown;  // successor count of the live boundary, when a merge counted it
     const unsigned stop = hc.no_tail ? p.n : std::max(p.tail_row, hc.row);
     for (unsigned row = hc.row; row < stop; ++row) {
+      if (const unsigned queued = run_queued_rows(ctx, p, f, row, stop, known_terms, rows, rs)) {
+        row += queued - 1;
+        continue;
+      }
       const auto t0 = std::chrono::steady_clock::now();
       const bool last_row = row + 1 == p.n;
       RowAcc& acc = rows[row];
@@ -1343,6 +1561,80 @@ static u64 explicit_partition_step(Ctx& ctx, const Plan& p, DevFrontier& f, cons
   }
 }
 
+// Site steps [0, count) of the explicit-C frontier as a chain (run_queued_rows
+// above has the idea), from the seed boundary. Returns the steps contracted:
+// count, or the first one that did not fit the chain's buffers (or whose
+// scalars the caller stops at); their scalars are in ctx.h_queue[1 ..].
+static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const std::vector<FrontierStepDev>& steps,
+                               const FrontierStepDev* d_steps, const std::vector<size_t>& open_after, size_t count,
+                               ExplicitRun& out) {
+  // Largest boundaries: 1.3 M entries at N = 12 (diamond), times about 5.8 per
+  // size; at most two matches an entry.
+  const double states = 1.4e6 * std::pow(5.8, (double)p.n - 12.0);
+  const u64 most = (u64)std::min((double)kQueueTerms, std::max(65536.0, 1.8 * states));
+  const u32 pcap = wide_key_partition_capacity();
+  const double mean = ctx.partition_fill * pcap;
+  const u32 parts_cap = (u32)((double)most / mean) + 1;
+  const u32 cstride = (parts_cap <= ctx.tune.spread_cursors_below) ? 8u : 1u;
+  const size_t region_bytes = (size_t)parts_cap * pcap * cand_bytes(p);
+  const size_t cursor_bytes = (size_t)parts_cap * 4 * cstride;
+  const size_t table_bytes = region_bytes + (cursor_bytes + 255) / 256 * 256;
+  const size_t eb = entry_bytes(p);
+  if (count < 2 || f.count > most || std::max<u64>(f.cap, most) * eb + table_bytes + (1u << 20) > p.budget) return 0;
+  if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
+  if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes)) return 0;
+  if (ctx.pool_bytes - ctx.table.bytes + table_bytes > p.budget) return 0;
+  buf_reserve(ctx, ctx.table, table_bytes, p.budget, "partition regions");
+  StepScalars* d = queue_scalars(ctx, p, count);
+  StepScalars* h = ctx.h_queue;
+  h[0].out_count = f.count;
+  void* regions = ctx.table.ptr;
+  u32* cursors = reinterpret_cast<u32*>(static_cast<char*>(ctx.table.ptr) + region_bytes);
+  const FrontierView view = view_of(p, ctx.front[0], f.cap);
+  PartitionCfg pc{};
+  pc.residues = p.R;
+  pc.sms = ctx.sms;
+  pc.cap = pcap;
+  pc.merge_blocks_per_sm = 2;
+  pc.cursor_stride = cstride;
+  pc.key_bits = 128;
+  cuda_check(cudaMemcpyAsync(d, h, (count + 1) * sizeof(StepScalars), cudaMemcpyHostToDevice, ctx.stream),
+             "queued step scalars");
+  cuda_check(cudaMemsetAsync(cursors, 0, cursor_bytes, ctx.stream), "clear partition cursors");
+  cuda_check(cudaEventRecord(ctx.ev[0], ctx.stream), "event");
+  cuda_check(launch_frontier_count(view, f.count, steps[0], ctx.sms, d, ctx.stream), "frontier count kernel");
+  u64 entries = f.count;
+  for (size_t i = 0; i < count; ++i) {
+    const u64 fits = std::min(most, 2 * entries);  // at most two matches an entry
+    pc.queued = StepSource{d + i, mean, parts_cap};
+    pc.parts = std::min<u32>(parts_cap, (u32)((double)fits / mean) + 1);
+    // The merge counts the next step's matches, for the chain or the step that
+    // follows it.
+    const bool next = i + 1 < steps.size() && open_after[i + 1] < 128;
+    cuda_check(launch_frontier_partition_scatter(pc, view, entries, steps[i], regions, cursors, d + i + 1, ctx.stream),
+               "frontier scatter kernel");
+    cuda_check(launch_wide_partition_merge(pc, regions, cursors, view, 0, true, d + i + 1, ctx.stream,
+                                           next ? d_steps + i + 1 : nullptr),
+               "frontier merge kernel");
+    entries = fits;
+  }
+  cuda_check(cudaEventRecord(ctx.ev[1], ctx.stream), "event");
+  cuda_check(cudaMemcpyAsync(h, d, (count + 1) * sizeof(StepScalars), cudaMemcpyDeviceToHost, ctx.stream),
+             "read step scalars");
+  cuda_check(cudaStreamSynchronize(ctx.stream), "queued sites");
+  ctx.h2d_bytes += (count + 1) * sizeof(StepScalars);
+  ctx.d2h_bytes += (count + 1) * sizeof(StepScalars);
+  out.launches += 1 + 2 * count;
+  float ms = 0;
+  cudaEventElapsedTime(&ms, ctx.ev[0], ctx.ev[1]);
+  out.device_ms += ms;
+  size_t done = 0;
+  while (done < count && !h[done + 1].error) ++done;
+  if (done < count && (h[done + 1].error & kErrBounds))
+    fail(QPEPS_ERR_CUDA, "explicit-C frontier: a kernel's bounds check failed (access skipped)");
+  return done;
+}
+
 static void explicit_frontier(Ctx& ctx, unsigned n, unsigned order, u64 support_limit, ExplicitRun& out) {
   const auto t0 = std::chrono::steady_clock::now();
   if (n > 21) fail(QPEPS_ERR_RANGE, "explicit-C frontier key supports N <= 21");
@@ -1504,7 +1796,32 @@ static void explicit_frontier(Ctx& ctx, unsigned n, unsigned order, u64 support_
   // Pass 2: the device steps.
   u64 weight_res[kMaxResidues] = {0, 0, 0, 0};
   u64 known_terms = kTermsUnknown;
-  for (size_t step = 0; step < total; ++step) {
+  auto merged_step = [&](size_t step, const StepScalars& sc) {  // false: the support limit stops here
+    const u64 merged = sc.out_count;
+    out.peak_open_bonds = std::max<u64>(out.peak_open_bonds, open_after[step]);
+    if (merged > support_limit) {
+      out.peak_states = std::max<u64>(out.peak_states, support_limit + 1);
+      out.contracted_sites = step;
+      out.elapsed = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+      return false;
+    }
+    f.count = merged;
+    for (int r = 0; r < p.R; ++r) weight_res[r] = sc.weight_sum[r] % kPrimes[r];
+    out.peak_states = std::max<u64>(out.peak_states, merged);
+    return true;
+  };
+  size_t chained = 0;  // leading steps that can be queued as a chain
+  if (partitioned && d_steps)
+    while (chained < total && chained != fail_step && open_after[chained] < 128) ++chained;
+  chained = chained ? run_queued_sites(ctx, p, f, steps, d_steps, open_after, chained, out) : 0;
+  for (size_t step = 0; step < chained; ++step) {
+    const StepScalars& sc = ctx.h_queue[step + 1];
+    out.examined += (u128)f.count * 17;
+    out.accepted += ctx.h_queue[step].next_terms;
+    if (!merged_step(step, sc)) return;
+    known_terms = sc.next_terms_ok ? sc.next_terms : kTermsUnknown;
+  }
+  for (size_t step = chained; step < total; ++step) {
     if (step == fail_step) fail(fail_code, fail_msg);
     const FrontierStepDev& st = steps[step];
     const size_t next_open = open_after[step];
@@ -1514,18 +1831,7 @@ static void explicit_frontier(Ctx& ctx, unsigned n, unsigned order, u64 support_
       const FrontierStepDev* next_dev = (d_steps && next_partitioned) ? d_steps + step + 1 : nullptr;
       const u64 terms = explicit_partition_step(ctx, p, f, st, next_dev, known_terms, out);
       out.accepted += terms;
-      const u64 merged = ctx.h_sc->out_count;
-      if (merged > support_limit) {
-        out.peak_states = std::max<u64>(out.peak_states, support_limit + 1);
-        out.peak_open_bonds = std::max<u64>(out.peak_open_bonds, next_open);
-        out.contracted_sites = step;
-        out.elapsed = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-        return;
-      }
-      f.count = merged;
-      for (int r = 0; r < p.R; ++r) weight_res[r] = ctx.h_sc->weight_sum[r] % kPrimes[r];
-      out.peak_states = std::max<u64>(out.peak_states, merged);
-      out.peak_open_bonds = std::max<u64>(out.peak_open_bonds, next_open);
+      if (!merged_step(step, *ctx.h_sc)) return;
       continue;
     }
     known_terms = kTermsUnknown;
@@ -1554,18 +1860,7 @@ static void explicit_frontier(Ctx& ctx, unsigned n, unsigned order, u64 support_
     cudaEventElapsedTime(&ms, ctx.ev[0], ctx.ev[1]);
     out.device_ms += ms;
     out.accepted += ctx.h_sc->terms;
-    const u64 merged = ctx.h_sc->out_count;
-    if (merged > support_limit) {
-      out.peak_states = std::max<u64>(out.peak_states, support_limit + 1);
-      out.peak_open_bonds = std::max<u64>(out.peak_open_bonds, next_open);
-      out.contracted_sites = step;
-      out.elapsed = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-      return;
-    }
-    f.count = merged;
-    for (int r = 0; r < p.R; ++r) weight_res[r] = ctx.h_sc->weight_sum[r] % kPrimes[r];
-    out.peak_states = std::max<u64>(out.peak_states, merged);
-    out.peak_open_bonds = std::max<u64>(out.peak_open_bonds, next_open);
+    if (!merged_step(step, *ctx.h_sc)) return;
   }
   if (!ends_closed) fail(QPEPS_ERR_INVALID, "explicit-C contraction ended with uncontracted virtual bonds");
   // No bond is open: the boundary is the single key 0 (or empty) and its
@@ -2047,6 +2342,9 @@ static void contract_impl(Ctx& ctx, unsigned n, const qpeps_options& o, const ui
     out.peak_states = std::max<u64>(out.peak_states, items.size());
     ++row0;
   }
+  // (Known for a whole board with the orbits, about twice that without them,
+  // estimated below a prefix.)
+  out.plan.batch_states = serve_estimate(n, k) * (k ? 3.0 : o.symmetry ? 1.0 : 2.0);
   // Predictive slicing: when the merged frontier is estimated not to fit the
   // device budget, contract groups of slices (first-row orbit slices, or
   // deeper prefix slices) one chunk at a time instead of halving a live
@@ -2070,6 +2368,7 @@ static void contract_impl(Ctx& ctx, unsigned n, const qpeps_options& o, const ui
           chunks.push_back(chunk_from_items(out.plan, part, row0));
         }
         out.slice_depth = row0;
+        out.plan.batch_states = std::min(est_item * (double)per_chunk, cap_states);
         run_chunks(ctx, out.plan, std::move(chunks), out.rows, out.rs);
         items.clear();
         break;

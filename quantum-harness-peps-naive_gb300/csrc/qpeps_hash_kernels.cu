@@ -90,7 +90,10 @@ __global__ void __launch_bounds__(BLOCK) row_count_kernel(const void* __restrict
     sw += sitewise_entries(fr, n);
   }
   unsigned long long t = block_sum_u64<BLOCK>(acc);
-  if (threadIdx.x == 0 && t) atomicAdd(&sc->terms, t);
+  if (threadIdx.x == 0 && t) {
+    atomicAdd(&sc->terms, t);
+    atomicAdd(&sc->next_terms, t);  // what a queued first step reads
+  }
   t = block_sum_u64<BLOCK>(sw);
   if (threadIdx.x == 0 && t) atomicAdd(&sc->sitewise_examined, t);
 }

@@ -39,6 +39,17 @@ struct StepScalars {
                                          // row kernel matches over the input (sitewise_entries())
   unsigned long long plan_units;         // class-grouped partitions: units of the step's plan (graph replay)
   unsigned long long next_terms;         // successor terms of the written boundary at the next row
+  unsigned long long t_scatter, t_merge; // queued steps: start of each kernel (global timer, ns)
+};
+
+// Sizes of a queued step: read on the device from the scalars the step before
+// left, so that the host queues a chain of steps without waiting for each. A
+// step that does not fit (or follows one that failed) raises a flag, and its
+// kernels and those after it return at once; its input boundary stands.
+struct StepSource {
+  const StepScalars* prev = nullptr;  // nullptr: the host passes the sizes
+  double mean = 0;                    // planned candidates per partition
+  uint32_t parts_cap = 0;             // partitions the regions hold
 };
 
 struct LaunchCfg {
@@ -128,6 +139,8 @@ struct PartitionCfg {
   uint32_t tl_nb = 0;             // two-level scatter: coarse buckets (0 = one-level scatter)
   uint32_t tl_p2 = 0;             // two-level scatter: partitions per bucket (parts = tl_nb * tl_p2)
   uint64_t tl_bcap = 0;           // two-level scatter: candidate slots per bucket
+  StepSource queued;              // one-level scatters and claim-list merges: sizes come from the device
+                                  // (`parts` and n_in bound the grids); the merge clears the cursors it reads
 };
 
 size_t candidate_bytes(int residues);

@@ -147,7 +147,9 @@ __global__ void __launch_bounds__(BLOCK) partition_scatter_kernel(const u64* __r
                                                                   const u32* __restrict__ res, u64 res_stride,
                                                                   u64 n_in, Layout L, Cand<R>* __restrict__ regions,
                                                                   u32* __restrict__ cursors, u32 cstride, u32 parts,
-                                                                  u32 cap, StepScalars* __restrict__ sc) {
+                                                                  u32 cap, StepScalars* __restrict__ sc, StepSource q) {
+  if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
+  if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   constexpr int WARPS = BLOCK / 32;
   constexpr int PW = 32 * kPPL;  // parents per warp iteration
   __shared__ u64 s_key[WARPS][PW];
@@ -264,7 +266,9 @@ __global__ void __launch_bounds__(BLOCK, (kPPL <= 2 ? 4 : 3)) partition_scatter_
                                                                        Cand<R>* __restrict__ regions,
                                                                        u32* __restrict__ cursors, u32 cstride,
                                                                        u32 parts, u32 cap,
-                                                                       StepScalars* __restrict__ sc) {
+                                                                       StepScalars* __restrict__ sc, StepSource q) {
+  if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
+  if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   constexpr int WARPS = BLOCK / 32;
   constexpr int PW = 32 * kPPL;  // parents per warp iteration
   constexpr int WIN = 32 * kKB;  // candidates per window
@@ -370,7 +374,9 @@ __global__ void __launch_bounds__(BLOCK, (kPPL <= 2 ? 4 : 3)) partition_scatter_
                                                                           Cand<R>* __restrict__ regions,
                                                                           u32* __restrict__ cursors, u32 cstride,
                                                                           u32 parts, u32 cap,
-                                                                          StepScalars* __restrict__ sc) {
+                                                                          StepScalars* __restrict__ sc, StepSource q) {
+  if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
+  if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   constexpr int WARPS = BLOCK / 32;
   constexpr int PW = 32 * kPPL;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -718,7 +724,7 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
                                                                      u32 parts, u64* __restrict__ keys_out,
                                                                      u32* __restrict__ res_out, u64 out_stride,
                                                                      Layout L, int write_out,
-                                                                     StepScalars* __restrict__ sc) {
+                                                                     StepScalars* __restrict__ sc, StepSource q) {
   static_assert((H & (H - 1)) == 0 && H >= 2 * CAP, "merge table size must be a power of two >= 2 CAP");
   constexpr int kLogH = 31 - __builtin_clz(H);
   constexpr int LPT = CAP / BLOCK;  // candidate loads per thread
@@ -739,6 +745,11 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
   if constexpr (Layout::kSlotted)
     for (int i = threadIdx.x; i < (int)kServeMaxSlots * R; i += BLOCK) s_slot_fin[i] = 0ull;
   if (*reinterpret_cast<volatile const u32*>(&sc->error)) return;
+  {
+    u64 n_in = 0;
+    if (!step_sizes(q, sc, out_stride, n_in, parts)) return;
+    if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_merge = global_ns();
+  }
   // write_out: bit 0 writes the merged boundary, bit 1 also counts its
   // successor terms at the next row (left out of CUDA-graph replays, whose
   // sizes are recorded).
@@ -841,6 +852,8 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
     unsigned long long out_base = 0ull;
     if (threadIdx.x == 0) {
       n_unique = s_nused;
+      // (Every thread read this partition's count before the barrier.)
+      if (q.prev) const_cast<u32*>(cursors)[(u64)part * cstride] = 0u;
       if (n_unique) out_base = atomicAdd(&sc->out_count, (unsigned long long)n_unique);
     }
 #pragma unroll
@@ -1343,18 +1356,18 @@ cudaError_t scatter_shape(const PartitionCfg& pc, const FrontierView& in, u64 n_
   if (pc.scatter_kind == 4) {
     partition_scatter_direct_kernel<R, BLOCK, PPL, Layout><<<grid, BLOCK, 0, stream>>>(
         reinterpret_cast<const u64*>(in.keys), in.res, in.cap, n_in, L, reinterpret_cast<Cand<R>*>(regions), cursors,
-        cstride, pc.parts, pc.cap, sc);
+        cstride, pc.parts, pc.cap, sc, pc.queued);
     return cudaGetLastError();
   }
   if (pc.scatter_kind != 0) {  // 2 without a two-level plan, or 3 where it does not apply: the window scatter
     partition_scatter_list_kernel<R, BLOCK, PPL, Layout><<<grid, BLOCK, 0, stream>>>(
         reinterpret_cast<const u64*>(in.keys), in.res, in.cap, n_in, L, reinterpret_cast<Cand<R>*>(regions), cursors,
-        cstride, pc.parts, pc.cap, sc);
+        cstride, pc.parts, pc.cap, sc, pc.queued);
     return cudaGetLastError();
   }
   partition_scatter_kernel<R, BLOCK, PPL, Layout><<<grid, BLOCK, 0, stream>>>(
       reinterpret_cast<const u64*>(in.keys), in.res, in.cap, n_in, L, reinterpret_cast<Cand<R>*>(regions), cursors,
-      cstride, pc.parts, pc.cap, sc);
+      cstride, pc.parts, pc.cap, sc, pc.queued);
   return cudaGetLastError();
 }
 
@@ -1394,19 +1407,26 @@ cudaError_t merge_shape(const PartitionCfg& pc, int blocks_per_sm, const void* r
                                                                   (R == 2 && !Layout::kSlotted) ? 2 : 0>)
                             : (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, R == 2 ? 1 : 0, kRegsOk>
                                     : partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, R == 2 ? 1 : 0>))
-                   : pc.merge_kind == 1 ? (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, 0, kRegsOk>
-                                                : partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout>)
-                                        : partition_merge_kernel<R, BLOCK, H, H / 2, Layout>;
+                   : (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, 0, kRegsOk>
+                           : partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout>);
+  auto scan_kern = partition_merge_kernel<R, BLOCK, H, H / 2, Layout>;
+  const bool scan = pc.merge_kind != 1;
+  if (scan && pc.queued.prev) return cudaErrorInvalidValue;
   const size_t smem = fold ? merge_smem<1, H>() + (size_t)(H / 2) * 4
                            : merge_smem<R, H>() + (pc.merge_kind == 1 ? (size_t)(H / 2) * 4 : 0);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = scan ? cudaFuncSetAttribute(scan_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                       : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const u64 capb = (u64)pc.sms * blocks_per_sm;
   const unsigned grid = (unsigned)std::max<u64>(1, std::min<u64>(pc.parts, capb));
-  kern<<<grid, BLOCK, smem, stream>>>(reinterpret_cast<const Cand<R>*>(regions), cursors,
-                                      pc.cursor_stride ? pc.cursor_stride : 1, pc.parts,
-                                      reinterpret_cast<u64*>(out.keys), out.res, out.cap, L,
-                                      (write_out ? 1 : 0) | (pc.count_next ? 2 : 0), sc);
+  const u32 cstride = pc.cursor_stride ? pc.cursor_stride : 1;
+  const int write = (write_out ? 1 : 0) | (pc.count_next ? 2 : 0);
+  if (scan)
+    scan_kern<<<grid, BLOCK, smem, stream>>>(reinterpret_cast<const Cand<R>*>(regions), cursors, cstride, pc.parts,
+                                             reinterpret_cast<u64*>(out.keys), out.res, out.cap, L, write, sc);
+  else
+    kern<<<grid, BLOCK, smem, stream>>>(reinterpret_cast<const Cand<R>*>(regions), cursors, cstride, pc.parts,
+                                        reinterpret_cast<u64*>(out.keys), out.res, out.cap, L, write, sc, pc.queued);
   return cudaGetLastError();
 }
 

@@ -151,7 +151,9 @@ __global__ void __launch_bounds__(BLOCK) wide_scatter_kernel(const u128* __restr
                                                             u64 res_stride, u64 n_in, unsigned n,
                                                             WCand<R>* __restrict__ regions,
                                                             u32* __restrict__ cursors, u32 cstride, u32 parts,
-                                                            u32 cap, StepScalars* __restrict__ sc) {
+                                                            u32 cap, StepScalars* __restrict__ sc, StepSource q) {
+  if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
+  if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   constexpr int WARPS = BLOCK / 32;
   constexpr int PW = 32 * kWPPL;
   constexpr int WIN = 32 * kWKB;
@@ -262,7 +264,7 @@ __global__ void __launch_bounds__(BLOCK, 2) wide_merge_kernel(const WCand<R>* __
                                                           u128* __restrict__ keys_out, u32* __restrict__ res_out,
                                                           u64 out_stride, unsigned n, int write_out,
                                                           const FrontierStepDev* __restrict__ next_step,
-                                                          StepScalars* __restrict__ sc) {
+                                                          StepScalars* __restrict__ sc, StepSource q) {
   static_assert((H & (H - 1)) == 0 && H >= 2 * CAP && CAP % BLOCK == 0, "merge shape");
   constexpr int kLogH = 31 - __builtin_clz(H);
   constexpr int LPT = CAP / BLOCK;
@@ -278,6 +280,11 @@ __global__ void __launch_bounds__(BLOCK, 2) wide_merge_kernel(const WCand<R>* __
   __shared__ u32 s_next_trans;
   const int lane = threadIdx.x & 31;
   if (*reinterpret_cast<volatile const u32*>(&sc->error)) return;
+  {
+    u64 n_in = 0;
+    if (!step_sizes(q, sc, out_stride, n_in, parts)) return;
+    if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_merge = global_ns();
+  }
   // write_out: bit 0 writes the merged boundary, bit 1 lets the row-key
   // merge count its successor terms at the next row.
   const bool count_next = (write_out & 1) && (kBond ? next_step != nullptr : (n > 0 && (write_out & 2)));
@@ -359,6 +366,8 @@ __global__ void __launch_bounds__(BLOCK, 2) wide_merge_kernel(const WCand<R>* __
     unsigned long long out_base = 0ull;
     if (threadIdx.x == 0) {
       n_unique = s_nused;
+      // (Every thread read this partition's count before the barrier.)
+      if (q.prev) const_cast<u32*>(cursors)[(u64)part * cstride] = 0u;
       if (n_unique) out_base = atomicAdd(&sc->out_count, (unsigned long long)n_unique);
     }
 #pragma unroll
@@ -443,7 +452,10 @@ __global__ void __launch_bounds__(BLOCK) frontier_count_kernel(const u128* __res
     for (u32 t = 0; t < st.n_trans; ++t) acc += (key & st.req_mask[t]) == st.req_value[t];
   }
   const unsigned long long t = wblock_sum<BLOCK>(acc);
-  if (threadIdx.x == 0 && t) atomicAdd(&sc->terms, t);
+  if (threadIdx.x == 0 && t) {
+    atomicAdd(&sc->terms, t);
+    atomicAdd(&sc->next_terms, t);  // what a queued first step reads
+  }
 }
 
 template <int R, int BLOCK>
@@ -452,7 +464,9 @@ __global__ void __launch_bounds__(BLOCK) frontier_scatter_kernel(const u128* __r
                                                                 u64 n_in, const __grid_constant__ FrontierStepDev st,
                                                                 WCand<R>* __restrict__ regions,
                                                                 u32* __restrict__ cursors, u32 cstride, u32 parts,
-                                                                u32 cap, StepScalars* __restrict__ sc) {
+                                                                u32 cap, StepScalars* __restrict__ sc, StepSource q) {
+  if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
+  if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   const u64 policy = wl2_keep_policy();
   bool overflow = false;
   for (u64 i = (u64)blockIdx.x * BLOCK + threadIdx.x; i < n_in; i += (u64)gridDim.x * BLOCK) {
@@ -485,7 +499,7 @@ cudaError_t wide_scatter(const PartitionCfg& pc, const FrontierView& in, u64 n_i
   const unsigned grid = (unsigned)std::max<u64>(1, std::min<u64>(want, (u64)pc.sms * 8));
   wide_scatter_kernel<R, kWScatterBlock><<<grid, kWScatterBlock, 0, stream>>>(
       reinterpret_cast<const u128*>(in.keys), in.res, in.cap, n_in, n, reinterpret_cast<WCand<R>*>(regions), cursors,
-      pc.cursor_stride ? pc.cursor_stride : 1, pc.parts, pc.cap, sc);
+      pc.cursor_stride ? pc.cursor_stride : 1, pc.parts, pc.cap, sc, pc.queued);
   return cudaGetLastError();
 }
 
@@ -502,7 +516,7 @@ cudaError_t wide_merge(const PartitionCfg& pc, const void* regions, const u32* c
   kern<<<grid, kWBlock, smem, stream>>>(reinterpret_cast<const WCand<R>*>(regions), cursors,
                                         pc.cursor_stride ? pc.cursor_stride : 1, pc.parts,
                                         reinterpret_cast<u128*>(out.keys), out.res, out.cap, n,
-                                        (write_out ? 1 : 0) | (pc.count_next ? 2 : 0), next_step, sc);
+                                        (write_out ? 1 : 0) | (pc.count_next ? 2 : 0), next_step, sc, pc.queued);
   return cudaGetLastError();
 }
 
@@ -563,7 +577,8 @@ cudaError_t launch_frontier_partition_scatter(const PartitionCfg& pc, const Fron
 #define QPEPS_FRONTIER_SCATTER(R)                                                                            \
   case R:                                                                                                   \
     frontier_scatter_kernel<R, kWScatterBlock><<<grid, kWScatterBlock, 0, stream>>>(                         \
-        keys, in.res, in.cap, n_in, step, reinterpret_cast<WCand<R>*>(regions), cursors, cs, pc.parts, pc.cap, sc); \
+        keys, in.res, in.cap, n_in, step, reinterpret_cast<WCand<R>*>(regions), cursors, cs, pc.parts, pc.cap, sc,  \
+        pc.queued);                                                                                          \
     break;
     QPEPS_FRONTIER_SCATTER(1)
     QPEPS_FRONTIER_SCATTER(2)
