@@ -296,23 +296,28 @@ __device__ __forceinline__ u64 global_ns() {
   return t;
 }
 
+// Queued kernels overlap: a kernel lets its successor launch at once, and the
+// successor prepares its shared memory before it waits for the kernel's
+// results. Both are no-ops in a launch without the attribute
+// (launch_overlapped in qpeps_internal.h).
+__device__ __forceinline__ void next_kernel_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // A step's input entries and partition count (StepSource); false when a queued
 // step must not run. `cap`: entries the boundary holds. One answer for the
-// whole grid: it depends only on the finished step before.
+// whole grid: it depends only on the finished step before. (The three loads
+// are issued together: a small step's time is its dependent trips to memory.)
 template <typename Source, typename Scalars>
 __device__ __forceinline__ bool step_sizes(const Source& q, Scalars* sc, u64 cap, u64& n_in, u32& parts) {
   if (!q.prev) return true;
-  if (q.prev->error) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->error, (u32)kErrSkipped);
+  const u32 error = q.prev->error;
+  const u64 terms = q.prev->next_terms, entries = q.prev->out_count;
+  const u64 p = q.partitions(terms);
+  if (error || p > q.parts_cap || terms > cap) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->error, (u32)(error ? kErrSkipped : kErrCapacity));
     return false;
   }
-  const u64 terms = q.prev->next_terms;
-  const u64 p = (u64)((double)terms / q.mean) + 1;
-  if (p > q.parts_cap || terms > cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->error, (u32)kErrCapacity);
-    return false;
-  }
-  n_in = terms ? q.prev->out_count : 0;
+  n_in = terms ? entries : 0;
   parts = (u32)p;
   return true;
 }

@@ -1036,7 +1036,10 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
       row >= stop || ctx.tune.merge_kind != 1)
     return 0;
   if (!wkeys && ((kind != 0 && kind != 1 && kind != 4) || (ctx.tune.wide_merge & 1u))) return 0;
-  const u64 most = (u64)std::min((double)kQueueTerms, std::max(65536.0, 1.6 * p.batch_states));  // terms of a row
+  // Terms a row may have, and those it is expected to have at most (the grids
+  // are sized for these; a grid covers any number).
+  const u64 most = (u64)std::min((double)kQueueTerms, std::max(1048576.0, 1.6 * p.batch_states));
+  const double likely = std::min((double)most, std::max(65536.0, 1.6 * p.batch_states));
   if (f.count > most || (known_terms != kTermsUnknown && known_terms > most)) return 0;
   // Rows expected to stay below that: a row of n columns with r queens on the
   // board leaves about n - 2.2 r free ones (fewer, and no more growth, from
@@ -1050,9 +1053,14 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   }
   if (count < 2) return 0;
   const size_t eb = entry_bytes(p);
-  const u32 pcap = wkeys ? wide_key_partition_capacity() : partition_capacity(0);
+  // Small merge CTAs (four an SM, 1024 candidates) where they exist: a chain's
+  // scatter waits for its deepest partition cursor, and half the candidates a
+  // partition halve that.
+  const u32 shape = !wkeys && wide_merge_supported(p.R) ? 2u : 0u;
+  const u32 pcap = wkeys ? wide_key_partition_capacity() : partition_capacity(shape);
   const double mean = ctx.partition_fill * pcap;
-  const u32 parts_cap = (u32)((double)most / mean) + 1;
+  StepSource source{nullptr, mean, 0, (shape == 2 ? 8u : 2u) * (u32)ctx.sms};
+  const u32 parts_cap = source.parts_cap = (u32)source.partitions(most);
   const u32 cstride = (parts_cap <= ctx.tune.spread_cursors_below) ? 8u : 1u;
   const size_t region_bytes = (size_t)parts_cap * pcap * cand_bytes(p);
   const size_t cursor_bytes = (size_t)parts_cap * 4 * cstride;
@@ -1071,7 +1079,7 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   u32* cursors = reinterpret_cast<u32*>(static_cast<char*>(ctx.table.ptr) + region_bytes);
   const FrontierView view = view_of(p, ctx.front[0], f.cap);
   PartitionCfg pc{p.R, ctx.sms, parts_cap, pcap, p.R == 1 ? 3 : p.R == 2 ? 2 : 1, cstride, ctx.tune.parents_per_lane,
-                  0, kind, ctx.tune.merge_kind,
+                  shape, kind, ctx.tune.merge_kind,
                   p.w64 ? 2u : (ctx.tune.fold_weights && p.R == 2 && p.free_rows <= 20) ? 1u : 0u};
   pc.merge_regs = ctx.tune.merge_compact;
   pc.scatter_block = ctx.tune.scatter_block;
@@ -1090,9 +1098,10 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   u64 entries = f.count;
   double terms = known_terms != kTermsUnknown ? (double)known_terms : (double)f.count * p.n;
   for (unsigned i = 0; i < count; ++i) {
-    const double fits = std::min((double)most, terms);
-    pc.queued = StepSource{d + i, mean, parts_cap};
-    pc.parts = std::min<u32>(parts_cap, (u32)(fits / mean) + 1);
+    const double fits = std::min(likely, terms);
+    pc.queued = source;
+    pc.queued.prev = d + i;
+    pc.parts = (u32)source.partitions((u64)fits);
     cuda_check(launch_partition_scatter(pc, view, entries, p.n, regions, cursors, d + i + 1, ctx.stream),
                "partition scatter kernel");
     cuda_check(launch_partition_merge(pc, regions, cursors, view, p.n, row + i + 1 < p.n, d + i + 1, ctx.stream),
@@ -1156,7 +1165,7 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
       if (tm) {
         g.pc = pc;
         g.pc.queued = StepSource{};
-        g.pc.parts = (u32)((double)tm / mean) + 1;
+        g.pc.parts = (u32)source.partitions(tm);
         g.pc.cursor_stride = (g.pc.parts <= ctx.tune.spread_cursors_below) ? 8u : 1u;
         g.n_in = in;
         g.terms = tm;
@@ -1574,7 +1583,8 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
   const u64 most = (u64)std::min((double)kQueueTerms, std::max(65536.0, 1.8 * states));
   const u32 pcap = wide_key_partition_capacity();
   const double mean = ctx.partition_fill * pcap;
-  const u32 parts_cap = (u32)((double)most / mean) + 1;
+  StepSource source{nullptr, mean, 0, 2 * (u32)ctx.sms};
+  const u32 parts_cap = source.parts_cap = (u32)source.partitions(most);
   const u32 cstride = (parts_cap <= ctx.tune.spread_cursors_below) ? 8u : 1u;
   const size_t region_bytes = (size_t)parts_cap * pcap * cand_bytes(p);
   const size_t cursor_bytes = (size_t)parts_cap * 4 * cstride;
@@ -1606,8 +1616,9 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
   u64 entries = f.count;
   for (size_t i = 0; i < count; ++i) {
     const u64 fits = std::min(most, 2 * entries);  // at most two matches an entry
-    pc.queued = StepSource{d + i, mean, parts_cap};
-    pc.parts = std::min<u32>(parts_cap, (u32)((double)fits / mean) + 1);
+    pc.queued = source;
+    pc.queued.prev = d + i;
+    pc.parts = (u32)source.partitions(fits);
     // The merge counts the next step's matches, for the chain or the step that
     // follows it.
     const bool next = i + 1 < steps.size() && open_after[i + 1] < 128;

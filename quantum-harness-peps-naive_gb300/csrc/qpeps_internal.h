@@ -50,7 +50,36 @@ struct StepSource {
   const StepScalars* prev = nullptr;  // nullptr: the host passes the sizes
   double mean = 0;                    // planned candidates per partition
   uint32_t parts_cap = 0;             // partitions the regions hold
+  uint32_t spread = 1;                // partitions of a small step, one for each merge CTA the device holds
+
+  // Partitions of a step. A small step takes more of them than its candidates
+  // fill: with 60 partitions for 100 K candidates the cursor atomics queue up
+  // 1,600 deep on each cursor, and most merge CTAs idle. At least 64 candidates
+  // each.
+  __host__ __device__ uint64_t partitions(uint64_t terms) const {
+    const uint64_t full = (uint64_t)((double)terms / mean) + 1, wide = terms / 64 + 1;
+    const uint64_t small = wide < spread ? wide : spread;
+    return full > small ? full : small;
+  }
 };
+
+// Launch a kernel of a chain so that it may start while the kernel before it
+// in the stream finishes (it waits for that kernel's results itself).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_overlapped(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem,
+                                     cudaStream_t stream, bool overlapped, Args... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlapped ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
 
 struct LaunchCfg {
   int key_bits;  // 64 or 128

@@ -130,6 +130,29 @@ __device__ __forceinline__ unsigned long long pblock_sum(unsigned long long v) {
   return t;
 }
 
+// Block sums of several values at once, in thread 0.
+template <int BLOCK, int V>
+__device__ __forceinline__ void pblock_sums(unsigned long long (&v)[V]) {
+  constexpr int WARPS = BLOCK / 32;
+  __shared__ unsigned long long s_part[V][WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v[i] += __shfl_xor_sync(kFullMask, v[i], d);
+    if (lane == 0) s_part[i][wid] = v[i];
+  }
+  __syncthreads();
+  if (wid == 0) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      v[i] = lane < WARPS ? s_part[i][lane] : 0ull;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) v[i] += __shfl_xor_sync(kFullMask, v[i], d);
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Scatter. Each warp takes 64 parents per iteration (two per lane; the next
 // iteration's parents are loaded before this iteration's atomics are waited
@@ -139,7 +162,7 @@ __device__ __forceinline__ unsigned long long pblock_sum(unsigned long long v) {
 
 constexpr int kKB = 4;  // successor rounds per atomic batch
 
-// kPPL parents per lane per iteration (2 or 4); partition cursors are
+// kPPL parents per lane per iteration (1, 2 or 4); partition cursors are
 // `cstride` u32 apart (a stride of 8 gives each cursor its own 32-byte sector,
 // spreading a small cursor array over more L2 slices).
 template <int R, int BLOCK, int kPPL, typename Layout>
@@ -148,6 +171,8 @@ __global__ void __launch_bounds__(BLOCK) partition_scatter_kernel(const u64* __r
                                                                   u64 n_in, Layout L, Cand<R>* __restrict__ regions,
                                                                   u32* __restrict__ cursors, u32 cstride, u32 parts,
                                                                   u32 cap, StepScalars* __restrict__ sc, StepSource q) {
+  next_kernel_may_start();
+  wait_for_kernel_before();
   if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
   if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   constexpr int WARPS = BLOCK / 32;
@@ -267,6 +292,8 @@ __global__ void __launch_bounds__(BLOCK, (kPPL <= 2 ? 4 : 3)) partition_scatter_
                                                                        u32* __restrict__ cursors, u32 cstride,
                                                                        u32 parts, u32 cap,
                                                                        StepScalars* __restrict__ sc, StepSource q) {
+  next_kernel_may_start();
+  wait_for_kernel_before();
   if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
   if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   constexpr int WARPS = BLOCK / 32;
@@ -375,6 +402,8 @@ __global__ void __launch_bounds__(BLOCK, (kPPL <= 2 ? 4 : 3)) partition_scatter_
                                                                           u32* __restrict__ cursors, u32 cstride,
                                                                           u32 parts, u32 cap,
                                                                           StepScalars* __restrict__ sc, StepSource q) {
+  next_kernel_may_start();
+  wait_for_kernel_before();
   if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
   if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   constexpr int WARPS = BLOCK / 32;
@@ -744,10 +773,14 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
   const int lane = threadIdx.x & 31;
   if constexpr (Layout::kSlotted)
     for (int i = threadIdx.x; i < (int)kServeMaxSlots * R; i += BLOCK) s_slot_fin[i] = 0ull;
-  if (*reinterpret_cast<volatile const u32*>(&sc->error)) return;
+  next_kernel_may_start();
+  for (int i = threadIdx.x; i < H; i += BLOCK) s_key[i] = kEmpty;
+  if (threadIdx.x == 0) s_nused = 0;
+  wait_for_kernel_before();
+  const u32 failed = *reinterpret_cast<volatile const u32*>(&sc->error);
   {
     u64 n_in = 0;
-    if (!step_sizes(q, sc, out_stride, n_in, parts)) return;
+    if (!step_sizes(q, sc, out_stride, n_in, parts) || failed) return;
     if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_merge = global_ns();
   }
   // write_out: bit 0 writes the merged boundary, bit 1 also counts its
@@ -763,8 +796,6 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
   bool bad = false;  // an output index beyond the boundary buffer (skipped)
 #pragma unroll
   for (int r = 0; r < R; ++r) wsum[r] = fsum[r] = 0;
-  for (int i = threadIdx.x; i < H; i += BLOCK) s_key[i] = kEmpty;
-  if (threadIdx.x == 0) s_nused = 0;
 
   Cand<R> buf[LPT];
   u32 bcnt = 0;
@@ -948,20 +979,30 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
     __syncthreads();
   }
   if (bad) atomicOr(&sc->error, kErrBounds);
+  // All the row's sums in one pass: shuffles, one trip through shared memory,
+  // one atomic a sum. (An exact weight has one sum, in plane 0.)
+  constexpr int SP = kAcc == 2 ? 1 : R;
+  unsigned long long sums[2 * SP + 2];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    unsigned long long t = pblock_sum<BLOCK>(wsum[r]);
-    if (threadIdx.x == 0 && t) atomicAdd(&sc->weight_sum[r], t);
-    t = pblock_sum<BLOCK>(fsum[r]);
-    if (threadIdx.x == 0 && t) atomicAdd(&sc->final_sum[r], t);
+  for (int r = 0; r < SP; ++r) {
+    sums[r] = wsum[r];
+    sums[SP + r] = fsum[r];
   }
-  const unsigned long long t = pblock_sum<BLOCK>(fstates);
-  if (threadIdx.x == 0 && t) atomicAdd(&sc->final_states, t);
-  if constexpr (kCountNext) {
-    if (write_out && count_next) {
-      const unsigned long long nt = pblock_sum<BLOCK>(nterms);
-      if (threadIdx.x == 0 && nt) atomicAdd(&sc->next_terms, nt);
-      if (blockIdx.x == 0 && threadIdx.x == 0) sc->next_terms_ok = 1u;
+  sums[2 * SP] = fstates;
+  sums[2 * SP + 1] = nterms;
+  pblock_sums<BLOCK>(sums);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int r = 0; r < SP; ++r) {
+      if (sums[r]) atomicAdd(&sc->weight_sum[r], sums[r]);
+      if (sums[SP + r]) atomicAdd(&sc->final_sum[r], sums[SP + r]);
+    }
+    if (sums[2 * SP]) atomicAdd(&sc->final_states, sums[2 * SP]);
+    if constexpr (kCountNext) {
+      if (write_out && count_next) {
+        if (sums[2 * SP + 1]) atomicAdd(&sc->next_terms, sums[2 * SP + 1]);
+        if (blockIdx.x == 0) sc->next_terms_ok = 1u;
+      }
     }
   }
   if constexpr (Layout::kSlotted) {
@@ -1359,12 +1400,10 @@ cudaError_t scatter_shape(const PartitionCfg& pc, const FrontierView& in, u64 n_
         cstride, pc.parts, pc.cap, sc, pc.queued);
     return cudaGetLastError();
   }
-  if (pc.scatter_kind != 0) {  // 2 without a two-level plan, or 3 where it does not apply: the window scatter
-    partition_scatter_list_kernel<R, BLOCK, PPL, Layout><<<grid, BLOCK, 0, stream>>>(
-        reinterpret_cast<const u64*>(in.keys), in.res, in.cap, n_in, L, reinterpret_cast<Cand<R>*>(regions), cursors,
-        cstride, pc.parts, pc.cap, sc, pc.queued);
-    return cudaGetLastError();
-  }
+  if (pc.scatter_kind != 0)  // 2 without a two-level plan, or 3 where it does not apply: the window scatter
+    return launch_overlapped(partition_scatter_list_kernel<R, BLOCK, PPL, Layout>, grid, BLOCK, 0, stream,
+                             pc.queued.prev != nullptr, reinterpret_cast<const u64*>(in.keys), in.res, in.cap, n_in, L,
+                             reinterpret_cast<Cand<R>*>(regions), cursors, cstride, pc.parts, pc.cap, sc, pc.queued);
   partition_scatter_kernel<R, BLOCK, PPL, Layout><<<grid, BLOCK, 0, stream>>>(
       reinterpret_cast<const u64*>(in.keys), in.res, in.cap, n_in, L, reinterpret_cast<Cand<R>*>(regions), cursors,
       cstride, pc.parts, pc.cap, sc, pc.queued);
@@ -1386,6 +1425,10 @@ cudaError_t scatter_ppl(const PartitionCfg& pc, const FrontierView& in, u64 n_in
 template <int R, typename Layout>
 cudaError_t scatter_impl(const PartitionCfg& pc, const FrontierView& in, u64 n_in, Layout L, void* regions,
                          u32* cursors, StepScalars* sc, cudaStream_t stream) {
+  // A boundary that leaves the chip short of warps at four parents a lane
+  // (fewer than about 8 blocks an SM) takes one a lane in small blocks.
+  if (!Layout::kSlotted && pc.scatter_kind == 1 && n_in <= (u64)pc.sms * 2048)
+    return scatter_shape<R, 1, 128, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
   if (pc.parents_per_lane == 4) return scatter_ppl<R, 4, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
   return scatter_ppl<R, 2, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
 }
@@ -1425,8 +1468,9 @@ cudaError_t merge_shape(const PartitionCfg& pc, int blocks_per_sm, const void* r
     scan_kern<<<grid, BLOCK, smem, stream>>>(reinterpret_cast<const Cand<R>*>(regions), cursors, cstride, pc.parts,
                                              reinterpret_cast<u64*>(out.keys), out.res, out.cap, L, write, sc);
   else
-    kern<<<grid, BLOCK, smem, stream>>>(reinterpret_cast<const Cand<R>*>(regions), cursors, cstride, pc.parts,
-                                        reinterpret_cast<u64*>(out.keys), out.res, out.cap, L, write, sc, pc.queued);
+    return launch_overlapped(kern, grid, BLOCK, smem, stream, pc.queued.prev != nullptr,
+                             reinterpret_cast<const Cand<R>*>(regions), cursors, cstride, pc.parts,
+                             reinterpret_cast<u64*>(out.keys), out.res, out.cap, L, write, sc, pc.queued);
   return cudaGetLastError();
 }
 

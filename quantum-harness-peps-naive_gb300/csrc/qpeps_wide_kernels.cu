@@ -140,6 +140,29 @@ __device__ __forceinline__ unsigned long long wblock_sum(unsigned long long v) {
   return t;
 }
 
+// Block sums of several values at once, in thread 0.
+template <int BLOCK, int V>
+__device__ __forceinline__ void wblock_sums(unsigned long long (&v)[V]) {
+  constexpr int WARPS = BLOCK / 32;
+  __shared__ unsigned long long s_part[V][WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v[i] += __shfl_xor_sync(kWFull, v[i], d);
+    if (lane == 0) s_part[i][wid] = v[i];
+  }
+  __syncthreads();
+  if (wid == 0) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      v[i] = lane < WARPS ? s_part[i][lane] : 0ull;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) v[i] += __shfl_xor_sync(kWFull, v[i], d);
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Scatter (the window scatter of the u64 path, with 128-bit keys).
 
@@ -152,6 +175,8 @@ __global__ void __launch_bounds__(BLOCK) wide_scatter_kernel(const u128* __restr
                                                             WCand<R>* __restrict__ regions,
                                                             u32* __restrict__ cursors, u32 cstride, u32 parts,
                                                             u32 cap, StepScalars* __restrict__ sc, StepSource q) {
+  next_kernel_may_start();
+  wait_for_kernel_before();
   if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
   if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   constexpr int WARPS = BLOCK / 32;
@@ -279,31 +304,34 @@ __global__ void __launch_bounds__(BLOCK, 2) wide_merge_kernel(const WCand<R>* __
   __shared__ u128 s_req_mask[kBond ? kFrontierMaxTrans : 1], s_req_value[kBond ? kFrontierMaxTrans : 1];
   __shared__ u32 s_next_trans;
   const int lane = threadIdx.x & 31;
-  if (*reinterpret_cast<volatile const u32*>(&sc->error)) return;
-  {
-    u64 n_in = 0;
-    if (!step_sizes(q, sc, out_stride, n_in, parts)) return;
-    if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_merge = global_ns();
-  }
-  // write_out: bit 0 writes the merged boundary, bit 1 lets the row-key
-  // merge count its successor terms at the next row.
-  const bool count_next = (write_out & 1) && (kBond ? next_step != nullptr : (n > 0 && (write_out & 2)));
-  write_out &= 1;
+  next_kernel_may_start();
+  for (int i = threadIdx.x; i < H; i += BLOCK) s_key[i] = kWEmpty;
+  if (threadIdx.x == 0) s_nused = 0;
   if constexpr (kBond) {
+    // (The step list is not written by the chain.)
     if (threadIdx.x == 0) s_next_trans = min(next_step->n_trans, (u32)kFrontierMaxTrans);
     for (int t = threadIdx.x; t < kFrontierMaxTrans; t += BLOCK) {
       s_req_mask[t] = next_step->req_mask[t];
       s_req_value[t] = next_step->req_value[t];
     }
   }
+  wait_for_kernel_before();
+  const u32 failed = *reinterpret_cast<volatile const u32*>(&sc->error);
+  {
+    u64 n_in = 0;
+    if (!step_sizes(q, sc, out_stride, n_in, parts) || failed) return;
+    if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_merge = global_ns();
+  }
+  // write_out: bit 0 writes the merged boundary, bit 1 lets the row-key
+  // merge count its successor terms at the next row.
+  const bool count_next = (write_out & 1) && (kBond ? next_step != nullptr : (n > 0 && (write_out & 2)));
+  write_out &= 1;
   const u64 mask = (n >= 64) ? ~0ull : ((1ull << n) - 1);
   unsigned long long wsum[R], fsum[R], fstates = 0;
   unsigned long long nterms = 0;  // the written boundary's successor terms at the next row (n > 0)
   bool bad = false;
 #pragma unroll
   for (int r = 0; r < R; ++r) wsum[r] = fsum[r] = 0;
-  for (int i = threadIdx.x; i < H; i += BLOCK) s_key[i] = kWEmpty;
-  if (threadIdx.x == 0) s_nused = 0;
 
   WCand<R> buf[LPT];
   u32 bcnt = 0;
@@ -417,19 +445,27 @@ __global__ void __launch_bounds__(BLOCK, 2) wide_merge_kernel(const WCand<R>* __
     __syncthreads();
   }
   if (bad) atomicOr(&sc->error, kErrBounds);
+  // All the step's sums in one pass.
+  unsigned long long sums[2 * R + 2];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    unsigned long long t = wblock_sum<BLOCK>(wsum[r]);
-    if (threadIdx.x == 0 && t) atomicAdd(&sc->weight_sum[r], t);
-    t = wblock_sum<BLOCK>(fsum[r]);
-    if (threadIdx.x == 0 && t) atomicAdd(&sc->final_sum[r], t);
+    sums[r] = wsum[r];
+    sums[R + r] = fsum[r];
   }
-  const unsigned long long t = wblock_sum<BLOCK>(fstates);
-  if (threadIdx.x == 0 && t) atomicAdd(&sc->final_states, t);
-  if (count_next) {
-    const unsigned long long nt = wblock_sum<BLOCK>(nterms);
-    if (threadIdx.x == 0 && nt) atomicAdd(&sc->next_terms, nt);
-    if (blockIdx.x == 0 && threadIdx.x == 0) sc->next_terms_ok = 1u;
+  sums[2 * R] = fstates;
+  sums[2 * R + 1] = nterms;
+  wblock_sums<BLOCK>(sums);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (sums[r]) atomicAdd(&sc->weight_sum[r], sums[r]);
+      if (sums[R + r]) atomicAdd(&sc->final_sum[r], sums[R + r]);
+    }
+    if (sums[2 * R]) atomicAdd(&sc->final_states, sums[2 * R]);
+    if (count_next) {
+      if (sums[2 * R + 1]) atomicAdd(&sc->next_terms, sums[2 * R + 1]);
+      if (blockIdx.x == 0) sc->next_terms_ok = 1u;
+    }
   }
 }
 
@@ -465,6 +501,8 @@ __global__ void __launch_bounds__(BLOCK) frontier_scatter_kernel(const u128* __r
                                                                 WCand<R>* __restrict__ regions,
                                                                 u32* __restrict__ cursors, u32 cstride, u32 parts,
                                                                 u32 cap, StepScalars* __restrict__ sc, StepSource q) {
+  next_kernel_may_start();
+  wait_for_kernel_before();
   if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
   if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   const u64 policy = wl2_keep_policy();
@@ -497,10 +535,10 @@ cudaError_t wide_scatter(const PartitionCfg& pc, const FrontierView& in, u64 n_i
                          u32* cursors, StepScalars* sc, cudaStream_t stream) {
   const u64 want = (n_in + kWScatterBlock * kWPPL - 1) / (kWScatterBlock * kWPPL);
   const unsigned grid = (unsigned)std::max<u64>(1, std::min<u64>(want, (u64)pc.sms * 8));
-  wide_scatter_kernel<R, kWScatterBlock><<<grid, kWScatterBlock, 0, stream>>>(
-      reinterpret_cast<const u128*>(in.keys), in.res, in.cap, n_in, n, reinterpret_cast<WCand<R>*>(regions), cursors,
-      pc.cursor_stride ? pc.cursor_stride : 1, pc.parts, pc.cap, sc, pc.queued);
-  return cudaGetLastError();
+  return launch_overlapped(wide_scatter_kernel<R, kWScatterBlock>, grid, kWScatterBlock, 0, stream,
+                           pc.queued.prev != nullptr, reinterpret_cast<const u128*>(in.keys), in.res, in.cap, n_in, n,
+                           reinterpret_cast<WCand<R>*>(regions), cursors, pc.cursor_stride ? pc.cursor_stride : 1,
+                           pc.parts, pc.cap, sc, pc.queued);
 }
 
 template <int R>
@@ -513,11 +551,11 @@ cudaError_t wide_merge(const PartitionCfg& pc, const void* regions, const u32* c
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const unsigned grid = (unsigned)std::max<u64>(1, std::min<u64>(pc.parts, (u64)pc.sms * 2));
-  kern<<<grid, kWBlock, smem, stream>>>(reinterpret_cast<const WCand<R>*>(regions), cursors,
-                                        pc.cursor_stride ? pc.cursor_stride : 1, pc.parts,
-                                        reinterpret_cast<u128*>(out.keys), out.res, out.cap, n,
-                                        (write_out ? 1 : 0) | (pc.count_next ? 2 : 0), next_step, sc, pc.queued);
-  return cudaGetLastError();
+  return launch_overlapped(kern, grid, kWBlock, smem, stream, pc.queued.prev != nullptr,
+                           reinterpret_cast<const WCand<R>*>(regions), cursors,
+                           pc.cursor_stride ? pc.cursor_stride : 1, pc.parts, reinterpret_cast<u128*>(out.keys),
+                           out.res, out.cap, n, (write_out ? 1 : 0) | (pc.count_next ? 2 : 0), next_step, sc,
+                           pc.queued);
 }
 
 }  // namespace
@@ -576,19 +614,16 @@ cudaError_t launch_frontier_partition_scatter(const PartitionCfg& pc, const Fron
   switch (pc.residues) {
 #define QPEPS_FRONTIER_SCATTER(R)                                                                            \
   case R:                                                                                                   \
-    frontier_scatter_kernel<R, kWScatterBlock><<<grid, kWScatterBlock, 0, stream>>>(                         \
-        keys, in.res, in.cap, n_in, step, reinterpret_cast<WCand<R>*>(regions), cursors, cs, pc.parts, pc.cap, sc,  \
-        pc.queued);                                                                                          \
-    break;
+    return launch_overlapped(frontier_scatter_kernel<R, kWScatterBlock>, grid, kWScatterBlock, 0, stream,     \
+                             pc.queued.prev != nullptr, keys, in.res, in.cap, n_in, step,                   \
+                             reinterpret_cast<WCand<R>*>(regions), cursors, cs, pc.parts, pc.cap, sc, pc.queued);
     QPEPS_FRONTIER_SCATTER(1)
     QPEPS_FRONTIER_SCATTER(2)
     QPEPS_FRONTIER_SCATTER(3)
     QPEPS_FRONTIER_SCATTER(4)
 #undef QPEPS_FRONTIER_SCATTER
-    default:
-      return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 static_assert(sizeof(WCand<1>) == 32 && sizeof(WCand<4>) == 32, "32-byte wide candidates");
