@@ -1195,6 +1195,119 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   return done;
 }
 
+// The per-site form's sites from (row, 0) on as a chain: two kernels a site
+// (expand and insert, compact), each site's table sized on the device from the
+// terms the compaction before counted. Returns the sites contracted; the row
+// of the first one left has its counters added when it is not its first.
+static u64 run_queued_sites_plain(Ctx& ctx, const Plan& p, DevFrontier& f, unsigned row, unsigned stop,
+                                  std::vector<RowAcc>& rows, RunStats& rs) {
+  if (p.grain != QPEPS_GRAIN_SITE || p.batch_states <= 0 || f.count == 0 || row >= stop) return 0;
+  // A boundary inside a row holds the placed and the unplaced states.
+  const double largest = 4.0 * p.batch_states;
+  const u64 most = (u64)std::min((double)kQueueTerms, std::max(65536.0, largest));
+  if (f.count > most / 2) return 0;
+  unsigned count = 0;  // rows expected to stay below that
+  double expect = (double)f.count;
+  while (row + count < stop && (largest <= (double)most || 4.0 * expect <= (double)most)) {
+    expect *= std::max(1.5, (double)p.n - 2.2 * (row + count));
+    ++count;
+  }
+  if (count == 0) return 0;
+  const size_t eb = entry_bytes(p);
+  TableSource source;
+  source.slots_cap = source.slots(most);
+  const size_t table_bytes = source.slots_cap * slot_bytes(p.key_bits, p.R);
+  if (std::max<u64>(f.cap, most) * eb + table_bytes + (1u << 20) > p.budget) return 0;
+  if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
+  if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes)) return 0;
+  if (ctx.pool_bytes - ctx.table.bytes + table_bytes > p.budget) return 0;
+  buf_reserve(ctx, ctx.table, table_bytes, p.budget, "hash table");
+  const size_t sites = (size_t)count * p.n;
+  StepScalars* d = queue_scalars(ctx, p, sites);
+  StepScalars* h = ctx.h_queue;
+  const auto t0 = std::chrono::steady_clock::now();
+  h[0].out_count = f.count;
+  const LaunchCfg cfg{p.key_bits, p.R, p.threads, ctx.sms};
+  const FrontierView view = view_of(p, ctx.front[0], f.cap);
+  // The first site's terms are at most two an entry; its row's counters come
+  // from a count of their own.
+  h[0].next_terms = 2 * f.count;
+  cuda_check(cudaMemcpyAsync(d, h, (sites + 1) * sizeof(StepScalars), cudaMemcpyHostToDevice, ctx.stream),
+             "queued step scalars");
+  cuda_check(cudaMemsetAsync(ctx.d_sc, 0, sizeof(StepScalars), ctx.stream), "clear step scalars");
+  cuda_check(cudaMemsetAsync(ctx.table.ptr, 0, table_bytes, ctx.stream), "clear hash table");
+  cuda_check(launch_row_count(cfg, view, f.count, p.n, ctx.d_sc, ctx.stream), "row count kernel");
+  cuda_check(cudaEventRecord(ctx.ev[0], ctx.stream), "event");
+  u64 entries = f.count;
+  for (size_t i = 0; i < sites; ++i) {
+    const unsigned r = row + (unsigned)(i / p.n), site = (unsigned)(i % p.n);
+    const u64 fits = std::min<u64>(most, 2 * entries);
+    source.prev = d + i;
+    const bool last = r + 1 == p.n && site + 1 == p.n;
+    cuda_check(launch_site_expand_insert(cfg, view, entries, p.n, site, ctx.table.ptr, source.slots(fits), d + i + 1,
+                                         ctx.stream, source),
+               "site expand-insert kernel");
+    cuda_check(launch_compact(cfg, ctx.table.ptr, source.slots(fits), view, p.n, !last, d + i + 1, ctx.stream, source,
+                              site + 1 == p.n ? 0u : site + 1),
+               "compact kernel");
+    entries = fits;
+  }
+  cuda_check(cudaEventRecord(ctx.ev[1], ctx.stream), "event");
+  cuda_check(cudaMemcpyAsync(h, d, (sites + 1) * sizeof(StepScalars), cudaMemcpyDeviceToHost, ctx.stream),
+             "read step scalars");
+  sync_scalars(ctx);
+  ctx.h2d_bytes += (sites + 1) * sizeof(StepScalars);
+  ctx.d2h_bytes += (sites + 1) * sizeof(StepScalars);
+  rs.launches += 1 + 2 * sites;
+  float ms = 0;
+  cudaEventElapsedTime(&ms, ctx.ev[0], ctx.ev[1]);
+  rs.device_ms += ms;
+  size_t done = 0;
+  while (done < sites && !h[done + 1].error) ++done;
+  if (done < sites && (h[done + 1].error & kErrProbeLimit))
+    fail(QPEPS_ERR_CAPACITY, row_msg("hash probe bound exceeded at row", row + (unsigned)(done / p.n) + 1));
+  const QueueTimes times = queue_times(h, done, ms);
+  const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+  if (ctx.rec) ctx.rec->ok = false;
+  for (size_t i = 0; i < done; ++i) {
+    const StepScalars& r = h[i + 1];
+    const unsigned at = row + (unsigned)(i / p.n), site = (unsigned)(i % p.n);
+    const u64 in = i ? h[i].out_count : f.count;
+    RowAcc& acc = rows[at];
+    acc.used = true;
+    acc.device_row = true;
+    if (site == 0) {
+      const u64 examined = i ? h[i].sitewise_examined : ctx.h_sc->sitewise_examined;
+      acc.input_states += in;
+      acc.completed += i ? h[i].row_terms : ctx.h_sc->terms;
+      acc.examined += examined;
+      acc.tmatched += examined;
+    }
+    if (r.terms) {
+      rs.scatter_ms += times.scatter[i];
+      rs.merge_ms += times.merge[i];
+      rs.merge_launches += 1;
+      rs.merge_bytes += (in + r.out_count) * eb;
+      rs.entries_in += in;
+      rs.entries_out += r.out_count;
+    }
+    acc.elapsed += ms > 0 ? wall * (times.scatter[i] + times.merge[i]) / ms : 0.0;
+    // (The first site's terms are a bound; what it merged is exact.)
+    rs.candidates += i ? r.terms : r.out_count;
+    if (site + 1 == p.n) {
+      const bool last = at + 1 == p.n;
+      acc.output_states += r.out_count;
+      for (int q = 0; q < p.Rc; ++q) {
+        acc.weight_res[q] = (acc.weight_res[q] + r.weight_sum[q] % kPrimes[q]) % kPrimes[q];
+        if (last) rs.final_res[q] = (rs.final_res[q] + r.final_sum[q] % kPrimes[q]) % kPrimes[q];
+      }
+      rs.peak_states = std::max<u64>(rs.peak_states, r.out_count);
+    }
+  }
+  if (done) f.count = row + done / p.n == p.n ? 0 : h[done].out_count;
+  return done;
+}
+
 // Contract every pending chunk to the last row. Each chunk is one merged
 // device boundary; under memory pressure a boundary is halved and the upper
 // half parked on the host (exact: the contraction is linear in the boundary).
@@ -1220,6 +1333,13 @@ static void run_chunks(Ctx& ctx, const Plan& p, std::vector<HostChunk> pending, 
         row += queued - 1;
         continue;
       }
+      if (site0 == 0 && !counted)
+        if (const u64 sites = run_queued_sites_plain(ctx, p, f, row, stop, rows, rs)) {
+          row += (unsigned)(sites / p.n);
+          site0 = (unsigned)(sites % p.n);
+          counted = site0 != 0;
+          if (row >= stop) break;
+        }
       const auto t0 = std::chrono::steady_clock::now();
       const bool last_row = row + 1 == p.n;
       RowAcc& acc = rows[row];

@@ -75,6 +75,44 @@ __device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long v
   return t;  // valid in thread 0
 }
 
+// Block sums of several values at once, in thread 0.
+template <int BLOCK, int V>
+__device__ __forceinline__ void block_sums(unsigned long long (&v)[V]) {
+  constexpr int WARPS = BLOCK / 32;
+  __shared__ unsigned long long s_part[V][WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v[i] += __shfl_xor_sync(kFull, v[i], d);
+    if (lane == 0) s_part[i][wid] = v[i];
+  }
+  __syncthreads();
+  if (wid == 0) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      v[i] = lane < WARPS ? s_part[i][lane] : 0ull;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) v[i] += __shfl_xor_sync(kFull, v[i], d);
+    }
+  }
+}
+
+// step_sizes for a step on the global table.
+__device__ __forceinline__ bool table_sizes(const TableSource& q, StepScalars* sc, u64 cap, u64& n_in, u64& slots) {
+  if (!q.prev) return true;
+  const u32 error = q.prev->error;
+  const u64 terms = q.prev->next_terms, entries = q.prev->out_count;
+  const u64 want = q.slots(terms);
+  if (error || want > q.slots_cap || terms > cap) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->error, (u32)(error ? kErrSkipped : kErrCapacity));
+    return false;
+  }
+  n_in = terms ? entries : 0;
+  slots = want;
+  return true;
+}
+
 // ---------------------------------------------------------------------------
 // Successor count of a row step: sum of popcount(~(cols|dr|dl) & mask).
 
@@ -219,7 +257,16 @@ __global__ void __launch_bounds__(BLOCK) site_expand_insert_kernel(const void* _
                                                                    const u32* __restrict__ res, u64 res_stride,
                                                                    u64 n_in, unsigned n, unsigned site,
                                                                    Slot<K, R>* __restrict__ table, u64 table_mask,
-                                                                   StepScalars* __restrict__ sc) {
+                                                                   StepScalars* __restrict__ sc, TableSource q) {
+  next_kernel_may_start();
+  wait_for_kernel_before();
+  u64 slots = table_mask + 1;
+  if (!table_sizes(q, sc, res_stride, n_in, slots)) return;
+  table_mask = slots - 1;
+  if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->t_scatter = global_ns();
+    sc->terms = q.prev->next_terms;
+  }
   const u64 mask = board_mask(n);
   for (u64 i = (u64)blockIdx.x * BLOCK + threadIdx.x; i < n_in; i += (u64)gridDim.x * BLOCK) {
     const K key = load_key<K>(keys, i);
@@ -250,18 +297,27 @@ __global__ void __launch_bounds__(BLOCK) site_expand_insert_kernel(const void* _
 // all set.
 
 template <typename K, int R, int BLOCK, int ITEMS>
-__global__ void __launch_bounds__(BLOCK) compact_kernel(const Slot<K, R>* __restrict__ table, u64 slots,
+__global__ void __launch_bounds__(BLOCK) compact_kernel(Slot<K, R>* __restrict__ table, u64 slots,
                                                         void* __restrict__ keys_out, u32* __restrict__ res_out,
                                                         u64 out_stride, unsigned n, int write_out,
-                                                        StepScalars* __restrict__ sc) {
+                                                        StepScalars* __restrict__ sc, TableSource q,
+                                                        unsigned next_site) {
   constexpr int WARPS = BLOCK / 32;
   __shared__ u32 s_warp[ITEMS][WARPS];
   __shared__ unsigned long long s_base;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const u64 mask = board_mask(n);
   const u64 chunk = (u64)BLOCK * ITEMS;
-  if (*reinterpret_cast<volatile const u32*>(&sc->error)) return;  // insertion failed: leave the boundary intact
+  next_kernel_may_start();
+  wait_for_kernel_before();
+  const u32 failed = *reinterpret_cast<volatile const u32*>(&sc->error);
+  {
+    u64 n_in = 0;
+    if (!table_sizes(q, sc, out_stride, n_in, slots) || failed) return;  // insertion failed: the boundary stays intact
+  }
+  if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_merge = global_ns();
   unsigned long long wsum[R], fsum[R], fstates = 0;
+  unsigned long long nterms = 0, row_terms = 0, sitewise = 0;  // queued: the next site's terms, the next row's
 #pragma unroll
   for (int r = 0; r < R; ++r) wsum[r] = fsum[r] = 0;
 
@@ -308,19 +364,45 @@ __global__ void __launch_bounds__(BLOCK) compact_kernel(const Slot<K, R>* __rest
           if (full) fsum[r] += v;
         }
         fstates += full;
+        if (q.prev) {
+          table[s] = Slot<K, R>{};
+          if (write_out) {
+            u32 rs;
+            nterms += c_table.count[site_signature<K>(key, n, next_site, &rs)];
+            if (next_site == 0) {
+              const State st = unpack<K>(key, n, mask);
+              const u64 fr = ~(st.cols | st.dr | st.dl) & mask;
+              row_terms += __popcll(fr);
+              sitewise += sitewise_entries(fr, n);
+            }
+          }
+        }
       }
     }
     __syncthreads();
   }
+  unsigned long long sums[2 * R + 4];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    unsigned long long t = block_sum_u64<BLOCK>(wsum[r]);
-    if (threadIdx.x == 0 && t) atomicAdd(&sc->weight_sum[r], t);
-    t = block_sum_u64<BLOCK>(fsum[r]);
-    if (threadIdx.x == 0 && t) atomicAdd(&sc->final_sum[r], t);
+    sums[r] = wsum[r];
+    sums[R + r] = fsum[r];
   }
-  unsigned long long t = block_sum_u64<BLOCK>(fstates);
-  if (threadIdx.x == 0 && t) atomicAdd(&sc->final_states, t);
+  sums[2 * R] = fstates;
+  sums[2 * R + 1] = nterms;
+  sums[2 * R + 2] = row_terms;
+  sums[2 * R + 3] = sitewise;
+  block_sums<BLOCK>(sums);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (sums[r]) atomicAdd(&sc->weight_sum[r], sums[r]);
+      if (sums[R + r]) atomicAdd(&sc->final_sum[r], sums[R + r]);
+    }
+    if (sums[2 * R]) atomicAdd(&sc->final_states, sums[2 * R]);
+    if (sums[2 * R + 1]) atomicAdd(&sc->next_terms, sums[2 * R + 1]);
+    if (sums[2 * R + 2]) atomicAdd(&sc->row_terms, sums[2 * R + 2]);
+    if (sums[2 * R + 3]) atomicAdd(&sc->sitewise_examined, sums[2 * R + 3]);
+  }
 }
 
 constexpr int kBlock = 256;
@@ -399,27 +481,35 @@ cudaError_t launch_site_count(const LaunchCfg& cfg, const FrontierView& in, uint
 
 cudaError_t launch_site_expand_insert(const LaunchCfg& cfg, const FrontierView& in, uint64_t n_in, unsigned n,
                                       unsigned site, void* table, uint64_t table_slots, StepScalars* sc,
-                                      cudaStream_t stream) {
+                                      cudaStream_t stream, const TableSource& queued) {
   if (n_in == 0) return cudaSuccess;
   return dispatch(cfg, [&](auto kz, auto rz) -> cudaError_t {
     using K = decltype(kz);
     constexpr int R = decltype(rz)::value;
     const unsigned grid = grid_for(n_in, kBlock, cfg.sms, 8);
-    site_expand_insert_kernel<K, R, kBlock><<<grid, kBlock, 0, stream>>>(
-        in.keys, in.res, in.cap, n_in, n, site, reinterpret_cast<Slot<K, R>*>(table), table_slots - 1, sc);
-    return cudaGetLastError();
+    return launch_overlapped(site_expand_insert_kernel<K, R, kBlock>, grid, kBlock, 0, stream, queued.prev != nullptr,
+                             in.keys, in.res, in.cap, n_in, n, site, reinterpret_cast<Slot<K, R>*>(table),
+                             table_slots - 1, sc, queued);
   });
 }
 
-cudaError_t launch_compact(const LaunchCfg& cfg, const void* table, uint64_t table_slots, const FrontierView& out,
-                           unsigned n, bool write_out, StepScalars* sc, cudaStream_t stream) {
+cudaError_t launch_compact(const LaunchCfg& cfg, void* table, uint64_t table_slots, const FrontierView& out,
+                           unsigned n, bool write_out, StepScalars* sc, cudaStream_t stream, const TableSource& queued,
+                           unsigned next_site) {
   return dispatch(cfg, [&](auto kz, auto rz) -> cudaError_t {
     using K = decltype(kz);
     constexpr int R = decltype(rz)::value;
-    const unsigned grid = grid_for(table_slots, kBlock * kCompactItems, cfg.sms, 8);
-    compact_kernel<K, R, kBlock, kCompactItems><<<grid, kBlock, 0, stream>>>(
-        reinterpret_cast<const Slot<K, R>*>(table), table_slots, out.keys, out.res, out.cap, n, write_out ? 1 : 0, sc);
-    return cudaGetLastError();
+    // Small tables (a queued step's, mostly) take fewer slots a thread, so
+    // that more of the device reads them.
+    auto run = [&](auto items) {
+      constexpr int I = decltype(items)::value;
+      const unsigned grid = grid_for(table_slots, kBlock * I, cfg.sms, 8);
+      return launch_overlapped(compact_kernel<K, R, kBlock, I>, grid, kBlock, 0, stream, queued.prev != nullptr,
+                               reinterpret_cast<Slot<K, R>*>(table), table_slots, out.keys, out.res, out.cap, n,
+                               write_out ? 1 : 0, sc, queued, next_site);
+    };
+    return table_slots <= (uint64_t)cfg.sms * 8 * kBlock * 2 ? run(std::integral_constant<int, 2>())
+                                                             : run(std::integral_constant<int, kCompactItems>());
   });
 }
 

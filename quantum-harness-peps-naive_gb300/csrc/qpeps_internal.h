@@ -40,6 +40,7 @@ struct StepScalars {
   unsigned long long plan_units;         // class-grouped partitions: units of the step's plan (graph replay)
   unsigned long long next_terms;         // successor terms of the written boundary at the next row
   unsigned long long t_scatter, t_merge; // queued steps: start of each kernel (global timer, ns)
+  unsigned long long row_terms;          // queued site steps that end a row: successor terms of its boundary
 };
 
 // Sizes of a queued step: read on the device from the scalars the step before
@@ -81,6 +82,19 @@ inline cudaError_t launch_overlapped(void (*kernel)(Params...), unsigned grid, u
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
+// The same for a queued step on the global table: the slots follow from the
+// terms the step before counted, and the compaction leaves the table empty.
+struct TableSource {
+  const StepScalars* prev = nullptr;  // nullptr: the host passes the sizes
+  uint64_t slots_cap = 0;             // slots the table holds (a power of two)
+
+  __host__ __device__ uint64_t slots(uint64_t terms) const {
+    uint64_t s = 1024;
+    while (s < 2 * terms) s <<= 1;
+    return s;
+  }
+};
+
 struct LaunchCfg {
   int key_bits;  // 64 or 128
   int residues;  // 1..4
@@ -106,11 +120,15 @@ cudaError_t launch_site_count(const LaunchCfg& cfg, const FrontierView& in, uint
 // Explicit-C site update (one launch per site) + global-table insertion.
 cudaError_t launch_site_expand_insert(const LaunchCfg& cfg, const FrontierView& in, uint64_t n_in, unsigned n,
                                       unsigned site, void* table, uint64_t table_slots, StepScalars* scalars,
-                                      cudaStream_t stream);
+                                      cudaStream_t stream, const TableSource& queued = TableSource{});
 
-// Table -> boundary buffer; accumulates weight sums and final (v1) sums.
-cudaError_t launch_compact(const LaunchCfg& cfg, const void* table, uint64_t table_slots, const FrontierView& out,
-                           unsigned n, bool write_out, StepScalars* scalars, cudaStream_t stream);
+// Table -> boundary buffer; accumulates weight sums and final (v1) sums. A
+// queued step's compaction also empties the table and counts the next site's
+// terms (`next_site` in [0, n); at 0 the successor terms and sitewise entries
+// of the row that follows, too).
+cudaError_t launch_compact(const LaunchCfg& cfg, void* table, uint64_t table_slots, const FrontierView& out,
+                           unsigned n, bool write_out, StepScalars* scalars, cudaStream_t stream,
+                           const TableSource& queued = TableSource{}, unsigned next_site = 0);
 
 // Bytes per table slot for a key width / residue count.
 size_t slot_bytes(int key_bits, int residues);
