@@ -423,6 +423,7 @@ struct Plan {
   size_t budget;
   int threads;
   unsigned tail_row;  // rows >= tail_row go to the slice-tail kernel (n = none)
+  bool prefix = false;      // a partly placed board
   double batch_states = 0;  // expected largest boundary of one device batch (0: unknown)
   bool w64 = false;   // residue planes 0/1 hold the low/high words of exact weights (partitioned row merge)
   int Rc = 0;         // residues of the CRT bookkeeping (= R except with w64, where R = 2 planes)
@@ -991,9 +992,9 @@ static void run_tail(Ctx& ctx, const Plan& p, DevFrontier& f, unsigned row0, std
 // more memory than the wait costs.
 constexpr u64 kQueueTerms = 4u << 20;
 
-// Scalars of `steps` queued steps and of the state before them ([0], which the
-// caller fills), pinned and on the device.
-static StepScalars* queue_scalars(Ctx& ctx, const Plan& p, size_t steps) {
+// Pinned scalars of `steps` steps and of the state before them ([0], which the
+// caller fills), zero.
+static StepScalars* pinned_scalars(Ctx& ctx, size_t steps) {
   const size_t n = steps + 1;
   if (ctx.h_queue_steps < n) {
     if (ctx.h_queue) cudaFreeHost(ctx.h_queue);
@@ -1002,8 +1003,14 @@ static StepScalars* queue_scalars(Ctx& ctx, const Plan& p, size_t steps) {
     cuda_check(cudaMallocHost(&ctx.h_queue, n * sizeof(StepScalars)), "pinned step scalars");
     ctx.h_queue_steps = n;
   }
-  buf_reserve(ctx, ctx.queue, n * sizeof(StepScalars), p.budget, "queued step scalars");
   std::memset(ctx.h_queue, 0, n * sizeof(StepScalars));
+  return ctx.h_queue;
+}
+
+// The same with their copy on the device.
+static StepScalars* queue_scalars(Ctx& ctx, const Plan& p, size_t steps) {
+  pinned_scalars(ctx, steps);
+  buf_reserve(ctx, ctx.queue, (steps + 1) * sizeof(StepScalars), p.budget, "queued step scalars");
   return static_cast<StepScalars*>(ctx.queue.ptr);
 }
 
@@ -1024,6 +1031,78 @@ static QueueTimes queue_times(const StepScalars* h, size_t steps, double total) 
   }
   if (steps) t.merge.back() += std::max(0.0, total - sum);
   return t;
+}
+
+// A finished row's metrics: `in` entries with `terms` successors. `exact`:
+// plane 0 carries exact sums.
+static void add_row(const Plan& p, unsigned row, u64 in, u64 terms, const StepScalars& r, bool exact,
+                    std::vector<RowAcc>& rows, RunStats& rs) {
+  RowAcc& acc = rows[row];
+  acc.used = true;
+  acc.device_row = true;
+  acc.input_states += in;
+  acc.candidates += (u128)in * p.n;
+  acc.matched += terms;
+  acc.completed += terms;
+  acc.output_states += r.out_count;
+  for (int q = 0; q < p.Rc; ++q) {
+    acc.weight_res[q] = (acc.weight_res[q] + r.weight_sum[exact ? 0 : q] % kPrimes[q]) % kPrimes[q];
+    if (row + 1 == p.n) rs.final_res[q] = (rs.final_res[q] + r.final_sum[exact ? 0 : q] % kPrimes[q]) % kPrimes[q];
+  }
+  rs.peak_states = std::max<u64>(rs.peak_states, r.out_count);
+  if (!terms) return;
+  rs.merge_launches += 1;
+  rs.merge_bytes += (in + r.out_count) * entry_bytes(p);
+  rs.entries_in += in;
+  rs.entries_out += r.out_count;
+  rs.candidates += terms;
+}
+
+// A partly placed board whose boundary is expected to fit one CTA's shared
+// memory, from its host entries to the last row in one launch that writes its
+// scalars to pinned memory. (Whole boards run row by row: they report each
+// row's time.) False, with nothing added, where it does not apply or the
+// boundary outgrew it.
+static bool run_resident(Ctx& ctx, const Plan& p, const HostChunk& hc, std::vector<RowAcc>& rows, RunStats& rs) {
+  if (!p.prefix || hc.count == 0 || hc.count > kResidentSeeds || hc.no_tail || hc.row >= p.n || p.tail_row < p.n ||
+      p.batch_states <= 0 || p.batch_states > 0.5 * resident_capacity() || p.grain != QPEPS_GRAIN_ROW ||
+      p.merge != QPEPS_MERGE_PARTITION || p.key_bits != 64 || p.free_rows > 20 || ctx.tune.merge_kind != 1 ||
+      ctx.tune.scatter_kind != 1 || ctx.tune.fold_weights != 2 || !(p.w64 || p.R == 1))
+    return false;
+  const auto t0 = std::chrono::steady_clock::now();
+  const unsigned count = p.n - hc.row;
+  StepScalars* h = pinned_scalars(ctx, count);
+  ResidentArgs a{};
+  a.n = p.n;
+  a.row = hc.row;
+  a.count = (u32)hc.count;
+  a.out = h + 1;
+  const u64 mask = (1ull << p.n) - 1;
+  h[0].out_count = hc.count;
+  for (u64 i = 0; i < hc.count; ++i) {
+    std::memcpy(&a.key[i], &hc.keys[i * 8], 8);
+    a.weight[i] = p.w64 ? (u64)hc.res[i] | ((u64)hc.res[hc.count + i] << 32) : hc.res[i];
+    const State st = unpack<u64>(a.key[i], p.n, mask);
+    h[0].next_terms += (u64)__builtin_popcountll(~(st.cols | st.dr | st.dl) & mask);
+  }
+  cuda_check(launch_resident_rows(a, ctx.stream), "resident rows kernel");
+  cuda_check(cudaStreamSynchronize(ctx.stream), "resident rows");
+  rs.launches += 1;
+  if (h[1].error) return false;
+  if (ctx.rec) ctx.rec->ok = false;
+  ctx.h2d_bytes += sizeof a;
+  ctx.d2h_bytes += count * sizeof(StepScalars);
+  rs.batches += 1;
+  const double ms = h[count].t_merge > h[1].t_scatter ? (double)(h[count].t_merge - h[1].t_scatter) * 1e-6 : 0.0;
+  rs.device_ms += ms;
+  rs.merge_ms += ms;
+  rs.peak_states = std::max<u64>(rs.peak_states, hc.count);
+  const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+  for (unsigned i = 0; i < count; ++i) {
+    rows[hc.row + i].elapsed += wall / count;
+    add_row(p, hc.row + i, h[i].out_count, h[i].next_terms, h[i + 1], true, rows, rs);
+  }
+  return true;
 }
 
 // Rows [row, stop) of the live boundary as a chain; returns how many were
@@ -1136,29 +1215,12 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
       if (bound >> 63) fail(QPEPS_ERR_OVERFLOW, row_msg("exact 64-bit weights are not certified at row", row + i + 1));
       f.weight_bound = r.weight_sum[0];
     }
-    RowAcc& acc = rows[row + i];
-    acc.used = true;
-    acc.device_row = true;
-    acc.input_states += in;
-    acc.candidates += (u128)in * p.n;
-    acc.matched += tm;
-    acc.completed += tm;
-    acc.output_states += r.out_count;
-    for (int q = 0; q < p.Rc; ++q) {
-      acc.weight_res[q] = (acc.weight_res[q] + r.weight_sum[p.w64 ? 0 : q] % kPrimes[q]) % kPrimes[q];
-      if (last) rs.final_res[q] = (rs.final_res[q] + r.final_sum[p.w64 ? 0 : q] % kPrimes[q]) % kPrimes[q];
-    }
-    acc.elapsed += ms > 0 ? wall * (times.scatter[i] + times.merge[i]) / ms : 0.0;
-    rs.peak_states = std::max<u64>(rs.peak_states, r.out_count);
+    rows[row + i].elapsed += ms > 0 ? wall * (times.scatter[i] + times.merge[i]) / ms : 0.0;
     if (tm) {
       rs.scatter_ms += times.scatter[i];
       rs.merge_ms += times.merge[i];
-      rs.merge_launches += 1;
-      rs.merge_bytes += (in + r.out_count) * eb;
-      rs.entries_in += in;
-      rs.entries_out += r.out_count;
-      rs.candidates += tm;
     }
+    add_row(p, row + i, in, tm, r, p.w64, rows, rs);
     if (ctx.rec) {
       // What the row would have recorded by itself.
       GraphStepRec g;
@@ -1321,6 +1383,7 @@ static void run_chunks(Ctx& ctx, const Plan& p, std::vector<HostChunk> pending, 
   while (!pending.empty()) {
     HostChunk hc = std::move(pending.back());
     pending.pop_back();
+    if (run_resident(ctx, p, hc, rows, rs)) continue;
     upload_chunk(ctx, p, hc, f);
     rs.batches += 1;
     rs.peak_states = std::max<u64>(rs.peak_states, f.count);
@@ -1621,7 +1684,7 @@ struct ExplicitRun {
 // the next step's matches, if `next_dev` (the next step on the device) was
 // given and the merge counted them.
 static u64 explicit_partition_step(Ctx& ctx, const Plan& p, DevFrontier& f, const FrontierStepDev& st,
-                                   const FrontierStepDev* next_dev, u64& known_terms, ExplicitRun& out) {
+                                   const FrontierStepDev* st_dev, const FrontierStepDev* next_dev, u64& known_terms, ExplicitRun& out) {
   float ms = 0;
   u64 terms = known_terms;
   known_terms = kTermsUnknown;
@@ -1668,7 +1731,7 @@ static u64 explicit_partition_step(Ctx& ctx, const Plan& p, DevFrontier& f, cons
     cuda_check(cudaMemsetAsync(ctx.d_sc, 0, sizeof(StepScalars), ctx.stream), "clear step scalars");
     cuda_check(cudaMemsetAsync(cursors, 0, (size_t)parts * 4 * cstride, ctx.stream), "clear partition cursors");
     cuda_check(cudaEventRecord(ctx.ev[0], ctx.stream), "event");
-    cuda_check(launch_frontier_partition_scatter(pc, view, f.count, st, regions, cursors, ctx.d_sc, ctx.stream),
+    cuda_check(launch_frontier_partition_scatter(pc, view, f.count, st_dev, regions, cursors, ctx.d_sc, ctx.stream),
                "frontier scatter kernel");
     cuda_check(launch_wide_partition_merge(pc, regions, cursors, view, 0, true, ctx.d_sc, ctx.stream, next_dev),
                "frontier merge kernel");
@@ -1742,7 +1805,7 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
     // The merge counts the next step's matches, for the chain or the step that
     // follows it.
     const bool next = i + 1 < steps.size() && open_after[i + 1] < 128;
-    cuda_check(launch_frontier_partition_scatter(pc, view, entries, steps[i], regions, cursors, d + i + 1, ctx.stream),
+    cuda_check(launch_frontier_partition_scatter(pc, view, entries, d_steps + i, regions, cursors, d + i + 1, ctx.stream),
                "frontier scatter kernel");
     cuda_check(launch_wide_partition_merge(pc, regions, cursors, view, 0, true, d + i + 1, ctx.stream,
                                            next ? d_steps + i + 1 : nullptr),
@@ -1916,7 +1979,7 @@ static void explicit_frontier(Ctx& ctx, unsigned n, unsigned order, u64 support_
   const bool partitioned = ctx.tune.merge_auto != QPEPS_MERGE_HASH;
   out.merge = partitioned ? QPEPS_MERGE_PARTITION : QPEPS_MERGE_HASH;
   FrontierStepDev* d_steps = nullptr;
-  if (partitioned && total > 1) {
+  if (partitioned) {
     buf_reserve(ctx, ctx.plan, total * sizeof(FrontierStepDev), p.budget, "explicit-C frontier steps");
     d_steps = static_cast<FrontierStepDev*>(ctx.plan.ptr);
     cuda_check(cudaMemcpyAsync(d_steps, steps.data(), total * sizeof(FrontierStepDev), cudaMemcpyHostToDevice,
@@ -1959,8 +2022,8 @@ static void explicit_frontier(Ctx& ctx, unsigned n, unsigned order, u64 support_
     out.examined += (u128)f.count * 17;
     if (partitioned && next_open < 128) {
       const bool next_partitioned = step + 1 < total && step + 1 != fail_step && open_after[step + 1] < 128;
-      const FrontierStepDev* next_dev = (d_steps && next_partitioned) ? d_steps + step + 1 : nullptr;
-      const u64 terms = explicit_partition_step(ctx, p, f, st, next_dev, known_terms, out);
+      const FrontierStepDev* next_dev = next_partitioned ? d_steps + step + 1 : nullptr;
+      const u64 terms = explicit_partition_step(ctx, p, f, st, d_steps + step, next_dev, known_terms, out);
       out.accepted += terms;
       if (!merged_step(step, *ctx.h_sc)) return;
       continue;
@@ -2476,6 +2539,7 @@ static void contract_impl(Ctx& ctx, unsigned n, const qpeps_options& o, const ui
   // (Known for a whole board with the orbits, about twice that without them,
   // estimated below a prefix.)
   out.plan.batch_states = serve_estimate(n, k) * (k ? 3.0 : o.symmetry ? 1.0 : 2.0);
+  out.plan.prefix = k > 0;
   // Predictive slicing: when the merged frontier is estimated not to fit the
   // device budget, contract groups of slices (first-row orbit slices, or
   // deeper prefix slices) one chunk at a time instead of halving a live

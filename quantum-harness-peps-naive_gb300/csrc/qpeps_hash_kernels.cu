@@ -252,13 +252,56 @@ __global__ void __launch_bounds__(BLOCK) site_count_kernel(const void* __restric
   if (threadIdx.x == 0 && t) atomicAdd(&sc->terms, t);
 }
 
+// Insert up to two children of one entry side by side: both compare-and-swaps
+// are in flight at once, and a child's first probe is the swap itself (a
+// small step's time is its dependent trips to memory, and its table is at most
+// half full).
+template <typename K, int R>
+__device__ __forceinline__ void table_insert_pair(Slot<K, R>* __restrict__ table, u64 mask, const K (&child)[2],
+                                                  const u32 (&w)[2][R], u32 have, u32* err) {
+  u64 pos[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) pos[c] = key_hash<K>(child[c]) & mask;
+  u32 todo = have;
+  for (u32 probe = 0; todo; ++probe) {
+    if (probe == kMaxProbe) {
+      atomicOr(err, kErrProbeLimit);
+      return;
+    }
+    K cur[2] = {0, 0};
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if ((todo >> c) & 1u) cur[c] = atomic_cas_key(&table[pos[c]].nkey, (K)0, ~child[c]);
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if ((todo >> c) & 1u) {
+        if (cur[c] == (K)0 || cur[c] == ~child[c]) {
+          todo ^= 1u << c;
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            atomicAdd((unsigned long long*)&table[pos[c]].acc[r], (unsigned long long)w[c][r]);
+        } else {
+          pos[c] = (pos[c] + 1) & mask;
+        }
+      }
+  }
+}
+
+// The C table is read through shared memory: the lanes of a warp have
+// different signatures, which constant memory serves one after the other, and
+// after a launch every line of it is a miss. The copy is made before the
+// kernel waits for the one before it.
 template <typename K, int R, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) site_expand_insert_kernel(const void* __restrict__ keys,
                                                                    const u32* __restrict__ res, u64 res_stride,
                                                                    u64 n_in, unsigned n, unsigned site,
                                                                    Slot<K, R>* __restrict__ table, u64 table_mask,
                                                                    StepScalars* __restrict__ sc, TableSource q) {
+  __shared__ CTableDev s_c;
   next_kernel_may_start();
+  for (u32 i = threadIdx.x; i < sizeof(CTableDev) / 4; i += BLOCK)
+    reinterpret_cast<u32*>(&s_c)[i] = reinterpret_cast<const u32*>(&c_table)[i];
+  __syncthreads();
   wait_for_kernel_before();
   u64 slots = table_mask + 1;
   if (!table_sizes(q, sc, res_stride, n_in, slots)) return;
@@ -275,17 +318,22 @@ __global__ void __launch_bounds__(BLOCK) site_expand_insert_kernel(const void* _
     for (int r = 0; r < R; ++r) w[r] = res[r * res_stride + i];
     u32 rs;
     const u32 sig = site_signature<K>(key, n, site, &rs);
-    const u32 cnt = c_table.count[sig];
-    for (u32 e = 0; e < cnt; ++e) {
-      K child;
-      if (!site_apply<K>(key, n, site, c_table.out[sig][e], mask, &child)) continue;
-      u32 cw[R];
+    const u32 cnt = s_c.count[sig];
+    for (u32 e0 = 0; e0 < cnt; e0 += 2) {
+      K child[2] = {0, 0};
+      u32 cw[2][R] = {}, have = 0;
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const u32 v = c_table.value_mod[sig][e][r];
-        cw[r] = v == 1u ? w[r] : mul_mod(w[r], v, prime_at(r));
+      for (u32 c = 0; c < 2; ++c) {
+        const u32 e = e0 + c;
+        if (e >= cnt || !site_apply<K>(key, n, site, s_c.out[sig][e], mask, &child[c])) continue;
+        have |= 1u << c;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const u32 v = s_c.value_mod[sig][e][r];
+          cw[c][r] = v == 1u ? w[r] : mul_mod(w[r], v, prime_at(r));
+        }
       }
-      table_insert<K, R>(table, table_mask, child, cw, kMaxProbe, &sc->error);
+      if (have) table_insert_pair<K, R>(table, table_mask, child, cw, have, &sc->error);
     }
   }
 }

@@ -88,9 +88,13 @@ struct TableSource {
   const StepScalars* prev = nullptr;  // nullptr: the host passes the sizes
   uint64_t slots_cap = 0;             // slots the table holds (a power of two)
 
+  // A small step's time is its longest probe sequence, a trip to L2 each: at
+  // loads up to 1/2, 30 K terms took 18 us, at up to 1/8 7 us. Larger steps
+  // are bound by reading the table back.
   __host__ __device__ uint64_t slots(uint64_t terms) const {
+    const uint64_t want = terms <= 65536 ? 8 * terms : terms <= 262144 ? 4 * terms : 2 * terms;
     uint64_t s = 1024;
-    while (s < 2 * terms) s <<= 1;
+    while (s < want) s <<= 1;
     return s;
   }
 };
@@ -216,8 +220,10 @@ cudaError_t launch_append_probe(uint32_t mode, uint64_t total, uint32_t parts, u
 // with n = 0). Keys must not set all 128 bits (at most 127 open bonds).
 cudaError_t launch_frontier_count(const FrontierView& in, uint64_t n_in, const FrontierStepDev& step, int sms,
                                   StepScalars* scalars, cudaStream_t stream);
+// (`step`: its copy on the device, at most kFrontierMaxRuns runs and
+// kFrontierMaxTrans transitions.)
 cudaError_t launch_frontier_partition_scatter(const PartitionCfg& pc, const FrontierView& in, uint64_t n_in,
-                                              const FrontierStepDev& step, void* regions, uint32_t* cursors,
+                                              const FrontierStepDev* step, void* regions, uint32_t* cursors,
                                               StepScalars* scalars, cudaStream_t stream);
 // Candidate slots per partition for a merge shape (PartitionCfg::wide).
 uint32_t partition_capacity(uint32_t wide = 0);
@@ -279,6 +285,22 @@ cudaError_t launch_partition_merge(const PartitionCfg& pc, const void* regions, 
                                    cudaStream_t stream);
 
 
+
+// Rows [row, n) of a few seed states in one CTA, the boundary in shared memory
+// (qpeps_resident_kernels.cu): u64 keys, exact 64-bit weights. out[i] takes row
+// row + i's scalars (out_count, next_terms, weight_sum[0], final_sum[0],
+// final_states; the start and end stamps of the whole in out[0].t_scatter and
+// the last row's t_merge); `out` may be pinned host memory. A boundary that
+// outgrows the CTA stops it with kErrCapacity in out[0].error.
+constexpr uint32_t kResidentSeeds = 24;
+struct ResidentArgs {
+  uint32_t n, row, count;
+  uint64_t key[kResidentSeeds];
+  uint64_t weight[kResidentSeeds];
+  StepScalars* out;
+};
+uint32_t resident_capacity();
+cudaError_t launch_resident_rows(const ResidentArgs& a, cudaStream_t stream);
 
 // Serving (slotted keys, R = 2): count, scatter and merge of a boundary
 // shared by requests of different board sizes. slot_mask[s] is the board mask

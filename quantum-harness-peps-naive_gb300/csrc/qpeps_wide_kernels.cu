@@ -494,35 +494,62 @@ __global__ void __launch_bounds__(BLOCK) frontier_count_kernel(const u128* __res
   }
 }
 
+// The step comes from device memory through shared memory, copied before the
+// kernel waits for the one before it: as a kernel parameter every line of its
+// 1.4 KB was a constant-cache miss, one after the other (a step of 338 entries
+// took 9.9 us). An entry's two candidates take their cursors side by side.
 template <int R, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) frontier_scatter_kernel(const u128* __restrict__ keys,
                                                                 const u32* __restrict__ res, u64 res_stride,
-                                                                u64 n_in, const __grid_constant__ FrontierStepDev st,
+                                                                u64 n_in, const FrontierStepDev* __restrict__ step,
                                                                 WCand<R>* __restrict__ regions,
                                                                 u32* __restrict__ cursors, u32 cstride, u32 parts,
                                                                 u32 cap, StepScalars* __restrict__ sc, StepSource q) {
+  __shared__ FrontierStepDev s_st;
+  static_assert(sizeof(FrontierStepDev) % 16 == 0, "copied in 16-byte words");
   next_kernel_may_start();
+  for (u32 i = threadIdx.x; i < sizeof(FrontierStepDev) / 16; i += BLOCK)
+    reinterpret_cast<uint4*>(&s_st)[i] = reinterpret_cast<const uint4*>(step)[i];
+  __syncthreads();
   wait_for_kernel_before();
   if (!step_sizes(q, sc, res_stride, n_in, parts)) return;
   if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_scatter = global_ns();
   const u64 policy = wl2_keep_policy();
   bool overflow = false;
+  const u32 n_runs = s_st.n_runs, n_trans = s_st.n_trans;
   for (u64 i = (u64)blockIdx.x * BLOCK + threadIdx.x; i < n_in; i += (u64)gridDim.x * BLOCK) {
     const u128 key = wload_key(keys + i);
-    u128 moved = 0;
-    for (u32 r = 0; r < st.n_runs; ++r) moved |= wshift(key & st.run_mask[r], st.run_shift[r]);
     WCand<R> c;
 #pragma unroll
     for (int r = 0; r < R; ++r) c.res[r] = __ldcs(res + r * res_stride + i);
-    for (u32 t = 0; t < st.n_trans; ++t) {
-      if ((key & st.req_mask[t]) != st.req_value[t]) continue;
-      c.key = moved | st.added[t];
-      const u32 part = wpartition_of(c.key, parts);
-      const u32 pos = atomicAdd(&cursors[(u64)part * cstride], 1u);
-      if (pos < cap)
-        wstore<R>(regions + (u64)part * cap + pos, c, policy);
-      else
-        overflow = true;
+    u128 moved = 0;
+    for (u32 r = 0; r < n_runs; ++r) moved |= wshift(key & wld_shared(&s_st.run_mask[r]), s_st.run_shift[r]);
+    for (u32 t = 0; t < n_trans;) {
+      u128 child[2] = {0, 0};
+      u32 found = 0;
+      for (; t < n_trans && found < 2; ++t)
+        if ((key & wld_shared(&s_st.req_mask[t])) == wld_shared(&s_st.req_value[t])) {
+          const u128 k = moved | wld_shared(&s_st.added[t]);
+          if (found) child[1] = k;
+          else child[0] = k;
+          ++found;
+        }
+      u32 part[2], pos[2] = {0, 0};
+#pragma unroll
+      for (u32 k = 0; k < 2; ++k)
+        if (k < found) {
+          part[k] = wpartition_of(child[k], parts);
+          pos[k] = atomicAdd(&cursors[(u64)part[k] * cstride], 1u);
+        }
+#pragma unroll
+      for (u32 k = 0; k < 2; ++k)
+        if (k < found) {
+          c.key = child[k];
+          if (pos[k] < cap)
+            wstore<R>(regions + (u64)part[k] * cap + pos[k], c, policy);
+          else
+            overflow = true;
+        }
     }
   }
   if (overflow) atomicOr(&sc->error, kErrOverflow);
@@ -601,11 +628,10 @@ cudaError_t launch_frontier_count(const FrontierView& in, uint64_t n_in, const F
 }
 
 cudaError_t launch_frontier_partition_scatter(const PartitionCfg& pc, const FrontierView& in, uint64_t n_in,
-                                              const FrontierStepDev& step, void* regions, uint32_t* cursors,
+                                              const FrontierStepDev* step, void* regions, uint32_t* cursors,
                                               StepScalars* sc, cudaStream_t stream) {
   if (n_in == 0) return cudaSuccess;
-  if (n_in > in.cap || pc.parts == 0 || pc.cap != (u32)kWCap || step.n_trans > (uint32_t)kFrontierMaxTrans ||
-      step.n_runs > (uint32_t)kFrontierMaxRuns || reinterpret_cast<uintptr_t>(regions) % 32)
+  if (n_in > in.cap || pc.parts == 0 || pc.cap != (u32)kWCap || !step || reinterpret_cast<uintptr_t>(regions) % 32)
     return cudaErrorInvalidValue;
   const u64 want = (n_in + kWScatterBlock - 1) / kWScatterBlock;
   const unsigned grid = (unsigned)std::max<u64>(1, std::min<u64>(want, (u64)pc.sms * 8));
