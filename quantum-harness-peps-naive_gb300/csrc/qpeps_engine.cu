@@ -305,9 +305,38 @@ struct Ctx {
   DevBuf queue;                  // queued steps: their scalars
   StepScalars* h_queue = nullptr;  // pinned: the scalars as uploaded, then as read back
   size_t h_queue_steps = 0;
+  uint8_t* h_seed = nullptr;     // pinned: a small chunk on its way to the device (kSeedStage bytes)
   uint64_t pool_gen = 0;         // bumped whenever a pool buffer is allocated or freed
   GraphRecorder* rec = nullptr;  // row steps of the running contraction (use_graph)
   GraphPlan* graph = nullptr;    // captured contraction (use_graph)
+};
+
+// Device memory a call may hold: the caller's figure, or 90 % of what is free
+// or already in the context's pool. Free memory is asked for only when the
+// pool alone does not answer the question (the query takes about 15 us, more
+// than a small board's launches).
+class Budget {
+ public:
+  Budget() = default;
+  explicit Budget(size_t bytes) : bytes_(bytes) {}
+  explicit Budget(const Ctx& ctx) : ctx_(&ctx) {}
+  bool known() const { return !ctx_ || bytes_; }
+  operator size_t() const {
+    if (!known()) {
+      size_t fr = 0, tot = 0;
+      cuda_check(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo");
+      bytes_ = (size_t)((double)(fr + ctx_->pool_bytes) * 0.90);
+    }
+    return bytes_;
+  }
+  bool holds(size_t need) const {
+    if (!known() && (double)need <= 0.90 * (double)ctx_->pool_bytes) return true;
+    return need <= (size_t)*this;
+  }
+
+ private:
+  const Ctx* ctx_ = nullptr;
+  mutable size_t bytes_ = 0;
 };
 
 static void buf_release(Ctx& ctx, DevBuf& b) {
@@ -320,7 +349,7 @@ static void buf_release(Ctx& ctx, DevBuf& b) {
   b.bytes = 0;
 }
 
-static void buf_reserve(Ctx& ctx, DevBuf& b, size_t bytes, size_t budget, const char* what) {
+static void buf_reserve(Ctx& ctx, DevBuf& b, size_t bytes, const Budget& budget, const char* what) {
   if (b.bytes >= bytes) return;
   size_t want = bytes + bytes / 4;
   if (ctx.pool_bytes - b.bytes + want > budget) want = bytes;
@@ -351,6 +380,7 @@ static void ctx_free(Ctx* ctx) {
   buf_release(*ctx, ctx->plan);
   buf_release(*ctx, ctx->queue);
   if (ctx->h_queue) cudaFreeHost(ctx->h_queue);
+  if (ctx->h_seed) cudaFreeHost(ctx->h_seed);
   if (ctx->d_sc) cudaFree(ctx->d_sc);
   if (ctx->h_sc) cudaFreeHost(ctx->h_sc);
   for (auto& e : ctx->ev)
@@ -420,7 +450,7 @@ struct Plan {
   int key_bits;
   int grain;
   int merge;  // QPEPS_MERGE_HASH or QPEPS_MERGE_PARTITION
-  size_t budget;
+  Budget budget;
   int threads;
   unsigned tail_row;  // rows >= tail_row go to the slice-tail kernel (n = none)
   bool prefix = false;      // a partly placed board
@@ -837,12 +867,15 @@ static void split_to_host(Ctx& ctx, const Plan& p, DevFrontier& f, unsigned row,
   pending.push_back(std::move(hc));
 }
 
+constexpr size_t kSeedStage = 64 << 10;
+
 static void upload_chunk(Ctx& ctx, const Plan& p, const HostChunk& hc, DevFrontier& f) {
   // Pooled buffers are dead between chunks; drop them only if they exceed
   // this call's budget or cannot hold the chunk.
   f.count = 0;
-  if (ctx.pool_bytes > p.budget) buf_release(ctx, ctx.table);
-  if (f.cap < hc.count || ctx.front[0].bytes > p.budget) {
+  const bool bounded = p.budget.known();
+  if (bounded && ctx.pool_bytes > p.budget) buf_release(ctx, ctx.table);
+  if (f.cap < hc.count || (bounded && ctx.front[0].bytes > p.budget)) {
     buf_release(ctx, ctx.front[0]);
     f.cap = 0;
   }
@@ -850,12 +883,25 @@ static void upload_chunk(Ctx& ctx, const Plan& p, const HostChunk& hc, DevFronti
     fail(QPEPS_ERR_CAPACITY, "device budget cannot hold the seed boundary");
   const size_t kb = key_bytes(p);
   char* dst = static_cast<char*>(ctx.front[0].ptr);
-  cuda_check(cudaMemcpyAsync(dst, hc.keys.data(), hc.count * kb, cudaMemcpyHostToDevice, ctx.stream), "upload keys");
+  // A small chunk goes through pinned memory, which the copies read while the
+  // host goes on (the chunk's last row is waited for before the next upload).
+  const size_t bytes = hc.count * (kb + 4u * p.R);
+  const uint8_t* keys = hc.keys.data();
+  const uint8_t* res = reinterpret_cast<const uint8_t*>(hc.res.data());
+  const bool staged = bytes <= kSeedStage;
+  if (staged) {
+    if (!ctx.h_seed) cuda_check(cudaMallocHost(&ctx.h_seed, kSeedStage), "pinned seed staging");
+    std::memcpy(ctx.h_seed, keys, hc.count * kb);
+    std::memcpy(ctx.h_seed + hc.count * kb, res, hc.count * 4u * p.R);
+    keys = ctx.h_seed;
+    res = ctx.h_seed + hc.count * kb;
+  }
+  cuda_check(cudaMemcpyAsync(dst, keys, hc.count * kb, cudaMemcpyHostToDevice, ctx.stream), "upload keys");
   for (int r = 0; r < p.R; ++r)
-    cuda_check(cudaMemcpyAsync(dst + f.cap * kb + (size_t)r * f.cap * 4, hc.res.data() + (size_t)r * hc.count,
-                               hc.count * 4, cudaMemcpyHostToDevice, ctx.stream),
+    cuda_check(cudaMemcpyAsync(dst + f.cap * kb + (size_t)r * f.cap * 4, res + (size_t)r * hc.count * 4, hc.count * 4,
+                               cudaMemcpyHostToDevice, ctx.stream),
                "upload residues");
-  cuda_check(cudaStreamSynchronize(ctx.stream), "upload synchronize");
+  if (!staged) cuda_check(cudaStreamSynchronize(ctx.stream), "upload synchronize");
   ctx.h2d_bytes += hc.count * (kb + 4u * p.R);
   f.count = hc.count;
   f.weight_bound = hc.weight_bound;
@@ -1033,6 +1079,16 @@ static QueueTimes queue_times(const StepScalars* h, size_t steps, double total) 
   return t;
 }
 
+// Room for a chain: a boundary of `most` entries and `table_bytes` of scratch.
+// Buffers that stand are not asked about again.
+static bool chain_buffers(Ctx& ctx, const Plan& p, DevFrontier& f, u64 most, size_t table_bytes) {
+  if (!p.budget.known() && f.cap >= most && ctx.table.bytes >= table_bytes) return true;
+  if (!p.budget.holds(std::max<u64>(f.cap, most) * entry_bytes(p) + table_bytes + (1u << 20))) return false;
+  if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
+  if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes)) return false;
+  return p.budget.holds(ctx.pool_bytes - ctx.table.bytes + table_bytes);
+}
+
 // A finished row's metrics: `in` entries with `terms` successors. `exact`:
 // plane 0 carries exact sums.
 static void add_row(const Plan& p, unsigned row, u64 in, u64 terms, const StepScalars& r, bool exact,
@@ -1144,10 +1200,7 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   const size_t region_bytes = (size_t)parts_cap * pcap * cand_bytes(p);
   const size_t cursor_bytes = (size_t)parts_cap * 4 * cstride;
   const size_t table_bytes = region_bytes + (cursor_bytes + 255) / 256 * 256;
-  if (std::max<u64>(f.cap, most) * eb + table_bytes + (1u << 20) > p.budget) return 0;
-  if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
-  if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes)) return 0;
-  if (ctx.pool_bytes - ctx.table.bytes + table_bytes > p.budget) return 0;
+  if (!chain_buffers(ctx, p, f, most, table_bytes)) return 0;
   buf_reserve(ctx, ctx.table, table_bytes, p.budget, "partition regions");
   StepScalars* d = queue_scalars(ctx, p, count);
   StepScalars* h = ctx.h_queue;
@@ -1279,10 +1332,7 @@ static u64 run_queued_sites_plain(Ctx& ctx, const Plan& p, DevFrontier& f, unsig
   TableSource source;
   source.slots_cap = source.slots(most);
   const size_t table_bytes = source.slots_cap * slot_bytes(p.key_bits, p.R);
-  if (std::max<u64>(f.cap, most) * eb + table_bytes + (1u << 20) > p.budget) return 0;
-  if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
-  if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes)) return 0;
-  if (ctx.pool_bytes - ctx.table.bytes + table_bytes > p.budget) return 0;
+  if (!chain_buffers(ctx, p, f, most, table_bytes)) return 0;
   buf_reserve(ctx, ctx.table, table_bytes, p.budget, "hash table");
   const size_t sites = (size_t)count * p.n;
   StepScalars* d = queue_scalars(ctx, p, sites);
@@ -1538,13 +1588,7 @@ static Plan make_plan(Ctx& ctx, unsigned n, const qpeps_options& o, unsigned fre
   else
     fail(QPEPS_ERR_INVALID, "key_bits must be 0, 64 or 128");
   if (p.key_bits == 64 && n > narrow_max) fail(QPEPS_ERR_RANGE, "packed boundary does not fit a u64 key for this N");
-  if (o.device_budget_bytes)
-    p.budget = (size_t)o.device_budget_bytes;
-  else {
-    size_t fr = 0, tot = 0;
-    cuda_check(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo");
-    p.budget = (size_t)((double)(fr + ctx.pool_bytes) * 0.90);
-  }
+  p.budget = o.device_budget_bytes ? Budget((size_t)o.device_budget_bytes) : Budget(ctx);
   p.threads = o.block_threads ? (int)o.block_threads : 256;
   const bool partition_ok = (p.key_bits == 64 || p.key_bits == 128) && p.grain == QPEPS_GRAIN_ROW;
   if (o.merge == QPEPS_MERGE_PARTITION && !partition_ok)
@@ -1773,10 +1817,7 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
   const size_t cursor_bytes = (size_t)parts_cap * 4 * cstride;
   const size_t table_bytes = region_bytes + (cursor_bytes + 255) / 256 * 256;
   const size_t eb = entry_bytes(p);
-  if (count < 2 || f.count > most || std::max<u64>(f.cap, most) * eb + table_bytes + (1u << 20) > p.budget) return 0;
-  if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
-  if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes)) return 0;
-  if (ctx.pool_bytes - ctx.table.bytes + table_bytes > p.budget) return 0;
+  if (count < 2 || f.count > most || !chain_buffers(ctx, p, f, most, table_bytes)) return 0;
   buf_reserve(ctx, ctx.table, table_bytes, p.budget, "partition regions");
   StepScalars* d = queue_scalars(ctx, p, count);
   StepScalars* h = ctx.h_queue;
@@ -1862,11 +1903,7 @@ static void explicit_frontier(Ctx& ctx, unsigned n, unsigned order, u64 support_
   p.key_bits = 128;
   p.grain = QPEPS_GRAIN_SITE;
   p.merge = QPEPS_MERGE_HASH;
-  {
-    size_t fr = 0, tot = 0;
-    cuda_check(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo");
-    p.budget = (size_t)((double)(fr + ctx.pool_bytes) * 0.90);
-  }
+  p.budget = Budget(ctx);
   p.threads = 256;
   p.tail_row = n;
   const size_t eb = entry_bytes(p);
@@ -2546,13 +2583,14 @@ static void contract_impl(Ctx& ctx, unsigned n, const qpeps_options& o, const ui
   // frontier at its peak and spilling it to the host.
   if (o.slice_depth == 0 && out.plan.grain == QPEPS_GRAIN_ROW && row0 < n && !items.empty()) {
     const double per_state = 2.0 * (double)entry_bytes(out.plan) + 1.25 * (double)cand_bytes(out.plan);
-    const double cap_states = 0.8 * (double)out.plan.budget / per_state;
     // A placed prefix's frontier is estimated from the average over all
     // prefixes of its depth; central prefixes run to several times that (N=22:
     // 1.8-2.6x at depth 3), and an underestimate costs host spills at the peak
     // rows, so prefixes are sliced on four times the estimate.
     double est_total = serve_estimate(n, k) * (k ? 4.0 : 1.0);
-    while (est_total > cap_states && row0 + 2 < n) {
+    const bool fits = out.plan.budget.holds((size_t)std::min(1e18, est_total * per_state / 0.8));
+    const double cap_states = fits ? est_total : 0.8 * (double)(size_t)out.plan.budget / per_state;
+    while (!fits && est_total > cap_states && row0 + 2 < n) {
       // Slices are uneven (centre columns carry more states): tuned margin.
       const double est_item = est_total / (double)items.size() * ctx.tune.slice_margin;
       if (est_item <= cap_states) {
@@ -2864,7 +2902,7 @@ static void serve_batch_loop(Server& sv) {
   p.key_bits = 64;
   p.grain = QPEPS_GRAIN_ROW;
   p.merge = QPEPS_MERGE_PARTITION;
-  p.budget = (size_t)sv.cfg.batch_budget_bytes;
+  p.budget = Budget((size_t)sv.cfg.batch_budget_bytes);
   p.threads = 256;
   p.tail_row = p.n;
   const size_t eb = entry_bytes(p);
