@@ -845,7 +845,10 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
               dup_bits |= (u32)(!fresh) << l;
               break;
             }
-            slot = (slot + 1) & (H - 1);
+            // A step of the key's own (odd: it reaches every slot). The warp
+            // waits for its longest probe sequence, and steps of one run into
+            // each other's clusters.
+            slot = (slot + ((u32)(fib_hash_b(c.key) >> 32) | 1u)) & (H - 1);
           }
         }
       }

@@ -361,7 +361,8 @@ __global__ void __launch_bounds__(BLOCK, 2) wide_merge_kernel(const WCand<R>* __
         const u128 key = buf[l].key;
         // The partition index takes the hash's top bits; the slot re-mixes
         // the whole hash so keys of one partition spread over the table.
-        slot = (u32)(fib_hash_b(key_hash<u128>(key)) >> (64 - kLogH));
+        const u64 hash = fib_hash_b(key_hash<u128>(key));
+        slot = (u32)(hash >> (64 - kLogH));
         for (int probe = 0; probe < H; ++probe) {
           const u128 cur = wscas(&s_key[slot], kWEmpty, key);
           if (cur == kWEmpty || cur == key) {
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__(BLOCK, 2) wide_merge_kernel(const WCand<R>* __
             dup_bits |= (u32)(!fresh) << l;
             break;
           }
-          slot = (slot + 1) & (H - 1);
+          slot = (slot + ((u32)(hash >> 32) | 1u)) & (H - 1);  // (a step of the key's own)
         }
       }
       slots[l] = slot;
