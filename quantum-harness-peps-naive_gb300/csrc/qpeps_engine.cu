@@ -2891,6 +2891,102 @@ static bool serve_seeds(unsigned n, const std::vector<uint32_t>& prefix, std::ve
 // more states); admission reserves this multiple of the estimate.
 constexpr double kAdmitMargin = 2.5;
 
+// Steps a shared batch takes between looking at its queue: new requests wait
+// for a chain's end, so a chain is short.
+constexpr unsigned kServeChain = 6;
+
+// Up to `want` rows of the shared boundary (f, with `terms` successor terms,
+// both updated): a chain of queued steps while it is small, one step with the
+// host's sizes otherwise. Returns the rows contracted (at least one).
+static unsigned serve_steps(Ctx& ctx, const Plan& p, DevFrontier& f, u64& terms, unsigned want, const u64* d_mask,
+                            unsigned long long* d_final) {
+  if (terms == 0) {  // no state has a successor: nothing is left to add
+    f.count = 0;
+    cuda_check(cudaStreamSynchronize(ctx.stream), "serve synchronize");  // (seeds may still be on their way)
+    return want;
+  }
+  const u32 shape = 2;  // small merge CTAs, as in run_queued_rows
+  const u32 pcap = partition_capacity(shape);
+  double mean = ctx.partition_fill * pcap;
+  StepSource source{nullptr, mean, 0, 8 * (u32)ctx.sms};
+  if (want > 1 && terms <= kQueueTerms) {
+    // A row multiplies the terms by less than 4 on average once three rows are
+    // placed; a chain that outgrows its buffers stops and is sized below.
+    const u64 most = std::min<u64>(kQueueTerms, std::max<u64>(1u << 20, 4 * terms));
+    const u32 parts_cap = source.parts_cap = (u32)source.partitions(most);
+    const size_t region_bytes = (size_t)parts_cap * pcap * cand_bytes(p);
+    const size_t cursor_bytes = (size_t)parts_cap * 4 * 8;
+    const size_t table_bytes = region_bytes + (cursor_bytes + 255) / 256 * 256;
+    if (chain_buffers(ctx, p, f, most, table_bytes)) {
+      buf_reserve(ctx, ctx.table, table_bytes, p.budget, "serve partitions");
+      StepScalars* d = queue_scalars(ctx, p, want);
+      StepScalars* h = ctx.h_queue;
+      h[0].out_count = f.count;
+      h[0].next_terms = terms;
+      u32* cursors = reinterpret_cast<u32*>(static_cast<char*>(ctx.table.ptr) + region_bytes);
+      const FrontierView view = view_of(p, ctx.front[0], f.cap);
+      PartitionCfg pc{2, ctx.sms, parts_cap, pcap, 2, 8, ctx.tune.parents_per_lane, shape, 1, 1, 2u};
+      cuda_check(cudaMemcpyAsync(d, h, (want + 1) * sizeof(StepScalars), cudaMemcpyHostToDevice, ctx.stream),
+                 "queued step scalars");
+      cuda_check(cudaMemsetAsync(cursors, 0, cursor_bytes, ctx.stream), "clear cursors");
+      u64 entries = f.count;
+      double likely = (double)terms;
+      for (unsigned i = 0; i < want; ++i) {
+        const u64 fits = (u64)std::min((double)most, likely);
+        pc.queued = source;
+        pc.queued.prev = d + i;
+        pc.parts = (u32)source.partitions(fits);
+        cuda_check(launch_serve_scatter(pc, view, std::max<u64>(entries, 1), d_mask, ctx.table.ptr, cursors, d + i + 1,
+                                        ctx.stream),
+                   "serve scatter");
+        cuda_check(launch_serve_merge(pc, ctx.table.ptr, cursors, view, d_mask, d_final, d + i + 1, ctx.stream),
+                   "serve merge");
+        entries = fits;
+        likely *= 4;
+      }
+      cuda_check(cudaMemcpyAsync(h, d, (want + 1) * sizeof(StepScalars), cudaMemcpyDeviceToHost, ctx.stream),
+                 "read step scalars");
+      cuda_check(cudaStreamSynchronize(ctx.stream), "serve chain");
+      unsigned done = 0;
+      while (done < want && !h[done + 1].error) ++done;
+      if (done) {
+        f.count = h[done].out_count;
+        terms = h[done].next_terms;
+      }
+      if (done < want && (h[done + 1].error & kErrBounds)) fail(QPEPS_ERR_CUDA, "serving: a bounds check failed");
+      if (done) return done;
+    }
+  }
+  for (int attempt = 0;; ++attempt) {
+    const u32 parts = (u32)std::max<u64>(1, (u64)((double)terms / mean) + 1);
+    const size_t region_bytes = (size_t)parts * pcap * cand_bytes(p);
+    const size_t table_bytes = region_bytes + ((size_t)parts * 4 + 255) / 256 * 256;
+    if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
+    if (!ensure_front(ctx, p, f, std::max<u64>(f.count, terms), ctx.table.ptr ? 0 : table_bytes))
+      fail(QPEPS_ERR_CAPACITY, "serving batch budget exceeded");
+    buf_reserve(ctx, ctx.table, table_bytes, p.budget, "serve partitions");
+    const FrontierView view = view_of(p, ctx.front[0], f.cap);
+    u32* cursors = reinterpret_cast<u32*>(static_cast<char*>(ctx.table.ptr) + region_bytes);
+    PartitionCfg pc{2, ctx.sms, parts, pcap, 2, 1, ctx.tune.parents_per_lane, shape, 1, 1, 2u};
+    cuda_check(cudaMemsetAsync(cursors, 0, (size_t)parts * 4, ctx.stream), "clear cursors");
+    cuda_check(cudaMemsetAsync(ctx.d_sc, 0, sizeof(StepScalars), ctx.stream), "clear scalars");
+    cuda_check(launch_serve_scatter(pc, view, f.count, d_mask, ctx.table.ptr, cursors, ctx.d_sc, ctx.stream),
+               "serve scatter");
+    cuda_check(launch_serve_merge(pc, ctx.table.ptr, cursors, view, d_mask, d_final, ctx.d_sc, ctx.stream),
+               "serve merge");
+    sync_scalars(ctx);
+    if (ctx.h_sc->error & kErrOverflow) {
+      if (attempt >= 4) fail(QPEPS_ERR_CAPACITY, "serving partition overflow persists");
+      mean *= 0.6;
+      continue;
+    }
+    if (ctx.h_sc->error) fail(QPEPS_ERR_CAPACITY, "serving device capacity error");
+    f.count = ctx.h_sc->out_count;
+    terms = ctx.h_sc->next_terms;
+    return 1;
+  }
+}
+
 static void serve_batch_loop(Server& sv) {
   Ctx& ctx = *sv.batch;
   cuda_check(cudaSetDevice(sv.device), "cudaSetDevice");
@@ -2905,6 +3001,7 @@ static void serve_batch_loop(Server& sv) {
   p.budget = Budget((size_t)sv.cfg.batch_budget_bytes);
   p.threads = 256;
   p.tail_row = p.n;
+  p.w64 = true;  // N <= 19: exact weights (19! < 2^63)
   const size_t eb = entry_bytes(p);
   buf_reserve(ctx, sv.slot_buf, kServeMaxSlots * 5 * sizeof(u64), p.budget, "serve slots");
   u64* d_mask = static_cast<u64*>(sv.slot_buf.ptr);
@@ -2912,14 +3009,30 @@ static void serve_batch_loop(Server& sv) {
   u64 h_mask[kServeMaxSlots] = {0};
   cuda_check(cudaMemsetAsync(sv.slot_buf.ptr, 0, kServeMaxSlots * 5 * sizeof(u64), ctx.stream), "clear slots");
   const double budget_states = (double)p.budget / (2.4 * (double)eb);
-  std::vector<u64> seed_keys;
-  std::vector<uint32_t> seed_res;
+  std::vector<u64> seed_keys, seed_weights;
   std::vector<std::pair<State, u64>> seeds;
-  unsigned long long h_final[kServeMaxSlots * 4];
+  u64 seed_terms = 0;
+  u64 next_terms = 0;  // successor terms of the shared boundary
+  // Finished boards' sums on the device grow on; a request's count is what its
+  // slot's sum grew by.
+  unsigned long long h_base[kServeMaxSlots] = {0};
+  unsigned long long* h_final = nullptr;  // pinned: the sums, then seed staging
+  uint8_t* h_stage = nullptr;
+  struct Pinned {
+    void* p = nullptr;
+    ~Pinned() {
+      if (p) cudaFreeHost(p);
+    }
+  } pinned;
+  cuda_check(cudaMallocHost(&pinned.p, kServeMaxSlots * 4 * sizeof(u64) + kSeedStage), "pinned serve buffers");
+  h_final = static_cast<unsigned long long*>(pinned.p);
+  h_stage = reinterpret_cast<uint8_t*>(h_final + kServeMaxSlots * 4);
+  std::memset(h_final, 0, kServeMaxSlots * 4 * sizeof(u64));
   while (true) {
     // Admission.
     seed_keys.clear();
-    seed_res.clear();
+    seed_weights.clear();
+    seed_terms = 0;
     bool mask_dirty = false;
     {
       std::unique_lock<std::mutex> lk(sv.mu);
@@ -2967,15 +3080,17 @@ static void serve_batch_loop(Server& sv) {
           h_mask[free_slot] = (1ull << r.n) - 1;
           mask_dirty = true;
           for (auto& sd : seeds) {
-            seed_keys.push_back(serve_key((unsigned)free_slot, sd.first.cols, sd.first.dr, sd.first.dl));
-            seed_res.push_back((uint32_t)(sd.second % kPrimes[0]));
-            seed_res.push_back((uint32_t)(sd.second % kPrimes[1]));
+            const State& st = sd.first;
+            seed_keys.push_back(serve_key((unsigned)free_slot, st.cols, st.dr, st.dl));
+            seed_weights.push_back(sd.second);
+            seed_terms += (u64)__builtin_popcountll(~(st.cols | st.dr | st.dl) & h_mask[free_slot]);
           }
           any = true;
         }
         lk.lock();
       }
     }
+    unsigned steps = 0;
     try {
       if (mask_dirty)
         cuda_check(cudaMemcpyAsync(d_mask, h_mask, sizeof h_mask, cudaMemcpyHostToDevice, ctx.stream), "slot masks");
@@ -2984,62 +3099,38 @@ static void serve_batch_loop(Server& sv) {
         const u64 m = seed_keys.size();
         if (!ensure_front(ctx, p, sv.f, sv.f.count + m, ctx.table.bytes))
           fail(QPEPS_ERR_CAPACITY, "serving batch budget cannot hold the admitted seeds");
+        // (At most 64 requests of at most 19 seeds: the staging holds them.)
         char* base = static_cast<char*>(ctx.front[0].ptr);
-        cuda_check(cudaMemcpyAsync(base + sv.f.count * 8, seed_keys.data(), m * 8, cudaMemcpyHostToDevice, ctx.stream),
-                   "seed keys");
-        std::vector<uint32_t> plane(m);
-        for (int r = 0; r < 2; ++r) {
-          for (u64 i = 0; i < m; ++i) plane[i] = seed_res[2 * i + r];
-          cuda_check(cudaMemcpyAsync(base + sv.f.cap * 8 + ((size_t)r * sv.f.cap + sv.f.count) * 4, plane.data(), m * 4,
-                                     cudaMemcpyHostToDevice, ctx.stream),
-                     "seed residues");
-          cuda_check(cudaStreamSynchronize(ctx.stream), "seed upload");
+        u64* st_key = reinterpret_cast<u64*>(h_stage);
+        u32* st_word = reinterpret_cast<u32*>(st_key + m);
+        static_assert(kServeMaxSlots * 19 * 16 <= kSeedStage, "seed staging");
+        for (u64 i = 0; i < m; ++i) {
+          st_key[i] = seed_keys[i];
+          st_word[i] = (u32)seed_weights[i];
+          st_word[m + i] = (u32)(seed_weights[i] >> 32);
         }
+        cuda_check(cudaMemcpyAsync(base + sv.f.count * 8, st_key, m * 8, cudaMemcpyHostToDevice, ctx.stream),
+                   "seed keys");
+        for (int r = 0; r < 2; ++r)
+          cuda_check(cudaMemcpyAsync(base + sv.f.cap * 8 + ((size_t)r * sv.f.cap + sv.f.count) * 4, st_word + r * m,
+                                     m * 4, cudaMemcpyHostToDevice, ctx.stream),
+                     "seed weights");
         sv.f.count += m;
+        next_terms += seed_terms;
       }
       bool active = false;
-      for (const ServeSlot& sl : sv.slots) active = active || sl.used;
-      if (!active) continue;
-      // One row for every admitted request.
-      StepScalars* sc = ctx.d_sc;
-      cuda_check(cudaMemsetAsync(sc, 0, sizeof(StepScalars), ctx.stream), "clear scalars");
-      FrontierView view = view_of(p, ctx.front[0], sv.f.cap);
-      cuda_check(launch_serve_count(view, sv.f.count, d_mask, sc, ctx.sms, ctx.stream), "serve count");
-      sync_scalars(ctx);
-      const u64 terms = ctx.h_sc->terms;
-      if (terms > 0) {
-        const u32 pcap = partition_capacity();
-        double mean = ctx.partition_fill * pcap;
-        for (int attempt = 0;; ++attempt) {
-          const u32 parts = (u32)std::max<u64>(1, (u64)((double)terms / mean) + 1);
-          const size_t region_bytes = (size_t)parts * pcap * candidate_bytes(2);
-          const size_t table_bytes = region_bytes + ((size_t)parts * 4 + 255) / 256 * 256;
-          if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
-          if (!ensure_front(ctx, p, sv.f, std::max<u64>(sv.f.count, terms), ctx.table.ptr ? 0 : table_bytes))
-            fail(QPEPS_ERR_CAPACITY, "serving batch budget exceeded");
-          buf_reserve(ctx, ctx.table, table_bytes, p.budget, "serve partitions");
-          view = view_of(p, ctx.front[0], sv.f.cap);
-          uint32_t* cursors = reinterpret_cast<uint32_t*>(static_cast<char*>(ctx.table.ptr) + region_bytes);
-          PartitionCfg pc{2, ctx.sms, parts, pcap, 2, 1, ctx.tune.parents_per_lane, 0, ctx.tune.scatter_kind,
-                          ctx.tune.merge_kind, ctx.tune.fold_weights ? 1u : 0u};  // serving: N <= 19
-          cuda_check(cudaMemsetAsync(cursors, 0, (size_t)parts * 4, ctx.stream), "clear cursors");
-          cuda_check(cudaMemsetAsync(sc, 0, sizeof(StepScalars), ctx.stream), "clear scalars");
-          cuda_check(launch_serve_scatter(pc, view, sv.f.count, d_mask, ctx.table.ptr, cursors, sc, ctx.stream),
-                     "serve scatter");
-          cuda_check(launch_serve_merge(pc, ctx.table.ptr, cursors, view, d_mask, d_final, sc, ctx.stream),
-                     "serve merge");
-          sync_scalars(ctx);
-          if (ctx.h_sc->error & kErrOverflow) {
-            if (attempt >= 4) fail(QPEPS_ERR_CAPACITY, "serving partition overflow persists");
-            mean *= 0.6;
-            continue;
-          }
-          if (ctx.h_sc->error) fail(QPEPS_ERR_CAPACITY, "serving device capacity error");
-          break;
+      unsigned first_end = ~0u;  // rows until the first request ends
+      for (const ServeSlot& sl : sv.slots)
+        if (sl.used) {
+          active = true;
+          first_end = std::min(first_end, sl.rows_left);
         }
-        sv.f.count = ctx.h_sc->out_count;
-      } else {
-        sv.f.count = 0;
+      if (!active) continue;
+      steps = serve_steps(ctx, p, sv.f, next_terms, std::min(first_end, kServeChain), d_mask, d_final);
+      if (steps == first_end) {
+        cuda_check(cudaMemcpyAsync(h_final, d_final, kServeMaxSlots * 4 * sizeof(u64), cudaMemcpyDeviceToHost, ctx.stream),
+                   "slot finals");
+        cuda_check(cudaStreamSynchronize(ctx.stream), "slot finals");
       }
     } catch (const Failure& e) {
       if (e.code != QPEPS_ERR_CAPACITY) throw;
@@ -3062,6 +3153,8 @@ static void serve_batch_loop(Server& sv) {
         h_mask[i] = 0;
       }
       sv.f.count = 0;
+      next_terms = 0;
+      std::memset(h_base, 0, sizeof h_base);
       buf_release(ctx, ctx.table);
       cuda_check(cudaMemsetAsync(sv.slot_buf.ptr, 0, kServeMaxSlots * 5 * sizeof(u64), ctx.stream), "clear slots");
       cuda_check(cudaStreamSynchronize(ctx.stream), "clear slots");
@@ -3076,21 +3169,18 @@ static void serve_batch_loop(Server& sv) {
     }
     {
       std::lock_guard<std::mutex> lk(sv.mu);
-      sv.stats.batch_steps += 1;
+      sv.stats.batch_steps += steps;
     }
     // Finished requests.
     bool any_done = false;
     for (ServeSlot& sl : sv.slots)
-      if (sl.used && --sl.rows_left == 0) any_done = true;
+      if (sl.used && (sl.rows_left -= steps) == 0) any_done = true;
     if (!any_done) continue;
-    cuda_check(cudaMemcpyAsync(h_final, d_final, sizeof h_final, cudaMemcpyDeviceToHost, ctx.stream), "slot finals");
-    cuda_check(cudaStreamSynchronize(ctx.stream), "slot finals");
     for (unsigned i = 0; i < kServeMaxSlots; ++i) {
       ServeSlot& sl = sv.slots[i];
       if (!sl.used || sl.rows_left != 0) continue;
-      u64 res[2] = {h_final[i * 4 + 0] % kPrimes[0], h_final[i * 4 + 1] % kPrimes[1]};
-      const u128 count = crt_reconstruct(res, 2);
-      cuda_check(cudaMemsetAsync(d_final + i * 4, 0, 4 * sizeof(u64), ctx.stream), "reset slot");
+      const u128 count = h_final[i * 4] - h_base[i];
+      h_base[i] = h_final[i * 4];
       h_mask[i] = 0;
       sl.used = false;
       {

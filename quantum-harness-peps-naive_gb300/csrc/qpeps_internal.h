@@ -302,12 +302,10 @@ struct ResidentArgs {
 uint32_t resident_capacity();
 cudaError_t launch_resident_rows(const ResidentArgs& a, cudaStream_t stream);
 
-// Serving (slotted keys, R = 2): count, scatter and merge of a boundary
-// shared by requests of different board sizes. slot_mask[s] is the board mask
-// of the request in slot s; finished boards are summed into
-// slot_final[s * 4 + r] and leave the boundary.
-cudaError_t launch_serve_count(const FrontierView& in, uint64_t n_in, const uint64_t* slot_mask, StepScalars* sc,
-                               int sms, cudaStream_t stream);
+// Serving (slotted keys, exact 64-bit weights in two planes): scatter and merge
+// of a boundary shared by requests of different board sizes. slot_mask[s] is
+// the board mask of the request in slot s; finished boards are summed into
+// slot_final[s * 4] and leave the boundary.
 cudaError_t launch_serve_scatter(const PartitionCfg& pc, const FrontierView& in, uint64_t n_in,
                                  const uint64_t* slot_mask, void* regions, uint32_t* cursors, StepScalars* sc,
                                  cudaStream_t stream);

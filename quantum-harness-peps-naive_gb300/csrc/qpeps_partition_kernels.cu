@@ -517,9 +517,9 @@ __device__ __forceinline__ unsigned long long next_terms_of(const FixedLayout& L
   const State st = L.unpack(key);
   return (unsigned long long)__popcll(~(st.cols | st.dr | st.dl) & L.mask);
 }
-template <typename Layout>
-__device__ __forceinline__ unsigned long long next_terms_of(const Layout&, u64) {
-  return 0ull;
+__device__ __forceinline__ unsigned long long next_terms_of(const SlotLayout& L, u64 key) {
+  const State st = L.unpack(key);
+  return (unsigned long long)__popcll(~(st.cols | st.dr | st.dl) & L.mask_of(key));
 }
 
 template <int R, int BLOCK, int H, int CAP, typename Layout>
@@ -760,7 +760,6 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
   static_assert(CAP % BLOCK == 0, "shape");
   constexpr bool kFold = kAcc != 0;  // one 64-bit accumulator plane
   static_assert(!kFold || R == 2, "the one-plane accumulators hold a residue pair or a weight's two words");
-  static_assert(kAcc != 2 || !Layout::kSlotted, "exact weights are not used by the serving layout");
   static_assert(!kRegs || !Layout::kSlotted, "register compaction is for the fixed layout");
   constexpr int AP = kFold ? 1 : R;  // accumulator planes
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -769,10 +768,11 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
   u32* s_list = reinterpret_cast<u32*>(smem_raw + sizeof(u64) * H * (1 + AP));                   // [CAP]
   __shared__ u32 s_nused, s_n;
   __shared__ unsigned long long s_base;
-  __shared__ unsigned long long s_slot_fin[Layout::kSlotted ? kServeMaxSlots * R : 1];
+  constexpr int SF = kAcc == 2 ? 1 : R;  // sums of a finished board: the exact weight, or its residues
+  __shared__ unsigned long long s_slot_fin[Layout::kSlotted ? kServeMaxSlots * SF : 1];
   const int lane = threadIdx.x & 31;
   if constexpr (Layout::kSlotted)
-    for (int i = threadIdx.x; i < (int)kServeMaxSlots * R; i += BLOCK) s_slot_fin[i] = 0ull;
+    for (int i = threadIdx.x; i < (int)kServeMaxSlots * SF; i += BLOCK) s_slot_fin[i] = 0ull;
   next_kernel_may_start();
   for (int i = threadIdx.x; i < H; i += BLOCK) s_key[i] = kEmpty;
   if (threadIdx.x == 0) s_nused = 0;
@@ -792,7 +792,7 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
   // The written boundary's successor terms at the next row (the next row
   // step's count, so that it needs no counting pass of its own).
   unsigned long long nterms = 0;
-  constexpr bool kCountNext = !Layout::kSlotted;
+  constexpr bool kCountNext = true;
   bool bad = false;  // an output index beyond the boundary buffer (skipped)
 #pragma unroll
   for (int r = 0; r < R; ++r) wsum[r] = fsum[r] = 0;
@@ -825,17 +825,42 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
       const u32 i = l * BLOCK + threadIdx.x;
       bool fresh = false;
       u32 slot = 0;
-      if (i < bcnt) {
-        const Cand<R>& c = buf[l];
-        bool finished = false;
-        if constexpr (Layout::kSlotted) {
-          const u64 m = L.mask_of(c.key);
-          if ((c.key & m) == m) {
+      bool finished = false;
+      if constexpr (Layout::kSlotted) {
+        // Finished boards leave the boundary. The rows in which a request's
+        // boards finish add them all to one sum: a warp adds up those of one
+        // request (and of a second one) before its atomic.
+        if (i < bcnt) {
+          const u64 m = L.mask_of(buf[l].key);
+          finished = (buf[l].key & m) == m;
+        }
+        u32 left = __ballot_sync(kFullMask, finished);
+        const u32 mine = finished ? L.slot(buf[l].key) : 0xffffffffu;
+        for (int round = 0; round < 2 && left; ++round) {
+          const int leader = __ffs(left) - 1;
+          const u32 of = __shfl_sync(kFullMask, mine, leader);
+          const bool in = finished && mine == of && ((left >> lane) & 1u);
+          left &= ~__ballot_sync(kFullMask, in);
 #pragma unroll
-            for (int r = 0; r < R; ++r) atomicAdd(&s_slot_fin[L.slot(c.key) * R + r], (unsigned long long)c.res[r]);
-            finished = true;
+          for (int r = 0; r < SF; ++r) {
+            unsigned long long v = !in ? 0ull
+                                   : kAcc == 2 ? one_plane<2>(buf[l].res[0], buf[l].res[R > 1 ? 1 : 0])
+                                               : (unsigned long long)buf[l].res[r];
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFullMask, v, d);
+            if (lane == leader) atomicAdd(&s_slot_fin[of * SF + r], v);
           }
         }
+        if ((left >> lane) & 1u) {
+#pragma unroll
+          for (int r = 0; r < SF; ++r)
+            atomicAdd(&s_slot_fin[mine * SF + r],
+                      kAcc == 2 ? one_plane<2>(buf[l].res[0], buf[l].res[R > 1 ? 1 : 0])
+                                : (unsigned long long)buf[l].res[r]);
+        }
+      }
+      if (i < bcnt) {
+        const Cand<R>& c = buf[l];
         if (!finished) {
           slot = (u32)(fib_hash_b(c.key) >> (64 - kLogH));
           for (int probe = 0; probe < H; ++probe) {
@@ -1010,23 +1035,9 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
   }
   if constexpr (Layout::kSlotted) {
     __syncthreads();
-    for (int i = threadIdx.x; i < (int)kServeMaxSlots * R; i += BLOCK)
-      if (s_slot_fin[i]) atomicAdd(&L.slot_final[(i / R) * 4 + (i % R)], s_slot_fin[i]);
+    for (int i = threadIdx.x; i < (int)kServeMaxSlots * SF; i += BLOCK)
+      if (s_slot_fin[i]) atomicAdd(&L.slot_final[(i / SF) * 4 + (i % SF)], s_slot_fin[i]);
   }
-}
-
-// Successor count of a slotted (serving) boundary.
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) slot_count_kernel(const u64* __restrict__ keys, u64 n_in, SlotLayout L,
-                                                           StepScalars* __restrict__ sc) {
-  unsigned long long acc = 0;
-  for (u64 i = (u64)blockIdx.x * BLOCK + threadIdx.x; i < n_in; i += (u64)gridDim.x * BLOCK) {
-    const u64 key = keys[i];
-    const State s = L.unpack(key);
-    acc += __popcll(~(s.cols | s.dr | s.dl) & L.mask_of(key));
-  }
-  const unsigned long long t = pblock_sum<BLOCK>(acc);
-  if (threadIdx.x == 0 && t) atomicAdd(&sc->terms, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -1430,7 +1441,7 @@ cudaError_t scatter_impl(const PartitionCfg& pc, const FrontierView& in, u64 n_i
                          u32* cursors, StepScalars* sc, cudaStream_t stream) {
   // A boundary that leaves the chip short of warps at four parents a lane
   // (fewer than about 8 blocks an SM) takes one a lane in small blocks.
-  if (!Layout::kSlotted && pc.scatter_kind == 1 && n_in <= (u64)pc.sms * 2048)
+  if (pc.scatter_kind == 1 && n_in <= (u64)pc.sms * 2048)
     return scatter_shape<R, 1, 128, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
   if (pc.parents_per_lane == 4) return scatter_ppl<R, 4, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
   return scatter_ppl<R, 2, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
@@ -1443,14 +1454,12 @@ cudaError_t merge_shape(const PartitionCfg& pc, int blocks_per_sm, const void* r
   const bool fold = R == 2 && pc.merge_kind == 1 && pc.fold;
   const bool exact = fold && pc.fold == 2;
   if (pc.fold == 2 && !exact) return cudaErrorInvalidValue;  // exact words need the claim-list merge
-  if constexpr (Layout::kSlotted)
-    if (exact) return cudaErrorInvalidValue;
   constexpr bool kRegsOk = !Layout::kSlotted;
   const bool regs = kRegsOk && pc.merge_regs;
   auto kern = fold ? (exact ? (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout,
-                                                                  (R == 2 && !Layout::kSlotted) ? 2 : 0, kRegsOk>
+                                                                  R == 2 ? 2 : 0, kRegsOk>
                                     : partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout,
-                                                                  (R == 2 && !Layout::kSlotted) ? 2 : 0>)
+                                                                  R == 2 ? 2 : 0>)
                             : (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, R == 2 ? 1 : 0, kRegsOk>
                                     : partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, R == 2 ? 1 : 0>))
                    : (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, 0, kRegsOk>
@@ -1495,16 +1504,6 @@ cudaError_t merge_impl(const PartitionCfg& pc, const void* regions, const u32* c
 }  // namespace
 
 size_t candidate_bytes(int residues) { return residues <= 2 ? 16 : 32; }
-
-cudaError_t launch_serve_count(const FrontierView& in, uint64_t n_in, const uint64_t* slot_mask, StepScalars* sc,
-                               int sms, cudaStream_t stream) {
-  if (n_in == 0) return cudaSuccess;
-  const u64 want = (n_in + 1023) / 1024;
-  const unsigned grid = (unsigned)std::max<u64>(1, std::min<u64>(want, (u64)sms * 8));
-  slot_count_kernel<256><<<grid, 256, 0, stream>>>(reinterpret_cast<const u64*>(in.keys), n_in,
-                                                   SlotLayout{slot_mask, nullptr}, sc);
-  return cudaGetLastError();
-}
 
 cudaError_t launch_serve_scatter(const PartitionCfg& pc, const FrontierView& in, uint64_t n_in,
                                  const uint64_t* slot_mask, void* regions, uint32_t* cursors, StepScalars* sc,
