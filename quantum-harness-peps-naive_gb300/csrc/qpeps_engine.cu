@@ -1056,7 +1056,11 @@ static StepScalars* pinned_scalars(Ctx& ctx, size_t steps) {
 // The same with their copy on the device.
 static StepScalars* queue_scalars(Ctx& ctx, const Plan& p, size_t steps) {
   pinned_scalars(ctx, steps);
+  // No captured graph holds this buffer (a replay has scalars of its own), so
+  // its growth does not end one.
+  const uint64_t gen = ctx.pool_gen;
   buf_reserve(ctx, ctx.queue, (steps + 1) * sizeof(StepScalars), p.budget, "queued step scalars");
+  ctx.pool_gen = gen;
   return static_cast<StepScalars*>(ctx.queue.ptr);
 }
 
