@@ -287,6 +287,7 @@ enum ErrorBits : u32 {
   kErrBounds = 8u,      // an index fell outside its buffer; the access was skipped
   kErrSkipped = 16u,    // queued step: an earlier step of the chain failed
   kErrCapacity = 32u,   // queued step: its terms do not fit the buffers
+  kErrNeedWide = 64u,   // grouped row: its weights may pass 32 bits
 };
 
 #if defined(__CUDACC__)

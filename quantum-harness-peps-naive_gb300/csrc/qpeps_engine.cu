@@ -301,6 +301,10 @@ struct Ctx {
     uint32_t slice_rows = 1;                    // rows enumerated on the host before slicing is considered
   } tune;
   DevBuf tail;                   // TailControl + overflow list
+  DevBuf grp_side[2];            // column-grouped rows: the two boundaries' keys and weights
+  DevBuf grp_dir;                // group and bucket directories, unit list, row scalars, binomials, seed
+  void* grp_pin = nullptr;       // pinned: row scalars read back, seed uploads
+  size_t grp_pin_bytes = 0;
   DevBuf plan;                   // class-grouped partitions: histogram, bucket table, scan partials
   DevBuf queue;                  // queued steps: their scalars
   StepScalars* h_queue = nullptr;  // pinned: the scalars as uploaded, then as read back
@@ -349,14 +353,30 @@ static void buf_release(Ctx& ctx, DevBuf& b) {
   b.bytes = 0;
 }
 
+// The column-grouped rows' buffers hold nothing between calls: another
+// buffer that does not fit beside them takes their room.
+static bool group_release(Ctx& ctx) {
+  bool any = false;
+  for (DevBuf* b : {&ctx.grp_side[0], &ctx.grp_side[1], &ctx.grp_dir}) {
+    any = any || b->ptr;
+    buf_release(ctx, *b);
+  }
+  return any;
+}
+
 static void buf_reserve(Ctx& ctx, DevBuf& b, size_t bytes, const Budget& budget, const char* what) {
   if (b.bytes >= bytes) return;
   size_t want = bytes + bytes / 4;
   if (ctx.pool_bytes - b.bytes + want > budget) want = bytes;
+  if (ctx.pool_bytes - b.bytes + want > budget) group_release(ctx);
   if (ctx.pool_bytes - b.bytes + want > budget)
     fail(QPEPS_ERR_CAPACITY, std::string("device budget exceeded by ") + what);
   buf_release(ctx, b);
   cudaError_t e = cudaMalloc(&b.ptr, want);
+  if (e != cudaSuccess && group_release(ctx)) {
+    cudaGetLastError();
+    e = cudaMalloc(&b.ptr, want);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     fail(QPEPS_ERR_CAPACITY, std::string("device allocation failed for ") + what);
@@ -379,6 +399,8 @@ static void ctx_free(Ctx* ctx) {
   buf_release(*ctx, ctx->tail);
   buf_release(*ctx, ctx->plan);
   buf_release(*ctx, ctx->queue);
+  group_release(*ctx);
+  if (ctx->grp_pin) cudaFreeHost(ctx->grp_pin);
   if (ctx->h_queue) cudaFreeHost(ctx->h_queue);
   if (ctx->h_seed) cudaFreeHost(ctx->h_seed);
   if (ctx->d_sc) cudaFree(ctx->d_sc);
@@ -455,6 +477,7 @@ struct Plan {
   unsigned tail_row;  // rows >= tail_row go to the slice-tail kernel (n = none)
   bool prefix = false;      // a partly placed board
   double batch_states = 0;  // expected largest boundary of one device batch (0: unknown)
+  double group_states = 0;  // column-grouped rows: expected largest boundary of a device batch (0: not used)
   bool w64 = false;   // residue planes 0/1 hold the low/high words of exact weights (partitioned row merge)
   int Rc = 0;         // residues of the CRT bookkeeping (= R except with w64, where R = 2 planes)
 };
@@ -559,8 +582,13 @@ static bool ensure_front(Ctx& ctx, const Plan& p, DevFrontier& f, u64 need, size
   const size_t live = ctx.front[0].bytes;
   if (live + want * eb + other_bytes > p.budget) want = need;
   if (live + want * eb + other_bytes > p.budget) return false;
+  if (ctx.pool_bytes + want * eb + other_bytes > p.budget) group_release(ctx);
   DevBuf nb;
   cudaError_t e = cudaMalloc(&nb.ptr, want * eb);
+  if (e != cudaSuccess && group_release(ctx)) {
+    cudaGetLastError();
+    e = cudaMalloc(&nb.ptr, want * eb);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return false;
@@ -1424,6 +1452,343 @@ static u64 run_queued_sites_plain(Ctx& ctx, const Plan& p, DevFrontier& f, unsig
   return done;
 }
 
+// ---- column-grouped rows (qpeps_group_kernels.cu) ---------------------------
+//
+// All rows of a device batch are queued at once: a row's plan and pull read
+// the sizes they need from the previous row's scalars on the device, so the
+// host waits once, at the end. A row whose output does not fit its buffer
+// marks itself and the rows after it return at once; the host grows the buffer
+// to the size the row counted and queues the rows again from there, the row's
+// input being untouched.
+
+struct GroupBinomials {
+  u32 v[(kGroupMaxN + 2) * (kGroupMaxN + 2)];
+  GroupBinomials() {
+    constexpr unsigned d = kGroupMaxN + 2;
+    for (unsigned i = 0; i < d; ++i)
+      for (unsigned k = 0; k < d; ++k)
+        v[i * d + k] = k == 0 ? 1u : i == 0 ? 0u : v[(i - 1) * d + k] + v[(i - 1) * d + k - 1];
+  }
+  u32 at(unsigned i, unsigned k) const { return v[i * (kGroupMaxN + 2) + k]; }
+};
+static const GroupBinomials kBinomials;
+
+// A seed boundary in the grouped layout: packed entries and their buckets.
+struct GroupSeed {
+  std::vector<u32> keys, weights;
+  std::vector<GroupSeedUnit> units;
+  GroupRow row{};
+};
+
+// Host entries beyond this are not regrouped (halves of a boundary split off
+// under memory pressure): they take the partitioned merge.
+constexpr u64 kGroupMaxSeeds = 4096;
+
+// Expected largest boundary that column-grouped rows are to hold, 0 where the
+// partitioned rows are faster. Device ms at N = 15 / 16 / 17 / 18 (peaks of 18,
+// 106 and 706 M entries; nine batches of 380 to 743 M): grouped 2.25 / 10.8 /
+// 75.6 / 702, partitioned 2.43 / 15.6 / 117 / 821; at N = 14 (2.8 M) the
+// partitioned rows' traffic stays in L2 and the grouped ones' smallest units are
+// nearly empty. Repeated contractions (use_graph) keep the rows that a graph can
+// replay up to 200 M entries. `room`: the buffers' size over the expected one.
+static double group_rows_states(double states, double room, bool replay) {
+  return states >= (replay ? 200e6 : 10e6) ? states * room : 0.0;
+}
+
+static bool group_applies(const Ctx& ctx, const Plan& p, const HostChunk& hc) {
+  // Exact weights: two words (w64; the seed's high words are zero), or one
+  // residue below which every weight stays (R = 1: (N - k)! < p0). The
+  // claim-list merge and the window scatter stand for the default row step;
+  // other kinds of the tuning keep their own kernels.
+  const bool exact = p.w64 || (p.R == 1 && ctx.tune.fold_weights == 2 && ctx.tune.merge_kind == 1);
+  return p.group_states > 0 && exact && p.merge == QPEPS_MERGE_PARTITION && p.grain == QPEPS_GRAIN_ROW &&
+         p.key_bits == 64 && p.tail_row >= p.n && p.n <= kGroupMaxN && p.free_rows <= 20 &&
+         ctx.tune.scatter_kind == 1 && ctx.tune.merge_compact == 0 && hc.count > 0 && hc.count <= kGroupMaxSeeds &&
+         !hc.no_tail && hc.row >= 1 && hc.row < p.n &&
+         (p.R == 1 || std::all_of(hc.res.begin() + hc.count, hc.res.begin() + 2 * hc.count,
+                                  [](u32 high) { return high == 0; }));
+}
+
+// Top u bits implied by the bucket, so that the stored diagonals fit 32 bits.
+static unsigned group_implied_bits(unsigned n) { return 2 * n - 2 > 32 ? 2 * n - 2 - 32 : 0; }
+
+static GroupSeed group_seed(const Plan& p, const HostChunk& hc) {
+  const unsigned n = p.n, rm = group_implied_bits(n), nu = n - 1 - rm;
+  const u64 mask = (1ull << n) - 1;
+  struct E {
+    u64 cols;
+    u32 bucket, quarter, key, w;
+  };
+  std::vector<E> es(hc.count);
+  GroupSeed sd;
+  for (u64 i = 0; i < hc.count; ++i) {
+    u64 k;
+    std::memcpy(&k, &hc.keys[i * 8], 8);
+    const State st = unpack<u64>(k, n, mask);
+    E& e = es[i];
+    e.cols = st.cols;
+    e.bucket = (u32)(st.dr >> (n - rm));
+    e.quarter = (u32)(st.dr >> (n - 2 - rm)) & 3u;
+    e.key = (u32)((st.dr >> 1) & ((1ull << nu) - 1)) | (u32)(st.dl << nu);
+    e.w = hc.res[i];
+    sd.row.next_terms += (u64)__builtin_popcountll(~(st.cols | st.dr | st.dl) & mask);
+    sd.row.weight_sum += e.w;
+    sd.row.weight_max = std::max<unsigned long long>(sd.row.weight_max, e.w);
+  }
+  std::sort(es.begin(), es.end(), [](const E& a, const E& b) {
+    return a.cols != b.cols ? a.cols < b.cols : a.bucket != b.bucket ? a.bucket < b.bucket : a.quarter < b.quarter;
+  });
+  size_t group = 0;  // its first bucket in sd.units
+  for (u64 i = 0; i < hc.count; ++i) {
+    const E& e = es[i];
+    if (i == 0 || es[i - 1].cols != e.cols) {
+      u32 rank = 0, j = 0;
+      for (u64 left = e.cols; left; left &= left - 1) rank += kBinomials.at((unsigned)__builtin_ctzll(left), ++j);
+      group = sd.units.size();
+      for (u32 q = 0; q < (1u << rm); ++q)
+        sd.units.push_back(GroupSeedUnit{(u32)i, (u32)sd.units.size(), 0u, 0u, rank, rm, 0u});
+    }
+    GroupSeedUnit& un = sd.units[group + e.bucket];
+    if (!(un.quarters01 | un.quarters23)) un.first = (u32)i;
+    (e.quarter & 2u ? un.quarters23 : un.quarters01) += e.quarter & 1u ? 0x10000u : 1u;
+    sd.units[group].total += 1;
+    sd.keys.push_back(e.key);
+    sd.weights.push_back(e.w);
+  }
+  sd.row.out_count = hc.count;
+  sd.row.merge_rate = 1.f;
+  return sd;
+}
+
+constexpr size_t kGroupEntryBytes = 8;  // key, weight
+
+// Layout of Ctx::grp_dir.
+struct GroupDirs {
+  u32 groups = 0, unit_cap = 0;
+  size_t off_gdir[2], off_udir[2], off_units, off_rows, off_bin, off_list, bytes;
+};
+static GroupDirs group_dirs(unsigned n, unsigned row0, u64 cap, u64 seed_units) {
+  GroupDirs d;
+  for (unsigned m = row0; m <= n; ++m) d.groups = std::max(d.groups, kBinomials.at(n, m));
+  // A group takes 2^rm buckets at least; beyond that buckets are cut so that
+  // more than half the target is expected in each, and cut units add pieces.
+  const u64 most = ((u64)d.groups << group_implied_bits(n)) + (u64)(4.0 * (double)cap / group_unit_target()) + 65536 +
+                   seed_units;
+  d.unit_cap = (u32)std::min<u64>(most, 0x7fffffffu);
+  size_t o = 0;
+  auto take = [&](size_t b) {
+    const size_t at = o;
+    o += (b + 255) / 256 * 256;
+    return at;
+  };
+  for (int i = 0; i < 2; ++i) d.off_gdir[i] = take((size_t)d.groups * sizeof(GroupDir));
+  for (int i = 0; i < 2; ++i) d.off_udir[i] = take((size_t)d.unit_cap * sizeof(uint4));
+  d.off_units = take((size_t)d.unit_cap * sizeof(uint2));
+  d.off_rows = take((kGroupMaxN + 1) * sizeof(GroupRow));
+  d.off_bin = take(sizeof kBinomials.v);
+  d.off_list = take((size_t)std::max<u64>(seed_units, 1) * sizeof(GroupSeedUnit));
+  d.bytes = o;
+  return d;
+}
+
+// Grow-only, exact when the budget is near; false when it does not fit.
+static bool group_reserve(Ctx& ctx, DevBuf& b, size_t bytes, const Budget& budget) {
+  if (b.bytes >= bytes) return true;
+  if (ctx.pool_bytes - b.bytes + bytes > budget) buf_release(ctx, ctx.table);
+  if (ctx.pool_bytes - b.bytes + bytes > budget) buf_release(ctx, ctx.front[0]);
+  if (ctx.pool_bytes - b.bytes + bytes > budget) return false;
+  buf_release(ctx, b);
+  if (cudaMalloc(&b.ptr, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    b.ptr = nullptr;
+    return false;
+  }
+  b.bytes = bytes;
+  ctx.pool_bytes += bytes;
+  ctx.peak_pool_bytes = std::max(ctx.peak_pool_bytes, ctx.pool_bytes);
+  ++ctx.pool_gen;
+  return true;
+}
+
+// The row step's arguments from the buffers as they stand: boundaries
+// alternate sides, the seed (m = row0) on side 0.
+static GroupStepArgs group_args(const Ctx& ctx, const Plan& p, const GroupDirs& d, unsigned row0, unsigned m) {
+  char* base = static_cast<char*>(ctx.grp_dir.ptr);
+  auto side = [&](unsigned i) {
+    GroupSide s{};
+    s.cap = std::min<u64>(ctx.grp_side[i].bytes / kGroupEntryBytes, 0xfffffff0ull);
+    s.keys = static_cast<u32*>(ctx.grp_side[i].ptr);
+    s.lo = s.keys + s.cap;
+    s.gdir = reinterpret_cast<GroupDir*>(base + d.off_gdir[i]);
+    s.udir = reinterpret_cast<uint4*>(base + d.off_udir[i]);
+    s.unit_cap = d.unit_cap;
+    return s;
+  };
+  GroupStepArgs a{};
+  a.in = side((m - 1 - row0) & 1u);
+  a.out = side((m - row0) & 1u);
+  GroupRow* rows = reinterpret_cast<GroupRow*>(base + d.off_rows);
+  a.prev = rows + (m - 1);
+  a.row = rows + m;
+  a.units = reinterpret_cast<uint2*>(base + d.off_units);
+  a.binomials = reinterpret_cast<const u32*>(base + d.off_bin);
+  a.n = p.n;
+  a.m = m;
+  a.rm = group_implied_bits(p.n);
+  a.max_bits = std::min(12u, p.n - 4);
+  a.write_out = m < p.n;
+  a.block = group_block(p.group_states, ctx.sms);
+  a.target = group_unit_target();
+  return a;
+}
+
+static void* group_pinned(Ctx& ctx, size_t bytes) {
+  if (ctx.grp_pin_bytes < bytes) {
+    if (ctx.grp_pin) cudaFreeHost(ctx.grp_pin);
+    ctx.grp_pin = nullptr;
+    ctx.grp_pin_bytes = 0;
+    cuda_check(cudaMallocHost(&ctx.grp_pin, bytes + bytes / 2), "pinned row scalars");
+    ctx.grp_pin_bytes = bytes + bytes / 2;
+  }
+  return ctx.grp_pin;
+}
+
+// Contract one batch with column-grouped rows. False (and nothing added to
+// the metrics) where they do not apply or the budget does not hold them.
+static bool run_chunk_grouped(Ctx& ctx, const Plan& p, const HostChunk& hc, std::vector<RowAcc>& rows, RunStats& rs) {
+  if (!group_applies(ctx, p, hc)) return false;
+  const unsigned n = p.n, row0 = hc.row;
+  const auto t0 = std::chrono::steady_clock::now();
+  const GroupSeed sd = group_seed(p, hc);
+  const u64 cap = std::max<u64>(group_capacity(p.group_states, ctx.sms), hc.count);
+  if (cap > 0xfffffff0ull) return false;
+  const GroupDirs d = group_dirs(n, row0, std::max<u64>(cap, ctx.grp_side[0].bytes / kGroupEntryBytes), sd.units.size());
+  if (2 * cap * kGroupEntryBytes + d.bytes > p.budget) return false;
+  if (ctx.pool_bytes > p.budget) {
+    buf_release(ctx, ctx.table);
+    buf_release(ctx, ctx.front[0]);
+    if (ctx.pool_bytes > p.budget) group_release(ctx);
+  }
+  for (int i = 0; i < 2; ++i)
+    if (!group_reserve(ctx, ctx.grp_side[i], cap * kGroupEntryBytes, p.budget)) return false;
+  if (!group_reserve(ctx, ctx.grp_dir, d.bytes, p.budget)) return false;
+  // Upload the seed: one pinned image, its parts copied to their places.
+  const size_t ns = sd.keys.size();
+  const size_t seed_bytes = ns * 8 + sd.units.size() * sizeof(GroupSeedUnit);
+  const size_t rows_bytes = (kGroupMaxN + 1) * sizeof(GroupRow);
+  char* pin = static_cast<char*>(group_pinned(ctx, 2 * rows_bytes + sizeof kBinomials.v + seed_bytes + 256));
+  GroupRow* h_rows = reinterpret_cast<GroupRow*>(pin);  // read back
+  size_t o = rows_bytes;
+  uint64_t h2d = 0;
+  char* base = static_cast<char*>(ctx.grp_dir.ptr);
+  auto put = [&](void* dst, const void* src, size_t bytes, const char* what) {
+    std::memcpy(pin + o, src, bytes);
+    cuda_check(cudaMemcpyAsync(dst, pin + o, bytes, cudaMemcpyHostToDevice, ctx.stream), what);
+    o += (bytes + 15) / 16 * 16;
+    h2d += bytes;
+  };
+  cuda_check(cudaEventRecord(ctx.ev[0], ctx.stream), "event");
+  const GroupStepArgs a0 = group_args(ctx, p, d, row0, row0 + 1);
+  std::vector<GroupRow> init(kGroupMaxN + 1);
+  init[row0] = sd.row;
+  put(base + d.off_rows, init.data(), rows_bytes, "row scalars");
+  put(base + d.off_bin, kBinomials.v, sizeof kBinomials.v, "binomials");
+  put(a0.in.keys, sd.keys.data(), ns * 4, "seed keys");
+  put(a0.in.lo, sd.weights.data(), ns * 4, "seed weights");
+  put(base + d.off_list, sd.units.data(), sd.units.size() * sizeof(GroupSeedUnit), "seed buckets");
+  cuda_check(cudaMemsetAsync(a0.in.gdir, 0, (size_t)kBinomials.at(n, row0) * sizeof(GroupDir), ctx.stream),
+             "clear seed directory");
+  cuda_check(launch_group_seed(reinterpret_cast<const GroupSeedUnit*>(base + d.off_list), (u32)sd.units.size(), a0.in,
+                               ctx.stream),
+             "group seed kernel");
+  uint64_t launches = 1;
+
+  unsigned from = row0 + 1;
+  for (int attempt = 0;; ++attempt) {
+    for (unsigned m = from; m <= n; ++m) {
+      const GroupStepArgs a = group_args(ctx, p, d, row0, m);
+      cuda_check(launch_group_plan(a, kBinomials.at(n, m), ctx.stream), "group plan kernel");
+      cuda_check(launch_group_pull(a, ctx.sms, ctx.stream), "group pull kernel");
+      launches += 2;
+    }
+    cuda_check(cudaEventRecord(ctx.ev[1], ctx.stream), "event");
+    cuda_check(cudaMemcpyAsync(h_rows, base + d.off_rows, rows_bytes, cudaMemcpyDeviceToHost, ctx.stream),
+               "read row scalars");
+    cuda_check(cudaStreamSynchronize(ctx.stream), "grouped rows");
+    ctx.d2h_bytes += rows_bytes;
+    unsigned bad = 0;
+    for (unsigned m = from; m <= n && !bad; ++m)
+      if (h_rows[m].error) bad = m;
+    if (!bad) break;
+    // Run again from the row that failed; its input stands.
+    const GroupRow& r = h_rows[bad];
+    if (attempt >= 40 || (r.error & kErrBounds)) return false;
+    // (More units or pieces than the directory holds, or weights beyond 32 bits:
+    // the partitioned rows take the batch.)
+    if ((r.error & kErrNeedWide) || r.units + r.pieces > d.unit_cap) return false;
+    const unsigned side = (bad - row0) & 1u;
+    const u64 need = (u64)r.alloc + r.alloc / 8 + 4096;
+    if (need > 0xfffffff0ull || !group_reserve(ctx, ctx.grp_side[side], need * kGroupEntryBytes, p.budget)) return false;
+    cuda_check(cudaMemsetAsync(base + d.off_rows + bad * sizeof(GroupRow), 0, (n + 1 - bad) * sizeof(GroupRow),
+                               ctx.stream),
+               "clear row scalars");
+    from = bad;
+  }
+  float ms = 0;
+  cudaEventElapsedTime(&ms, ctx.ev[0], ctx.ev[1]);
+
+  // Certify the weights as the row-by-row path does: a row's output total is
+  // at most its input total times its free columns.
+  u128 total = 0;
+  for (u64 i = 0; i < hc.count; ++i) total += p.R == 1 ? hc.res[i] : (u64)hc.res[i] | ((u64)hc.res[hc.count + i] << 32);
+  for (unsigned m = row0 + 1; m <= n; ++m) {
+    if ((total * (u128)(n - m + 1)) >> 63)
+      fail(QPEPS_ERR_OVERFLOW, row_msg("exact 64-bit weights are not certified at row", m));
+    total = h_rows[m].weight_sum;
+  }
+  if (ctx.rec) ctx.rec->ok = false;
+  ctx.h2d_bytes += h2d;
+  const size_t eb = entry_bytes(p);
+  rs.batches += 1;
+  rs.launches += launches;
+  rs.device_ms += ms;
+  rs.peak_states = std::max<u64>(rs.peak_states, hc.count);
+  u64 in = hc.count, terms = sd.row.next_terms;
+  u64 ns_all = 0;
+  for (unsigned m = row0 + 1; m <= n; ++m) ns_all += h_rows[m].t_end > h_rows[m].t_plan ? h_rows[m].t_end - h_rows[m].t_plan : 0;
+  const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+  for (unsigned m = row0 + 1; m <= n; ++m) {
+    const GroupRow& r = h_rows[m];
+    RowAcc& acc = rows[m - 1];
+    acc.used = true;
+    acc.device_row = true;
+    acc.input_states += in;
+    acc.candidates += (u128)in * n;
+    acc.matched += terms;
+    acc.completed += terms;
+    acc.output_states += r.out_count;
+    for (int q = 0; q < p.Rc; ++q) acc.weight_res[q] = (acc.weight_res[q] + r.weight_sum % kPrimes[q]) % kPrimes[q];
+    if (m == n)
+      for (int q = 0; q < p.Rc; ++q) rs.final_res[q] = (rs.final_res[q] + r.weight_sum % kPrimes[q]) % kPrimes[q];
+    const u64 t = r.t_end > r.t_plan ? r.t_end - r.t_plan : 0;
+    acc.elapsed += ns_all ? wall * (double)t / (double)ns_all : 0.0;
+    if (terms) {
+      rs.scatter_ms += r.t_pull > r.t_plan ? (double)(r.t_pull - r.t_plan) * 1e-6 : 0.0;
+      rs.merge_ms += r.t_end > r.t_pull ? (double)(r.t_end - r.t_pull) * 1e-6 : 0.0;
+      rs.merge_launches += 1;
+      rs.merge_bytes += (in + r.out_count) * eb;
+      rs.entries_in += in;
+      rs.entries_out += r.out_count;
+      rs.candidates += terms;
+    }
+    rs.peak_states = std::max<u64>(rs.peak_states, r.out_count);
+    in = r.out_count;
+    terms = r.next_terms;
+  }
+  return true;
+}
+
+
 // Contract every pending chunk to the last row. Each chunk is one merged
 // device boundary; under memory pressure a boundary is halved and the upper
 // half parked on the host (exact: the contraction is linear in the boundary).
@@ -1438,6 +1803,8 @@ static void run_chunks(Ctx& ctx, const Plan& p, std::vector<HostChunk> pending, 
     HostChunk hc = std::move(pending.back());
     pending.pop_back();
     if (run_resident(ctx, p, hc, rows, rs)) continue;
+    if (run_chunk_grouped(ctx, p, hc, rows, rs)) continue;
+    f.cap = ctx.front[0].ptr ? ctx.front[0].bytes / entry_bytes(p) : 0;  // (it may have been given back)
     upload_chunk(ctx, p, hc, f);
     rs.batches += 1;
     rs.peak_states = std::max<u64>(rs.peak_states, f.count);
@@ -2581,6 +2948,8 @@ static void contract_impl(Ctx& ctx, unsigned n, const qpeps_options& o, const ui
   // estimated below a prefix.)
   out.plan.batch_states = serve_estimate(n, k) * (k ? 3.0 : o.symmetry ? 1.0 : 2.0);
   out.plan.prefix = k > 0;
+  if (n <= kGroupMaxN)
+    out.plan.group_states = group_rows_states(out.plan.batch_states / (k ? 3.0 : 1.0), k ? 3.0 : 1.01, o.use_graph);
   // Predictive slicing: when the merged frontier is estimated not to fit the
   // device budget, contract groups of slices (first-row orbit slices, or
   // deeper prefix slices) one chunk at a time instead of halving a live
@@ -2606,6 +2975,9 @@ static void contract_impl(Ctx& ctx, unsigned n, const qpeps_options& o, const ui
         }
         out.slice_depth = row0;
         out.plan.batch_states = std::min(est_item * (double)per_chunk, cap_states);
+        if (n <= kGroupMaxN)
+          out.plan.group_states = group_rows_states(est_total / (double)items.size() * (double)per_chunk,
+                                                    std::min(2.5, ctx.tune.slice_margin), o.use_graph);
         run_chunks(ctx, out.plan, std::move(chunks), out.rows, out.rs);
         items.clear();
         break;

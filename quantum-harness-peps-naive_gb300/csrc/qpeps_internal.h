@@ -302,6 +302,68 @@ struct ResidentArgs {
 uint32_t resident_capacity();
 cudaError_t launch_resident_rows(const ResidentArgs& a, cudaStream_t stream);
 
+// Column-grouped row step (qpeps_group_kernels.cu): exact weights, the
+// boundary grouped by column set.
+constexpr unsigned kGroupMaxN = 18;  // widest board whose 2 N - 2 live diagonal bits fit 32 but for two
+
+struct GroupDir {   // per column set, in colex rank order
+  uint32_t base;    // unit of its first bucket
+  uint32_t bits;    // log2 of its buckets
+  uint32_t total;   // entries
+  uint32_t pad;
+};
+
+// One row's scalars (device; zero before the row's plan runs).
+struct GroupRow {
+  unsigned long long out_count;   // merged entries
+  unsigned long long alloc;       // output entries handed out in blocks (counted past the buffer's end too)
+  unsigned long long next_terms;  // their successor terms at the next row
+  unsigned long long weight_sum, weight_max;
+  unsigned long long t_plan, t_pull, t_end;  // global timer, ns
+  uint32_t units, next_unit, pieces, ctas_done;
+  uint32_t error;
+  float merge_rate;  // merged entries per term
+};
+
+struct GroupSide {    // a boundary
+  uint32_t* keys;     // [cap]
+  uint32_t* lo;       // [cap] weights
+  uint64_t cap;       // < 2^32
+  GroupDir* gdir;     // [C(n, m)]
+  uint4* udir;        // [unit_cap] {first entry, entries of quarters 0 | 1 << 16, 2 | 3 << 16,
+                      //  further piece or 0}
+  uint32_t unit_cap;
+};
+
+struct GroupStepArgs {
+  GroupSide in, out;
+  const GroupRow* prev;  // the input boundary's scalars
+  GroupRow* row;
+  uint2* units;          // [unit_cap] {columns | bits << 24, bucket}
+  const uint32_t* binomials;  // [(kGroupMaxN + 2)^2]
+  uint32_t n, m;         // board size, columns set after the row
+  uint32_t rm;           // top u bits implied by the bucket
+  uint32_t max_bits;
+  uint32_t write_out;
+  uint32_t block;        // output entries a CTA takes at a time, at least a table's
+  float target;          // expected outputs of a unit
+};
+
+float group_unit_target();
+// Output block of a boundary of about `states` entries, and the entries its
+// buffer needs with the blocks' unused ends.
+uint32_t group_block(double states, int sms);
+uint64_t group_capacity(double states, int sms);
+cudaError_t launch_group_plan(const GroupStepArgs& a, uint32_t groups, cudaStream_t stream);
+cudaError_t launch_group_pull(const GroupStepArgs& a, int sms, cudaStream_t stream);
+// One bucket of the seed boundary, its entries in place: the directories.
+struct GroupSeedUnit {
+  uint32_t first, unit;
+  uint32_t quarters01, quarters23;  // entries by quarter, 16 bits each
+  uint32_t rank, bits, total;       // the group's entry, with its first bucket (total > 0)
+};
+cudaError_t launch_group_seed(const GroupSeedUnit* list, uint32_t count, const GroupSide& side, cudaStream_t stream);
+
 // Serving (slotted keys, exact 64-bit weights in two planes): scatter and merge
 // of a boundary shared by requests of different board sizes. slot_mask[s] is
 // the board mask of the request in slot s; finished boards are summed into
