@@ -20,13 +20,12 @@
 // contiguous runs, never a filtered scan of a whole group (a parent group cut
 // more coarsely than the output is read with the missing bits as a filter).
 //
-// What bounds it: instruction issue and shared-memory insertions (N = 16's row
-// of 92 M candidates: 394 warp instructions per 32 candidates at 1.9 a cycle,
-// DRAM at 10 %). GB300, device ms of a board, partitioned rows against these:
-// N = 15 2.43 / 2.25, N = 16 15.6 / 10.8, N = 17 117 / 75.6, N = 18 (nine
-// batches) 821 / 702. The partitioned rows' time is their scatter, a random
-// 16-byte append a candidate at 42 to 48 G/s, and a merge on top of it; here
-// a large row runs at 38 to 60 G candidates/s all told.
+// What bounds it: instruction issue and the latency of shared-memory insertions
+// (N = 16's largest row: about 340 warp instructions per 32 candidates at 1.9 a
+// cycle, DRAM at 10 %). GB300, device ms of a board, partitioned rows against
+// these: N = 15 2.43 / 1.98, N = 16 15.6 / 8.4, N = 17 117 / 54.5, N = 18 (nine
+// batches) 821 / 495. The partitioned rows' time is their scatter, a random
+// 16-byte append a candidate at 42 to 48 G/s, and a merge on top of it.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -186,9 +185,9 @@ __device__ __forceinline__ int bar_empty(int p) { return 3 + 2 * p; }
 
 template <int W, int P, int H>
 struct PullSmem {
-  u32 key[H];
-  u32 lo[H];
-  uint2 queue[W][kBatch + 64];      // per warp: matches {table key, parent entry}
+  u32 key[H + 32];                  // the last 32: standing keys for idle lanes
+  u32 lo[H + 32];
+  uint2 queue[W][2 * kBatch];       // per warp: matches {table key, parent entry}
   PullUnit unit[P];
   unsigned long long red[3][W];
   unsigned long long apos[2], aend; // this CTA's output block
@@ -348,6 +347,7 @@ __global__ void __launch_bounds__((W + P) * 32, CTAS) group_pull_kernel(GroupSte
   constexpr int BLOCK = (W + P) * 32;
   constexpr int CONS = W * 32;
   constexpr u32 kEmpty = kFull;
+  constexpr u32 kStanding = kFull - 1u;  // no key: at most 26 of 32 diagonals are ever taken
   using Smem = PullSmem<W, P, H>;
   constexpr u32 kList = Smem::kList;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -368,8 +368,8 @@ __global__ void __launch_bounds__((W + P) * 32, CTAS) group_pull_kernel(GroupSte
   if (blockIdx.x == 0 && tid == 0) row->t_pull = global_ns();
   const u32 units = min(row->units, a.out.unit_cap);
   const KeyShape ks(n, rm);
-  for (int i = tid; i < H; i += BLOCK) {
-    s.key[i] = kEmpty;
+  for (int i = tid; i < H + 32; i += BLOCK) {
+    s.key[i] = i < H ? kEmpty : kStanding;
     s.lo[i] = 0u;
   }
   if (tid == 0) {
@@ -466,50 +466,67 @@ __global__ void __launch_bounds__((W + P) * 32, CTAS) group_pull_kernel(GroupSte
       // Scan this warp's runs for matches; insert them 128 at a time.
       u32 qn = 0;
       uint2* const q = s.queue[wid];
-      auto insert = [&](u32 first, u32 count) {  // queue entries [first, first + count), count <= 128
-        u32 k[4], slot[4], lo[4];
-        u32 todo = 0, fresh = 0;
-        const int rem = (int)count - lane;
+      // Queue entries [first, first + count), 128 of them if `full`. Lanes
+      // beyond the last one insert the key that stands in a slot beyond the
+      // table, so that nothing below is predicated.
+      auto insert = [&](auto full, u32 first, u32 count) {
+        constexpr int I = 4;
+        u32 k[I], slot[I], lo[I];
+        u32 todo = (1u << I) - 1u, fresh = 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          k[i] = 0;
-          if (rem > i * 32) {
-            const uint2 e = q[first + i * 32 + lane];
-            k[i] = e.x;
-            lo[i] = a.in.lo[e.y];
-            todo |= 1u << i;
-          }
-          slot[i] = __umulhi(k[i] * 0x9E3779B1u, (u32)H);
+        for (int i = 0; i < I; ++i) {
+          const u32 at = i * 32 + lane;
+          uint2 e;
+          if constexpr (decltype(full)::value)
+            e = q[first + at];
+          else
+            e = q[first + min(at, count - 1u)];
+          lo[i] = a.in.lo[e.y];
+          k[i] = e.x;
+          slot[i] = __umulhi(e.x * 0x9E3779B1u, (u32)H);
+          if constexpr (!decltype(full)::value)
+            if (at >= count) {
+              k[i] = kStanding;
+              slot[i] = (u32)H + lane;
+            }
         }
         __syncwarp();
-        const u32 valid = todo;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (rem > i * 32) {
-            const u32 old = atomicCAS(&s.key[slot[i]], kEmpty, k[i]);
-            if (old == kEmpty) fresh |= 1u << i;
-            if (old == kEmpty || old == k[i]) todo ^= 1u << i;
-          }
+        for (int i = 0; i < I; ++i) {
+          const u32 old = atomicCAS(&s.key[slot[i]], kEmpty, k[i]);
+          if (old == kEmpty) fresh |= 1u << i;
+          if (old == kEmpty || old == k[i]) todo ^= 1u << i;
+        }
         for (u32 probes = 0; todo; ++probes) {
-          if (probes == 192u) {
+          if (probes == 256u) {
             s.over = 1u;
             break;
           }
+          // The lowest one left takes its next slot, a step of the key's own away.
+          // (One a turn: 8 % of the board's time less than all four's tests.)
+          const u32 one = todo & (0u - todo);
+          u32 at = slot[0], key = k[0];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if ((todo >> i) & 1u) {
-              slot[i] = slot[i] + 1 == (u32)H ? 0u : slot[i] + 1;
-              const u32 old = atomicCAS(&s.key[slot[i]], kEmpty, k[i]);
-              if (old == kEmpty) fresh |= 1u << i;
-              if (old == kEmpty || old == k[i]) todo ^= 1u << i;
+          for (int i = 1; i < I; ++i)
+            if (one == 1u << i) {
+              at = slot[i];
+              key = k[i];
             }
+          at += ((key * 0x9E3779B1u) >> 4 & 63u) | 1u;
+          at = at >= (u32)H ? at - (u32)H : at;
+          const u32 old = atomicCAS(&s.key[at], kEmpty, key);
+#pragma unroll
+          for (int i = 0; i < I; ++i)
+            if (one == 1u << i) slot[i] = at;
+          if (old == kEmpty) fresh |= one;
+          if (old == kEmpty || old == key) todo ^= one;
         }
         __syncwarp();
         // List the claimed slots by quarter: one scan of four byte counts (at
         // most 128 each), two atomics a warp.
         u32 mine = 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mine += ((fresh >> i) & 1u) << (((k[i] >> quarter_at) & 3u) * 8u);
+        for (int i = 0; i < I; ++i) mine += ((fresh >> i) & 1u) << (((k[i] >> quarter_at) & 3u) * 8u);
         u32 incl = mine;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -527,8 +544,8 @@ __global__ void __launch_bounds__((W + P) * 32, CTAS) group_pull_kernel(GroupSte
         const u32 at0 = __shfl_sync(kFull, at, 0), at1 = __shfl_sync(kFull, at, 1);
         u32 excl = incl - mine;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if ((valid >> i) & 1u) atomicAdd(&s.lo[slot[i]], lo[i]);
+        for (int i = 0; i < I; ++i) {
+          atomicAdd(&s.lo[slot[i]], lo[i]);
           if ((fresh >> i) & 1u) {
             const u32 qt = (k[i] >> quarter_at) & 3u, sh = qt * 8u;
             const u32 base = qt & 2u ? at1 : at0;
@@ -538,50 +555,48 @@ __global__ void __launch_bounds__((W + P) * 32, CTAS) group_pull_kernel(GroupSte
           }
         }
       };
-      auto scan = [&](auto ranged) {
-        while (r < runs) {
-          u32 kc[4];
+      while (r < runs) {
+        u32 kc[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) kc[i] = kn[i];
-          const u32 tmask = u.test_mask[sg], tval = u.test_value[sg], add = u.added[sg];
-          const u32 entry = src + lane;
-          const int rem = (int)left - lane;
-          if (left > 128u) {
-            src += 128u;
-            left -= 128u;
+        for (int i = 0; i < 4; ++i) kc[i] = kn[i];
+        const u32 tmask = u.test_mask[sg], tval = u.test_value[sg], add = u.added[sg];
+        const u32 entry = src + lane;
+        const int rem = (int)left - lane;
+        if (left > 128u) {
+          src += 128u;
+          left -= 128u;
+          fetch();
+        } else {
+          r += W;
+          if (r < runs) {
+            load_run(u);
             fetch();
-          } else {
-            r += W;
-            if (r < runs) {
-              load_run(u);
-              fetch();
-            }
-          }
-#pragma unroll
-          for (int h = 0; h < 4; h += 2) {
-#pragma unroll
-            for (int i = h; i < h + 2; ++i) {
-              const u32 key = (kc[i] & ks.keep) | add;
-              bool hit = (kc[i] & tmask) == tval && rem > i * 32;
-              if constexpr (decltype(ranged)::value) hit = hit && (key * 0xC2B2AE35u) - from < width;
-              const u32 bal = __ballot_sync(kFull, hit);
-              if (hit) q[qn + __popc(bal & lt)] = make_uint2(key, entry + i * 32);
-              qn += __popc(bal);
-            }
-            if (qn >= kBatch) {
-              __syncwarp();
-              qn -= kBatch;
-              insert(qn, kBatch);
-            }
           }
         }
-      };
-      if (width)
-        scan(TrueTag{});
-      else
-        scan(FalseTag{});
+        bool hit[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          hit[i] = (kc[i] & tmask) == tval && rem > i * 32;
+          kc[i] = (kc[i] & ks.keep) | add;
+        }
+        if (width) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) hit[i] = hit[i] && (kc[i] * 0xC2B2AE35u) - from < width;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const u32 bal = __ballot_sync(kFull, hit[i]);
+          if (hit[i]) q[qn + __popc(bal & lt)] = make_uint2(kc[i], entry + i * 32);
+          qn += __popc(bal);
+        }
+        if (qn >= kBatch) {
+          __syncwarp();
+          qn -= kBatch;
+          insert(TrueTag{}, qn, kBatch);
+        }
+      }
       __syncwarp();
-      if (qn) insert(0, qn);
+      if (qn) insert(FalseTag{}, 0, qn);
       bar_sync(kBarConsumers, CONS);
       const bool over = s.over != 0;
       const u32 c01 = s.claims[abuf][0], c23 = s.claims[abuf][1];
@@ -728,23 +743,23 @@ __global__ void group_seed_kernel(const GroupSeedUnit* __restrict__ list, u32 co
 }
 
 constexpr int kPlanBlock = 256;
-// Two CTAs an SM with tables as large as fit, since a unit costs about 2 us
-// besides its candidates, and few enough warps for 91 registers each. N = 16 /
-// 17, device ms, warps + producers x slots x CTAs an SM: 8 + 2 x 9216 x 2
-// 10.9 / 75.5; 10 + 2 x 8192 x 2 11.4 / 75.8; 13 + 3 x 8192 x 2 (64 registers)
-// 13.9 / 90; 8 + 1 x 9216 x 2 13.9 / 91; 6 + 2 x 5376 x 3 13.3 / 91;
-// 29 + 3 x 16384 x 1 14.9 / 100.
-constexpr int kPullWarps = 8;
+// Two CTAs an SM with tables as large as fit beside the queues, since a unit
+// costs about 2 us besides its candidates. N = 16 / 17, device ms, warps +
+// producers x slots at two CTAs: 12 + 2 x 7744 8.4 / 54.5; 10 + 2 x 8192
+// 8.7 / 56.1; 9 + 2 x 8416 8.8 / 57.1; 13 + 2 x 7520 9.1 / 57.7 and 14 + 2 x 7296
+// 9.4 / 59.6 (too few registers); 10 + 3 x 7872 9.0 / 56.9; 12 + 1 x 7872
+// 10.7 / 68.5. Three CTAs with 5376 slots were 20 % slower, one with 16384 30 %.
+constexpr int kPullWarps = 12;
 constexpr int kPullProducers = 2;
-constexpr int kPullTable = 9216;
+constexpr int kPullTable = 7744;
 constexpr int kPullCtas = 2;  // per SM
 
 }  // namespace
 
 // Buckets of a group are uneven (the largest hundredth hold 3 to 4 times the
 // mean), and one beyond 0.65 of the table is scanned twice or more. N = 16 / 17,
-// ms, at 0.12: 11.4 / 79.7, at 0.15: 10.9 / 75.9, at 0.2: 11.6 / 75.1.
-float group_unit_target() { return 0.17f * kPullTable; }
+// ms, at 0.22: 8.7 / 56.4, at 0.25: 8.45 / 55.2, at 0.28: 8.44 / 54.5.
+float group_unit_target() { return 0.28f * kPullTable; }
 
 uint32_t group_block(double states, int sms) {
   const double share = states / ((double)sms * kPullCtas * 16.0);
