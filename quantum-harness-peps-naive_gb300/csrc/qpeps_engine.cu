@@ -1486,8 +1486,8 @@ constexpr u64 kGroupMaxSeeds = 4096;
 
 // Expected largest boundary that column-grouped rows are to hold, 0 where the
 // partitioned rows are faster. Device ms at N = 15 / 16 / 17 / 18 (peaks of 18,
-// 106 and 706 M entries; nine batches of 380 to 743 M): grouped 1.98 / 8.4 /
-// 54.5 / 495, partitioned 2.43 / 15.6 / 117 / 821; at N = 14 (2.8 M) the
+// 106 and 706 M entries; nine batches of 380 to 743 M): grouped 1.97 / 8.4 /
+// 54.1 / 487, partitioned 2.43 / 15.6 / 117 / 821; at N = 14 (2.8 M) the
 // partitioned rows' traffic stays in L2 and the grouped ones' smallest units are
 // nearly empty. Repeated contractions (use_graph) keep the rows that a graph can
 // replay up to 200 M entries. `room`: the buffers' size over the expected one.
@@ -1639,6 +1639,7 @@ static GroupStepArgs group_args(const Ctx& ctx, const Plan& p, const GroupDirs& 
   a.write_out = m < p.n;
   a.block = group_block(p.group_states, ctx.sms);
   a.target = group_unit_target();
+  a.share = group_unit_share(ctx.sms);
   return a;
 }
 

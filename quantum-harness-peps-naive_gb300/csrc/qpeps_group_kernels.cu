@@ -23,8 +23,8 @@
 // What bounds it: instruction issue and the latency of shared-memory insertions
 // (N = 16's largest row: about 340 warp instructions per 32 candidates at 1.9 a
 // cycle, DRAM at 10 %). GB300, device ms of a board, partitioned rows against
-// these: N = 15 2.43 / 1.98, N = 16 15.6 / 8.4, N = 17 117 / 54.5, N = 18 (nine
-// batches) 821 / 495. The partitioned rows' time is their scatter, a random
+// these: N = 15 2.43 / 1.97, N = 16 15.6 / 8.4, N = 17 117 / 54.1, N = 18 (nine
+// batches) 821 / 487. The partitioned rows' time is their scatter, a random
 // 16-byte append a candidate at 42 to 48 G/s, and a merge on top of it.
 #include <cuda_runtime.h>
 
@@ -122,7 +122,10 @@ __global__ void __launch_bounds__(BLOCK) group_plan_kernel(GroupStepArgs a) {
       // A bucket reads at most two buckets a side of a parent cut two bits
       // more finely, which bounds the segment list.
       if (deepest > 2 && deepest - 2 > b) b = deepest - 2;
-      while (b < a.max_bits && est > a.target * (float)(1u << b)) ++b;
+      // A row with few outputs is cut finely enough for eight units a CTA.
+      const float share = (float)prev->next_terms * prev->merge_rate * a.share;
+      const float target = fminf(a.target, fmaxf(share, 64.f));
+      while (b < a.max_bits && est > target * (float)(1u << b)) ++b;
       units = 1u << b;
     }
   }
@@ -232,20 +235,16 @@ struct KeyShape {
 
 // One warp: the runs of parents that hold a unit's matches, into `u`.
 // Lane = column c.
-__device__ __forceinline__ bool group_unit_runs(const GroupStepArgs& a, GroupRow* row, const KeyShape& ks, u32 units,
-                                                PullUnit& u) {
+__device__ __forceinline__ bool group_unit_runs(const GroupStepArgs& a, const KeyShape& ks, u32 units,
+                                                u32 unit, uint2 ud, PullUnit& u) {
   const u32 lane = threadIdx.x & 31, lt = lt_mask();
   const u32 n = a.n;
-  u32 unit = 0;
-  if (lane == 0) unit = atomicAdd(&row->next_unit, 1u);
-  unit = __shfl_sync(kFull, unit, 0);
   if (lane == 0) {
     u.valid = unit < units;
     u.unit = unit;
     u.nseg = u.nrun = u.nlong = u.pairs = 0;
   }
   if (unit >= units) return false;
-  const uint2 ud = a.units[unit];
   const u32 cols = ud.x & 0xffffffu, b = ud.x >> 24, beta = ud.y;
   const u32 c = lane;
   const bool in_c = c < n && ((cols >> c) & 1u);
@@ -341,7 +340,8 @@ __device__ __forceinline__ bool group_unit_runs(const GroupStepArgs& a, GroupRow
 // W warps scan and insert ("consumers"); P more build the runs of the coming
 // units, each in a slot of its own: a unit's runs take four dependent trips to
 // L2 (its number, its columns, its parents' directories, their buckets), about
-// 3 us, which P units in the making hide.
+// 3 us, of which the first two are made for the unit after (N = 18 497 -> 489 ms)
+// and which P units in the making hide.
 template <int W, int P, int H, int CTAS>
 __global__ void __launch_bounds__((W + P) * 32, CTAS) group_pull_kernel(GroupStepArgs a) {
   constexpr int BLOCK = (W + P) * 32;
@@ -379,13 +379,20 @@ __global__ void __launch_bounds__((W + P) * 32, CTAS) group_pull_kernel(GroupSte
   __syncthreads();
   if (wid >= W) {
     // Producer: build, hand over, wait for the slot; ends with an invalid unit.
+    // The unit after is taken, and its columns read, meanwhile.
     const int p = wid - W;
+    auto take = [&]() { return lane == 0 ? atomicAdd(&row->next_unit, 1u) : 0u; };
+    u32 unit = __shfl_sync(kFull, take(), 0);
+    uint2 ud = unit < units ? a.units[unit] : make_uint2(0u, 0u);
     for (;;) {
-      const bool more = group_unit_runs(a, row, ks, units, s.unit[p]);
+      u32 next = take();
+      const bool more = group_unit_runs(a, ks, units, unit, ud, s.unit[p]);
       __syncwarp();
       __threadfence_block();
       bar_arrive(bar_full(p), CONS + 32);
       if (!more) return;
+      unit = __shfl_sync(kFull, next, 0);
+      ud = unit < units ? a.units[unit] : make_uint2(0u, 0u);
       bar_sync(bar_empty(p), CONS + 32);
     }
   }
@@ -760,6 +767,11 @@ constexpr int kPullCtas = 2;  // per SM
 // mean), and one beyond 0.65 of the table is scanned twice or more. N = 16 / 17,
 // ms, at 0.22: 8.7 / 56.4, at 0.25: 8.45 / 55.2, at 0.28: 8.44 / 54.5.
 float group_unit_target() { return 0.28f * kPullTable; }
+
+// A row with few outputs is cut finely enough for eight units a CTA: its largest
+// bucket is one CTA's work (the last row of N = 15 was 128 buckets and 143 us;
+// board 2.07 -> 1.97 ms).
+float group_unit_share(int sms) { return 1.f / (8.f * (float)(sms * kPullCtas)); }
 
 uint32_t group_block(double states, int sms) {
   const double share = states / ((double)sms * kPullCtas * 16.0);

@@ -346,10 +346,12 @@ struct GroupStepArgs {
   uint32_t max_bits;
   uint32_t write_out;
   uint32_t block;        // output entries a CTA takes at a time, at least a table's
-  float target;          // expected outputs of a unit
+  float target;          // expected outputs of a unit, at most
+  float share;           // and at most this share of the row's
 };
 
 float group_unit_target();
+float group_unit_share(int sms);
 // Output block of a boundary of about `states` entries, and the entries its
 // buffer needs with the blocks' unused ends.
 uint32_t group_block(double states, int sms);
