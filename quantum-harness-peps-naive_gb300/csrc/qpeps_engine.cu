@@ -1486,8 +1486,8 @@ constexpr u64 kGroupMaxSeeds = 4096;
 
 // Expected largest boundary that column-grouped rows are to hold, 0 where the
 // partitioned rows are faster. Device ms at N = 15 / 16 / 17 / 18 (peaks of 18,
-// 106 and 706 M entries; nine batches of 380 to 743 M): grouped 1.97 / 8.4 /
-// 54.1 / 487, partitioned 2.43 / 15.6 / 117 / 821; at N = 14 (2.8 M) the
+// 106 and 706 M entries; nine batches of 380 to 743 M): grouped 1.96 / 8.3 /
+// 53.4 / 481, partitioned 2.43 / 15.6 / 117 / 821; at N = 14 (2.8 M) the
 // partitioned rows' traffic stays in L2 and the grouped ones' smallest units are
 // nearly empty. Repeated contractions (use_graph) keep the rows that a graph can
 // replay up to 200 M entries. `room`: the buffers' size over the expected one.

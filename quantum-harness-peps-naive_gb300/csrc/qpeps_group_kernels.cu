@@ -20,12 +20,12 @@
 // contiguous runs, never a filtered scan of a whole group (a parent group cut
 // more coarsely than the output is read with the missing bits as a filter).
 //
-// What bounds it: instruction issue and the latency of shared-memory insertions
-// (N = 16's largest row: about 340 warp instructions per 32 candidates at 1.9 a
-// cycle, DRAM at 10 %). GB300, device ms of a board, partitioned rows against
-// these: N = 15 2.43 / 1.97, N = 16 15.6 / 8.4, N = 17 117 / 54.1, N = 18 (nine
-// batches) 821 / 487. The partitioned rows' time is their scatter, a random
-// 16-byte append a candidate at 42 to 48 G/s, and a merge on top of it.
+// What bounds it: instruction issue (N = 16's largest row, 119 M candidates:
+// about 400 warp instructions per 32 candidates at 2.5 a cycle and SM, half of
+// them the insertions; DRAM at 13 %). GB300, device ms of a board, partitioned
+// rows against these: N = 15 2.43 / 1.96, N = 16 15.6 / 8.3, N = 17 117 / 53.4,
+// N = 18 (nine batches) 821 / 481. The partitioned rows' time is their scatter,
+// a random 16-byte append a candidate at 42 to 48 G/s, and a merge on top of it.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,6 +40,10 @@ namespace {
 constexpr u32 kFull = 0xffffffffu;
 constexpr int kBinDim = kGroupMaxN + 2;
 
+template <int I>
+struct Items {
+  static constexpr int value = I;
+};
 struct TrueTag {
   static constexpr bool value = true;
 };
@@ -473,11 +477,11 @@ __global__ void __launch_bounds__((W + P) * 32, CTAS) group_pull_kernel(GroupSte
       // Scan this warp's runs for matches; insert them 128 at a time.
       u32 qn = 0;
       uint2* const q = s.queue[wid];
-      // Queue entries [first, first + count), 128 of them if `full`. Lanes
+      // Queue entries [first, first + count), 32 * items of them if `full`. Lanes
       // beyond the last one insert the key that stands in a slot beyond the
       // table, so that nothing below is predicated.
-      auto insert = [&](auto full, u32 first, u32 count) {
-        constexpr int I = 4;
+      auto insert = [&](auto items, auto full, u32 first, u32 count) {
+        constexpr int I = decltype(items)::value;
         u32 k[I], slot[I], lo[I];
         u32 todo = (1u << I) - 1u, fresh = 0;
 #pragma unroll
@@ -599,11 +603,16 @@ __global__ void __launch_bounds__((W + P) * 32, CTAS) group_pull_kernel(GroupSte
         if (qn >= kBatch) {
           __syncwarp();
           qn -= kBatch;
-          insert(TrueTag{}, qn, kBatch);
+          insert(Items<4>{}, TrueTag{}, qn, kBatch);
         }
       }
       __syncwarp();
-      if (qn) insert(FalseTag{}, 0, qn);
+      // (A warp's last part batch is 40 matches on average: half as wide, N = 17
+      // takes 53.4 ms instead of 54.0. Narrower still, in turns: 54.6 and 55.9.)
+      if (qn > 64u)
+        insert(Items<4>{}, FalseTag{}, 0, qn);
+      else if (qn)
+        insert(Items<2>{}, FalseTag{}, 0, qn);
       bar_sync(kBarConsumers, CONS);
       const bool over = s.over != 0;
       const u32 c01 = s.claims[abuf][0], c23 = s.claims[abuf][1];
