@@ -7,7 +7,9 @@ orbit slices) through the library's C ABI. Prints one JSON line. By default
 the contraction runs with use_graph: the first warm-up step records its row
 steps and captures them as one CUDA graph, and every later step replays the
 whole contraction on the device from its seeds (checked row by row against the
-recorded run); --no-graph contracts eagerly every step.
+recorded run); --no-graph contracts eagerly every step. Boundaries of over
+200 M entries (N = 17, 18) run column-grouped, all rows of a device batch
+queued at once, and need no replay (`run.rows` says which ran).
 
 value  : boundary entries per second = (boundary entries of the merged
          contraction: the sum over device rows of the merged frontier's input
@@ -21,9 +23,9 @@ value  : boundary entries per second = (boundary entries of the merged
 e2e    : the same entries / wall time of the C-ABI call (host seeding,
          host->device upload of the seed boundary, all row steps, device->host
          read-back of every row's metrics and of the count residues).
-roofline: the merge step (scatter + merge kernels), algorithmic bytes
-         E*(S_in+S_out) summed over the row steps of one contraction over
-         those kernels' CUDA-event time. `traffic` is DRAM bytes per step
+roofline: the merge step (scatter + merge kernels, or plan + pull kernels of
+         column-grouped rows), algorithmic bytes E*(S_in+S_out), E = 16, summed
+         over the row steps of one contraction over those kernels' time. `traffic` is DRAM bytes per step
          scaled from a small ncu capture of peak-row launches (see
          TRAFFIC_PER_ALGORITHMIC_BYTE); null where none applies.
 cpu_baseline: the CPU oracle (threaded restatement of the reference's
@@ -66,6 +68,9 @@ PACKAGE = "quantum-harness-peps-naive_gb300"
 # algorithmic bytes by it (an upper estimate: the peak rows re-read the most).
 # Keyed by the scatter kind the figure was captured with (1, the window scatter).
 TRAFFIC_PER_ALGORITHMIC_BYTE: dict = {1: 171.290302464 / 56.96632816}
+# Column-grouped rows hold an entry in 8 bytes: the pulls of Q(16) rows 10-12
+# moved 5.474 GB for (51.4 + 87.8 + 87.8 + 105.5 + 105.5 + 79.5) M entries.
+GROUPED_TRAFFIC_PER_ALGORITHMIC_BYTE = 5.474 / (16 * 0.5176)
 METRIC = "Q(N) wall time & boundary entries/s at N=18 (bit-exact)"
 UNIT = "boundary entries/s"
 
@@ -356,11 +361,16 @@ def run_ours(args):
     tuning = ctx.tuning
     kind = tuning.get("scatter_kind")
     # The capture behind the factor is of the u64 row path's scatter and merge.
-    tpb = (TRAFFIC_PER_ALGORITHMIC_BYTE.get(kind)
-           if d["merge"] == 2 and args.grain == "row" and d["key_bits"] == 64 else None)
+    u64_rows = d["merge"] == 2 and args.grain == "row" and d["key_bits"] == 64
+    # Column-grouped rows report their plan kernels as the scatter: 1 % of the
+    # time, where a scatter is two thirds.
+    grouped = u64_rows and d["scatter_kernel_ms"] < 0.1 * d["merge_kernel_ms"]
+    tpb = (GROUPED_TRAFFIC_PER_ALGORITHMIC_BYTE if grouped
+           else TRAFFIC_PER_ALGORITHMIC_BYTE.get(kind) if u64_rows else None)
     roofline = {
         "bound": "hbm",
-        "kernel": ("merge step: partition scatter + partition merge kernels" if d["merge"] == 2
+        "kernel": ("merge step: plan + pull kernels of column-grouped rows" if grouped
+                   else "merge step: partition scatter + partition merge kernels" if d["merge"] == 2
                    else "merge step: row_expand_insert_kernel + compact_kernel (global table)"),
         "achieved": achieved,
         "peak": peak,
@@ -368,7 +378,9 @@ def run_ours(args):
         "unit": "GB/s",
         "frac": achieved / peak,
         "traffic": (tpb * d["merge_kernel_bytes"]) if tpb else None,
-        "traffic_scope": ("DRAM bytes per step: the step's algorithmic bytes x 3.007, the DRAM bytes per algorithmic "
+        "traffic_scope": ("DRAM bytes per step: the step's algorithmic bytes x 0.661, the DRAM bytes per algorithmic "
+                          "byte that ncu measured on the pull launches of Q(16) rows 10-12 (8-byte entries)" if grouped
+                          else "DRAM bytes per step: the step's algorithmic bytes x 3.007, the DRAM bytes per algorithmic "
                           "byte that ncu measured on the scatter and merge launches of Q(17) rows 11-13 (an upper "
                           "estimate)" if tpb else "no capture for this configuration"),
         "algorithmic_bytes_per_step": d["merge_kernel_bytes"],
@@ -379,9 +391,12 @@ def run_ours(args):
         # Successor candidates per step, and per second of scatter-kernel time
         # (summed over concurrent lanes, so a per-kernel rate).
         "candidates_per_step": d["candidates"],
-        "scatter_candidates_per_s": d["candidates"] / max(d["scatter_kernel_ms"] / 1e3, 1e-12),
+        "scatter_candidates_per_s": (None if grouped
+                                     else d["candidates"] / max(d["scatter_kernel_ms"] / 1e3, 1e-12)),
     }
-    if d["exact_weights"]:
+    if grouped:
+        dtype = "32-bit group keys + exact u32 weights (certified row by row), exact u64 sums"
+    elif d["exact_weights"]:
         dtype = f"u{d['key_bits']} keys + exact u64 weights (2x u32 words), host-side CRT bookkeeping"
     else:
         dtype = f"u{d['key_bits']} keys + {d['residues']}x u32 residues"
@@ -406,7 +421,8 @@ def run_ours(args):
             "exact_weights": bool(d["exact_weights"]),
             "key_bits": d["key_bits"],
             "merge": {1: "hash", 2: "partition"}.get(d["merge"], d["merge"]),
-            "cuda_graph": not args.no_graph,
+            "rows": "column-grouped" if grouped else "partitioned",
+            "cuda_graph": not args.no_graph and not grouped,
             "tuning": tuning,
             "tuning_cache": tuning_note,
         },
@@ -443,7 +459,8 @@ def run_ours(args):
         # The scatter's access pattern alone on this device (random 16-byte
         # appends into hash partitions, one cursor atomic each), measured
         # after the timed region: the time the step's candidates need at that
-        # rate bounds the merge step from below, whatever the DRAM bandwidth.
+        # rate bounds partitioned rows from below, whatever the DRAM bandwidth
+        # (column-grouped rows append nothing and pass it: frac above 1).
         cand = 512 << 20
         fill = float(tuning.get("partition_fill", 0.75))
         parts = int(cand / (fill * 2048)) + 1

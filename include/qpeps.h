@@ -123,7 +123,9 @@ typedef struct qpeps_options {
   uint32_t use_graph;            /* 1 = the first contraction with these options (and tuning) on a
                                     context records its row steps and captures them as one CUDA
                                     graph; later identical contractions replay it (one launch, one
-                                    synchronisation) and check every row against the recorded run */
+                                    synchronisation) and check every row against the recorded run.
+                                    Device batches of over 200 M entries (N = 17, 18) run
+                                    column-grouped rows instead, queued at once and not captured */
   uint64_t device_budget_bytes;  /* 0 = auto (a fraction of free device memory) */
   uint32_t tail_row;             /* rows >= tail_row run in the slice-tail kernel (a CTA contracts
                                     batches of boundary entries in shared memory); 0 = auto (never),
