@@ -1062,9 +1062,12 @@ static void run_tail(Ctx& ctx, const Plan& p, DevFrontier& f, unsigned row0, std
 // the merges clear the partition cursors they read, and the host waits once
 // for all of them. A row that does not fit the chain's buffers stops it with
 // its input intact, and the host goes on from that row as before.
-// Above kQueueTerms a row runs for 0.1 ms and more, and its exact sizes save
-// more memory than the wait costs.
+// Larger rows, from kQueueTerms to kLargeQueueTerms, are a chain of their own in
+// the merge's 2048-candidate shape: a row that runs by itself waits about 25 us
+// for its sizes. Beyond that a row runs for 2 ms and more, and its exact sizes
+// save more memory than the wait costs.
 constexpr u64 kQueueTerms = 4u << 20;
+constexpr u64 kLargeQueueTerms = 64u << 20;
 
 // Pinned scalars of `steps` steps and of the state before them ([0], which the
 // caller fills), zero.
@@ -1205,25 +1208,32 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   if (!wkeys && ((kind != 0 && kind != 1 && kind != 4) || (ctx.tune.wide_merge & 1u))) return 0;
   // Terms a row may have, and those it is expected to have at most (the grids
   // are sized for these; a grid covers any number).
-  const u64 most = (u64)std::min((double)kQueueTerms, std::max(1048576.0, 1.6 * p.batch_states));
+  // A chain of larger rows starts where a row is known to have more than a
+  // chain of small ones holds.
+  const bool large = known_terms != kTermsUnknown && known_terms > kQueueTerms;
+  const u64 most = (u64)std::min((double)(large ? kLargeQueueTerms : kQueueTerms),
+                                 std::max(1048576.0, 1.6 * p.batch_states));
   const double likely = std::min((double)most, std::max(65536.0, 1.6 * p.batch_states));
   if (f.count > most || (known_terms != kTermsUnknown && known_terms > most)) return 0;
-  // Rows expected to stay below that: a row of n columns with r queens on the
-  // board leaves about n - 2.2 r free ones (fewer, and no more growth, from
-  // the middle of the board on).
+  // Rows that may stay below that: an entry with r of n rows placed has about
+  // n (1 - r / n)^2.3 successors (N = 17: 6.7 at r = 5, 3.6 at 8, 2.2 at 10, 1.3
+  // at 12). Boards differ by a factor of four either way; a row too many costs
+  // two launches that return at once, one too few a wait.
   unsigned count = 0;
-  double expect = known_terms != kTermsUnknown ? (double)known_terms
-                                               : (double)f.count * std::max(1.0, (double)p.n - 2.2 * row);
-  while (row + count < stop && (1.6 * p.batch_states <= (double)most || 2 * row > p.n || expect <= (double)most)) {
+  auto growth = [&](unsigned r) { return std::max(1.0, p.n * std::pow(1.0 - (double)r / p.n, 2.3)); };
+  double expect = known_terms != kTermsUnknown ? (double)known_terms : (double)f.count * growth(row);
+  while (row + count < stop &&
+         (1.6 * p.batch_states <= (double)most || 2 * row > p.n || expect <= 4.0 * (double)most)) {
     ++count;
-    expect *= std::max(1.5, (double)p.n - 2.2 * (row + count));
+    expect *= growth(row + count);
   }
   if (count < 2) return 0;
   const size_t eb = entry_bytes(p);
   // Small merge CTAs (four an SM, 1024 candidates) where they exist: a chain's
   // scatter waits for its deepest partition cursor, and half the candidates a
   // partition halve that.
-  const u32 shape = !wkeys && wide_merge_supported(p.R) ? 2u : 0u;
+  // (Large rows scatter faster into half as many partitions.)
+  const u32 shape = !wkeys && !large && wide_merge_supported(p.R) ? 2u : 0u;
   const u32 pcap = wkeys ? wide_key_partition_capacity() : partition_capacity(shape);
   const double mean = ctx.partition_fill * pcap;
   StepSource source{nullptr, mean, 0, (shape == 2 ? 8u : 2u) * (u32)ctx.sms};

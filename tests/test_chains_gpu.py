@@ -70,6 +70,18 @@ def test_chains_around_large_rows(fresh, qp, key_bits):
     assert _layers(g) == _layers(t)
 
 
+# Rows of 4 to 64 M terms are a chain of their own; the last one is below that
+# again. The prefix's estimate is above (N = 19) and below (N = 17) its boundary.
+@pytest.mark.parametrize("n,prefix", [(19, [0, 2, 5]), (17, [8, 2])])
+def test_chains_of_large_rows(fresh, qp, n, prefix):
+    count, g = fresh.count_with_stats(n, prefix)
+    want, t = fresh.count_with_stats(n, prefix, merge=qp.MERGE_HASH)
+    assert count == want
+    assert (g.peak_states, g.row_operator_candidates, g.row_operator_matched) == (
+        t.peak_states, t.row_operator_candidates, t.row_operator_matched)
+    assert g.device["gpu_launches"] < t.device["gpu_launches"]
+
+
 @pytest.mark.parametrize("n", [2, 11, 13, 14])
 def test_site_chains(fresh, qp, n):
     s = fresh.contract_rows(n, granularity=qp.GRAIN_SITE)
