@@ -287,28 +287,33 @@ __device__ __forceinline__ void table_insert_pair(Slot<K, R>* __restrict__ table
   }
 }
 
-// The C table is read through shared memory: the lanes of a warp have
-// different signatures, which constant memory serves one after the other, and
-// after a launch every line of it is a miss. The copy is made before the
-// kernel waits for the one before it.
-template <typename K, int R, int BLOCK>
+// QUEUED (a step of a chain): the C table is read through shared memory: the
+// lanes of a warp have different signatures, which constant memory serves one
+// after the other, and after a launch every line of it is a miss. The copy is
+// made before the kernel waits for the one before it. A large step by itself
+// is bound by its table's random sectors instead, and looks at a slot before
+// it swaps: most children meet a key that stands (N = 15, a launch per site:
+// 112 ms, against 134 with the chain's form of this kernel and the compaction).
+template <typename K, int R, int BLOCK, bool QUEUED>
 __global__ void __launch_bounds__(BLOCK) site_expand_insert_kernel(const void* __restrict__ keys,
                                                                    const u32* __restrict__ res, u64 res_stride,
                                                                    u64 n_in, unsigned n, unsigned site,
                                                                    Slot<K, R>* __restrict__ table, u64 table_mask,
                                                                    StepScalars* __restrict__ sc, TableSource q) {
   __shared__ CTableDev s_c;
-  next_kernel_may_start();
-  for (u32 i = threadIdx.x; i < sizeof(CTableDev) / 4; i += BLOCK)
-    reinterpret_cast<u32*>(&s_c)[i] = reinterpret_cast<const u32*>(&c_table)[i];
-  __syncthreads();
-  wait_for_kernel_before();
-  u64 slots = table_mask + 1;
-  if (!table_sizes(q, sc, res_stride, n_in, slots)) return;
-  table_mask = slots - 1;
-  if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) {
-    sc->t_scatter = global_ns();
-    sc->terms = q.prev->next_terms;
+  if constexpr (QUEUED) {
+    next_kernel_may_start();
+    for (u32 i = threadIdx.x; i < sizeof(CTableDev) / 4; i += BLOCK)
+      reinterpret_cast<u32*>(&s_c)[i] = reinterpret_cast<const u32*>(&c_table)[i];
+    __syncthreads();
+    wait_for_kernel_before();
+    u64 slots = table_mask + 1;
+    if (!table_sizes(q, sc, res_stride, n_in, slots)) return;
+    table_mask = slots - 1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      sc->t_scatter = global_ns();
+      sc->terms = q.prev->next_terms;
+    }
   }
   const u64 mask = board_mask(n);
   for (u64 i = (u64)blockIdx.x * BLOCK + threadIdx.x; i < n_in; i += (u64)gridDim.x * BLOCK) {
@@ -318,22 +323,37 @@ __global__ void __launch_bounds__(BLOCK) site_expand_insert_kernel(const void* _
     for (int r = 0; r < R; ++r) w[r] = res[r * res_stride + i];
     u32 rs;
     const u32 sig = site_signature<K>(key, n, site, &rs);
-    const u32 cnt = s_c.count[sig];
-    for (u32 e0 = 0; e0 < cnt; e0 += 2) {
-      K child[2] = {0, 0};
-      u32 cw[2][R] = {}, have = 0;
+    if constexpr (QUEUED) {
+      const u32 cnt = s_c.count[sig];
+      for (u32 e0 = 0; e0 < cnt; e0 += 2) {
+        K child[2] = {0, 0};
+        u32 cw[2][R] = {}, have = 0;
 #pragma unroll
-      for (u32 c = 0; c < 2; ++c) {
-        const u32 e = e0 + c;
-        if (e >= cnt || !site_apply<K>(key, n, site, s_c.out[sig][e], mask, &child[c])) continue;
-        have |= 1u << c;
+        for (u32 c = 0; c < 2; ++c) {
+          const u32 e = e0 + c;
+          if (e >= cnt || !site_apply<K>(key, n, site, s_c.out[sig][e], mask, &child[c])) continue;
+          have |= 1u << c;
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const u32 v = s_c.value_mod[sig][e][r];
+            cw[c][r] = v == 1u ? w[r] : mul_mod(w[r], v, prime_at(r));
+          }
+        }
+        if (have) table_insert_pair<K, R>(table, table_mask, child, cw, have, &sc->error);
+      }
+    } else {
+      const u32 cnt = c_table.count[sig];
+      for (u32 e = 0; e < cnt; ++e) {
+        K child;
+        if (!site_apply<K>(key, n, site, c_table.out[sig][e], mask, &child)) continue;
+        u32 cw[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          const u32 v = s_c.value_mod[sig][e][r];
-          cw[c][r] = v == 1u ? w[r] : mul_mod(w[r], v, prime_at(r));
+          const u32 v = c_table.value_mod[sig][e][r];
+          cw[r] = v == 1u ? w[r] : mul_mod(w[r], v, prime_at(r));
         }
+        table_insert<K, R>(table, table_mask, child, cw, kMaxProbe, &sc->error);
       }
-      if (have) table_insert_pair<K, R>(table, table_mask, child, cw, have, &sc->error);
     }
   }
 }
@@ -344,7 +364,7 @@ __global__ void __launch_bounds__(BLOCK) site_expand_insert_kernel(const void* _
 // final v1/v2 contraction (src/lib.rs:5393-5401): entries whose columns are
 // all set.
 
-template <typename K, int R, int BLOCK, int ITEMS>
+template <typename K, int R, int BLOCK, int ITEMS, bool QUEUED>
 __global__ void __launch_bounds__(BLOCK) compact_kernel(Slot<K, R>* __restrict__ table, u64 slots,
                                                         void* __restrict__ keys_out, u32* __restrict__ res_out,
                                                         u64 out_stride, unsigned n, int write_out,
@@ -356,14 +376,18 @@ __global__ void __launch_bounds__(BLOCK) compact_kernel(Slot<K, R>* __restrict__
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const u64 mask = board_mask(n);
   const u64 chunk = (u64)BLOCK * ITEMS;
-  next_kernel_may_start();
-  wait_for_kernel_before();
-  const u32 failed = *reinterpret_cast<volatile const u32*>(&sc->error);
-  {
-    u64 n_in = 0;
-    if (!table_sizes(q, sc, out_stride, n_in, slots) || failed) return;  // insertion failed: the boundary stays intact
+  if constexpr (QUEUED) {
+    next_kernel_may_start();
+    wait_for_kernel_before();
   }
-  if (q.prev && blockIdx.x == 0 && threadIdx.x == 0) sc->t_merge = global_ns();
+  // An insertion that failed leaves the boundary intact.
+  const u32 failed = *reinterpret_cast<volatile const u32*>(&sc->error);
+  if constexpr (QUEUED) {
+    u64 n_in = 0;
+    if (!table_sizes(q, sc, out_stride, n_in, slots)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !failed) sc->t_merge = global_ns();
+  }
+  if (failed) return;
   unsigned long long wsum[R], fsum[R], fstates = 0;
   unsigned long long nterms = 0, row_terms = 0, sitewise = 0;  // queued: the next site's terms, the next row's
 #pragma unroll
@@ -412,7 +436,7 @@ __global__ void __launch_bounds__(BLOCK) compact_kernel(Slot<K, R>* __restrict__
           if (full) fsum[r] += v;
         }
         fstates += full;
-        if (q.prev) {
+        if constexpr (QUEUED) {
           table[s] = Slot<K, R>{};
           if (write_out) {
             u32 rs;
@@ -535,9 +559,12 @@ cudaError_t launch_site_expand_insert(const LaunchCfg& cfg, const FrontierView& 
     using K = decltype(kz);
     constexpr int R = decltype(rz)::value;
     const unsigned grid = grid_for(n_in, kBlock, cfg.sms, 8);
-    return launch_overlapped(site_expand_insert_kernel<K, R, kBlock>, grid, kBlock, 0, stream, queued.prev != nullptr,
-                             in.keys, in.res, in.cap, n_in, n, site, reinterpret_cast<Slot<K, R>*>(table),
-                             table_slots - 1, sc, queued);
+    auto run = [&](auto* kernel) {
+      return launch_overlapped(kernel, grid, kBlock, 0, stream, queued.prev != nullptr, in.keys, in.res, in.cap, n_in, n,
+                               site, reinterpret_cast<Slot<K, R>*>(table), table_slots - 1, sc, queued);
+    };
+    return queued.prev ? run(site_expand_insert_kernel<K, R, kBlock, true>)
+                       : run(site_expand_insert_kernel<K, R, kBlock, false>);
   });
 }
 
@@ -552,9 +579,12 @@ cudaError_t launch_compact(const LaunchCfg& cfg, void* table, uint64_t table_slo
     auto run = [&](auto items) {
       constexpr int I = decltype(items)::value;
       const unsigned grid = grid_for(table_slots, kBlock * I, cfg.sms, 8);
-      return launch_overlapped(compact_kernel<K, R, kBlock, I>, grid, kBlock, 0, stream, queued.prev != nullptr,
-                               reinterpret_cast<Slot<K, R>*>(table), table_slots, out.keys, out.res, out.cap, n,
-                               write_out ? 1 : 0, sc, queued, next_site);
+      auto launch = [&](auto* kernel) {
+        return launch_overlapped(kernel, grid, kBlock, 0, stream, queued.prev != nullptr,
+                                 reinterpret_cast<Slot<K, R>*>(table), table_slots, out.keys, out.res, out.cap, n,
+                                 write_out ? 1 : 0, sc, queued, next_site);
+      };
+      return queued.prev ? launch(compact_kernel<K, R, kBlock, I, true>) : launch(compact_kernel<K, R, kBlock, I, false>);
     };
     return table_slots <= (uint64_t)cfg.sms * 8 * kBlock * 2 ? run(std::integral_constant<int, 2>())
                                                              : run(std::integral_constant<int, kCompactItems>());
