@@ -572,13 +572,13 @@ static size_t key_bytes(const Plan& p) { return (size_t)p.key_bits / 8; }
 
 // Grow front[0] to hold `need` entries, keeping the live ones. Returns false
 // when the budget cannot hold the grown buffer next to `other_bytes`.
-static bool ensure_front(Ctx& ctx, const Plan& p, DevFrontier& f, u64 need, size_t other_bytes) {
+static bool ensure_front(Ctx& ctx, const Plan& p, DevFrontier& f, u64 need, size_t other_bytes, bool grows = true) {
   if (f.cap >= need) return true;
   const size_t eb = entry_bytes(p);
   // Grow in large steps (x3, capped where the step's scratch would no longer
   // fit next to the boundary) so that a growing frontier is copied rarely.
   const u64 step_cap = (u64)((double)p.budget / ((double)eb + 1.25 * (double)cand_bytes(p)));
-  u64 want = std::max<u64>(need, std::min<u64>(need * 3, step_cap));
+  u64 want = grows ? std::max<u64>(need, std::min<u64>(need * 3, step_cap)) : need;
   const size_t live = ctx.front[0].bytes;
   if (live + want * eb + other_bytes > p.budget) want = need;
   if (live + want * eb + other_bytes > p.budget) return false;
@@ -1120,7 +1120,8 @@ static bool chain_buffers(Ctx& ctx, const Plan& p, DevFrontier& f, u64 most, siz
   if (!p.budget.known() && f.cap >= most && ctx.table.bytes >= table_bytes) return true;
   if (!p.budget.holds(std::max<u64>(f.cap, most) * entry_bytes(p) + table_bytes + (1u << 20))) return false;
   if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
-  if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes)) return false;
+  // (A large chain's boundary is sized for its largest row.)
+  if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes, most <= kQueueTerms)) return false;
   return p.budget.holds(ctx.pool_bytes - ctx.table.bytes + table_bytes);
 }
 
