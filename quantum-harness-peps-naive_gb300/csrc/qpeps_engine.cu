@@ -614,6 +614,32 @@ static bool ensure_front(Ctx& ctx, const Plan& p, DevFrontier& f, u64 need, size
   return true;
 }
 
+// Give back what front[0] holds beyond `need` entries (a buffer of an earlier
+// call, larger than a small budget can keep beside a step's scratch). The live
+// entries move through the host: the two buffers together would pass the
+// budget.
+static void shrink_front(Ctx& ctx, const Plan& p, DevFrontier& f, u64 need) {
+  const size_t kb = key_bytes(p), eb = entry_bytes(p);
+  std::vector<char> live(f.count * eb);
+  const char* src = static_cast<const char*>(ctx.front[0].ptr);
+  char* dst = live.data();
+  auto parts = [&](auto&& copy, u64 cap) {
+    copy(0, 0, f.count * kb);
+    for (int r = 0; r < p.R; ++r) copy(f.count * kb + (size_t)r * f.count * 4, cap * kb + (size_t)r * cap * 4, f.count * 4);
+  };
+  cuda_check(cudaStreamSynchronize(ctx.stream), "shrink synchronize");
+  parts([&](size_t host, size_t dev, size_t bytes) {
+    cuda_check(cudaMemcpy(dst + host, src + dev, bytes, cudaMemcpyDeviceToHost), "save boundary");
+  }, f.cap);
+  buf_release(ctx, ctx.front[0]);
+  buf_reserve(ctx, ctx.front[0], need * eb, p.budget, "boundary");
+  f.cap = ctx.front[0].bytes / eb;
+  char* to = static_cast<char*>(ctx.front[0].ptr);
+  parts([&](size_t host, size_t dev, size_t bytes) {
+    cuda_check(cudaMemcpy(to + dev, dst + host, bytes, cudaMemcpyHostToDevice), "restore boundary");
+  }, f.cap);
+}
+
 static u64 count_terms(Ctx& ctx, const Plan& p, const DevFrontier& f, bool site, unsigned site_idx, RunStats& rs) {
   if (f.count == 0) return 0;
   LaunchCfg cfg{p.key_bits, p.R, p.threads, ctx.sms};
@@ -742,6 +768,11 @@ static StepStatus merge_step(Ctx& ctx, const Plan& p, DevFrontier& f, bool site,
       table_bytes = slots * slot_bytes(p.key_bits, p.R);
     }
     const u64 need_cap = final_step ? n_in : std::max<u64>(n_in, so.terms);
+    if (f.cap > need_cap && f.cap * eb + table_bytes > p.budget && need_cap * eb * 5 / 4 + table_bytes <= p.budget &&
+        f.count <= need_cap) {
+      buf_release(ctx, ctx.table);
+      shrink_front(ctx, p, f, need_cap);
+    }
     if (std::max<u64>(f.cap, need_cap) * eb + table_bytes > p.budget) {
       if (n_in <= 1) fail(QPEPS_ERR_CAPACITY, row_msg("device budget exceeded at row", row + 1));
       return StepStatus::NeedSplit;
@@ -1495,15 +1526,26 @@ struct GroupSeed {
 // under memory pressure): they take the partitioned merge.
 constexpr u64 kGroupMaxSeeds = 4096;
 
+// Top u bits implied by the bucket, so that the stored diagonals fit 32 bits.
+static unsigned group_implied_bits(unsigned n) { return 2 * n - 2 > 32 ? 2 * n - 2 - 32 : 0; }
+
 // Expected largest boundary that column-grouped rows are to hold, 0 where the
-// partitioned rows are faster. Device ms at N = 15 / 16 / 17 / 18 (peaks of 18,
-// 106 and 706 M entries; nine batches of 380 to 743 M): grouped 1.96 / 8.3 /
-// 53.4 / 481, partitioned 2.43 / 15.6 / 117 / 821; at N = 14 (2.8 M) the
-// partitioned rows' traffic stays in L2 and the grouped ones' smallest units are
-// nearly empty. Repeated contractions (use_graph) keep the rows that a graph can
-// replay up to 200 M entries. `room`: the buffers' size over the expected one.
-static double group_rows_states(double states, double room, bool replay) {
-  return states >= (replay ? 200e6 : 10e6) ? states * room : 0.0;
+// partitioned rows are faster. A row costs about 2 us a CTA and bucket besides
+// its entries, so the line lies at 1200 expected entries a bucket: `states` over
+// the column sets of the board's middle (C(N - k, (N - k) / 2) below k placed
+// rows) and the buckets a set has at least. Device ms at N = 15 / 16 / 17 / 18
+// (2.8, 8.2, 29 and 4.9 K entries a bucket): grouped 1.96 / 8.3 / 53.4 / 481,
+// partitioned 2.4 / 15.6 / 117 / 821; N = 14 without the orbits (1.7 K) 0.90
+// against 1.08, N = 16 below one row (2 K) 1.75 to 2.04 against 1.67 to 2.32;
+// N = 14 (0.8 K) 0.70 against 0.53, N = 18 below two rows (0.6 K) 5.4 to 7.2
+// against 3.8 to 8.2. Repeated contractions (use_graph) keep the rows that a
+// graph can replay up to 200 M entries. `room`: the buffers' size over the
+// expected one.
+static double group_rows_states(unsigned n, unsigned placed, double states, double room, bool replay) {
+  if (n > kGroupMaxN) return 0.0;
+  const unsigned left = n - std::min(placed, n);
+  const double buckets = (double)kBinomials.at(left, left / 2) * (1u << group_implied_bits(n));
+  return states >= std::max(1200.0 * buckets, replay ? 200e6 : 0.0) ? states * room : 0.0;
 }
 
 static bool group_applies(const Ctx& ctx, const Plan& p, const HostChunk& hc) {
@@ -1519,9 +1561,6 @@ static bool group_applies(const Ctx& ctx, const Plan& p, const HostChunk& hc) {
          (p.R == 1 || std::all_of(hc.res.begin() + hc.count, hc.res.begin() + 2 * hc.count,
                                   [](u32 high) { return high == 0; }));
 }
-
-// Top u bits implied by the bucket, so that the stored diagonals fit 32 bits.
-static unsigned group_implied_bits(unsigned n) { return 2 * n - 2 > 32 ? 2 * n - 2 - 32 : 0; }
 
 static GroupSeed group_seed(const Plan& p, const HostChunk& hc) {
   const unsigned n = p.n, rm = group_implied_bits(n), nu = n - 1 - rm;
@@ -2960,8 +2999,8 @@ static void contract_impl(Ctx& ctx, unsigned n, const qpeps_options& o, const ui
   // estimated below a prefix.)
   out.plan.batch_states = serve_estimate(n, k) * (k ? 3.0 : o.symmetry ? 1.0 : 2.0);
   out.plan.prefix = k > 0;
-  if (n <= kGroupMaxN)
-    out.plan.group_states = group_rows_states(out.plan.batch_states / (k ? 3.0 : 1.0), k ? 3.0 : 1.01, o.use_graph);
+  out.plan.group_states =
+      group_rows_states(n, k, out.plan.batch_states / (k ? 3.0 : 1.0), k ? 3.0 : 1.01, o.use_graph);
   // Predictive slicing: when the merged frontier is estimated not to fit the
   // device budget, contract groups of slices (first-row orbit slices, or
   // deeper prefix slices) one chunk at a time instead of halving a live
@@ -2987,9 +3026,8 @@ static void contract_impl(Ctx& ctx, unsigned n, const qpeps_options& o, const ui
         }
         out.slice_depth = row0;
         out.plan.batch_states = std::min(est_item * (double)per_chunk, cap_states);
-        if (n <= kGroupMaxN)
-          out.plan.group_states = group_rows_states(est_total / (double)items.size() * (double)per_chunk,
-                                                    std::min(2.5, ctx.tune.slice_margin), o.use_graph);
+        out.plan.group_states = group_rows_states(n, k, est_total / (double)items.size() * (double)per_chunk,
+                                                  std::min(2.5, ctx.tune.slice_margin), o.use_graph);
         run_chunks(ctx, out.plan, std::move(chunks), out.rows, out.rs);
         items.clear();
         break;
