@@ -1,4 +1,4 @@
-"""Column-grouped rows (boundaries beyond 10 M entries, up to N = 18) against
+"""Column-grouped rows (large boundaries, up to N = 18) against
 the partitioned rows, which run with the direct scatter: every row's metrics,
 the peak and the count are equal."""
 from __future__ import annotations
