@@ -616,28 +616,36 @@ static bool ensure_front(Ctx& ctx, const Plan& p, DevFrontier& f, u64 need, size
 
 // Give back what front[0] holds beyond `need` entries (a buffer of an earlier
 // call, larger than a small budget can keep beside a step's scratch). The live
-// entries move through the host: the two buffers together would pass the
-// budget.
-static void shrink_front(Ctx& ctx, const Plan& p, DevFrontier& f, u64 need) {
+// entries move through the host, on the context's stream like everything that
+// reads them: the two buffers together would pass the budget. False, with
+// nothing changed, when the budget does not hold the smaller buffer beside the
+// pool's others.
+static bool shrink_front(Ctx& ctx, const Plan& p, DevFrontier& f, u64 need) {
   const size_t kb = key_bytes(p), eb = entry_bytes(p);
+  const auto fits = [&] { return ctx.pool_bytes - ctx.front[0].bytes + need * eb <= p.budget; };
+  if (!fits() && !(group_release(ctx) && fits())) return false;
   std::vector<char> live(f.count * eb);
-  const char* src = static_cast<const char*>(ctx.front[0].ptr);
-  char* dst = live.data();
-  auto parts = [&](auto&& copy, u64 cap) {
-    copy(0, 0, f.count * kb);
-    for (int r = 0; r < p.R; ++r) copy(f.count * kb + (size_t)r * f.count * 4, cap * kb + (size_t)r * cap * 4, f.count * 4);
+  const auto move = [&](bool save) {
+    char* const dev = static_cast<char*>(ctx.front[0].ptr);
+    size_t at = 0;
+    const auto part = [&](size_t off, size_t bytes) {
+      char* const host = live.data() + at;
+      cuda_check(save ? cudaMemcpyAsync(host, dev + off, bytes, cudaMemcpyDeviceToHost, ctx.stream)
+                      : cudaMemcpyAsync(dev + off, host, bytes, cudaMemcpyHostToDevice, ctx.stream),
+                 save ? "save boundary" : "restore boundary");
+      at += bytes;
+    };
+    part(0, f.count * kb);
+    for (int r = 0; r < p.R; ++r) part(f.cap * kb + (size_t)r * f.cap * 4, f.count * 4);
+    cuda_check(cudaStreamSynchronize(ctx.stream), "shrink synchronize");
+    (save ? ctx.d2h_bytes : ctx.h2d_bytes) += at;
   };
-  cuda_check(cudaStreamSynchronize(ctx.stream), "shrink synchronize");
-  parts([&](size_t host, size_t dev, size_t bytes) {
-    cuda_check(cudaMemcpy(dst + host, src + dev, bytes, cudaMemcpyDeviceToHost), "save boundary");
-  }, f.cap);
+  move(true);
   buf_release(ctx, ctx.front[0]);
   buf_reserve(ctx, ctx.front[0], need * eb, p.budget, "boundary");
   f.cap = ctx.front[0].bytes / eb;
-  char* to = static_cast<char*>(ctx.front[0].ptr);
-  parts([&](size_t host, size_t dev, size_t bytes) {
-    cuda_check(cudaMemcpy(to + dev, dst + host, bytes, cudaMemcpyHostToDevice), "restore boundary");
-  }, f.cap);
+  move(false);
+  return true;
 }
 
 static u64 count_terms(Ctx& ctx, const Plan& p, const DevFrontier& f, bool site, unsigned site_idx, RunStats& rs) {

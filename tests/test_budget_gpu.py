@@ -1,0 +1,56 @@
+"""Calls with a device budget on a context that keeps larger buffers of an
+earlier call: equal results, and no more memory held than the budget."""
+from __future__ import annotations
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("row", "input_states", "row_operator_candidates", "row_operator_matched", "completed_row_terms",
+          "output_states", "output_weight")
+
+
+@pytest.fixture()
+def fresh(qp):
+    c = qp.Context(0)
+    yield c
+    c.close()
+
+
+def _layers(r):
+    return [tuple(getattr(l, f) for f in FIELDS) for l in r.layers]
+
+
+def _held(r):
+    return r.layers[-1].peak_rss_bytes
+
+
+# A kept boundary buffer (540 MiB, of N = 15 row by row) that the budget holds
+# but not beside a row's scratch: the live boundary moves into a smaller one
+# through the host, which the bytes copied show. The call after it finds the
+# context as any other.
+@pytest.mark.parametrize("budget", [541, 544])
+def test_a_kept_boundary_gives_way(fresh, qp, budget):
+    c = qp.Context(0)
+    try:
+        c.set_tuning(scatter_kind=qp.SCATTER_DIRECT)
+        c.contract_rows(15)
+        for again in (False, True):
+            g = c.contract_rows(14, symmetry=0, device_budget_bytes=budget << 20)
+            assert _layers(g) == _layers(fresh.contract_rows(14, symmetry=0))
+            assert _held(g) <= budget << 20
+            if not again:
+                assert min(g.device["h2d_bytes"], g.device["d2h_bytes"]) > 1 << 20
+        assert _layers(c.contract_rows(13)) == _layers(fresh.contract_rows(13))
+    finally:
+        c.close()
+
+
+# Budgets that hold neither form's buffers of the whole board, or the grouped
+# rows but not beside what the context already keeps.
+@pytest.mark.parametrize("budget", [1 << 30, 3 << 30])
+def test_held_memory_stays_within_the_budget(fresh, qp, budget):
+    fresh.contract_rows(16)
+    g = fresh.contract_rows(16, device_budget_bytes=budget)
+    assert g.count == qp.known_count(16)
+    assert _held(g) <= budget
