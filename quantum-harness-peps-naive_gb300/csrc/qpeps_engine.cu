@@ -1123,14 +1123,9 @@ static StepScalars* pinned_scalars(Ctx& ctx, size_t steps) {
   return ctx.h_queue;
 }
 
-// The same with their copy on the device.
-static StepScalars* queue_scalars(Ctx& ctx, const Plan& p, size_t steps) {
+// The same with their copy on the device (chain_buffers has made its room).
+static StepScalars* queue_scalars(Ctx& ctx, size_t steps) {
   pinned_scalars(ctx, steps);
-  // No captured graph holds this buffer (a replay has scalars of its own), so
-  // its growth does not end one.
-  const uint64_t gen = ctx.pool_gen;
-  buf_reserve(ctx, ctx.queue, (steps + 1) * sizeof(StepScalars), p.budget, "queued step scalars");
-  ctx.pool_gen = gen;
   return static_cast<StepScalars*>(ctx.queue.ptr);
 }
 
@@ -1153,15 +1148,37 @@ static QueueTimes queue_times(const StepScalars* h, size_t steps, double total) 
   return t;
 }
 
-// Room for a chain: a boundary of `most` entries and `table_bytes` of scratch.
-// Buffers that stand are not asked about again.
-static bool chain_buffers(Ctx& ctx, const Plan& p, DevFrontier& f, u64 most, size_t table_bytes) {
-  if (!p.budget.known() && f.cap >= most && ctx.table.bytes >= table_bytes) return true;
-  if (!p.budget.holds(std::max<u64>(f.cap, most) * entry_bytes(p) + table_bytes + (1u << 20))) return false;
+// buf_reserve's answer instead of its exception.
+static bool try_reserve(Ctx& ctx, DevBuf& b, size_t bytes, const Budget& budget, const char* what) {
+  try {
+    buf_reserve(ctx, b, bytes, budget, what);
+    return true;
+  } catch (const Failure& e) {
+    if (e.code != QPEPS_ERR_CAPACITY) throw;
+    return false;
+  }
+}
+
+// Room for a chain of `steps` steps: their scalars, a boundary of `most`
+// entries and `table_bytes` of scratch, or false. Buffers that stand are not
+// asked about again.
+static bool chain_buffers(Ctx& ctx, const Plan& p, DevFrontier& f, u64 most, size_t table_bytes, size_t steps,
+                          const char* what) {
+  const size_t scalar_bytes = (steps + 1) * sizeof(StepScalars);
+  if (!p.budget.known() && f.cap >= most && ctx.table.bytes >= table_bytes && ctx.queue.bytes >= scalar_bytes) return true;
+  if (!p.budget.holds(std::max<u64>(f.cap, most) * entry_bytes(p) + table_bytes + scalar_bytes)) return false;
   if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
+  // The scalars come before the table, which takes what is left of the budget
+  // up to a quarter more than it needs. No captured graph holds their buffer (a
+  // replay has scalars of its own), so its growth does not end one.
+  const uint64_t gen = ctx.pool_gen;
+  const bool scalars = try_reserve(ctx, ctx.queue, scalar_bytes, p.budget, "queued step scalars");
+  ctx.pool_gen = gen;
+  if (!scalars) return false;
   // (A large chain's boundary is sized for its largest row.)
   if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes, most <= kQueueTerms)) return false;
-  return p.budget.holds(ctx.pool_bytes - ctx.table.bytes + table_bytes);
+  return p.budget.holds(ctx.pool_bytes - ctx.table.bytes + table_bytes) &&
+         try_reserve(ctx, ctx.table, table_bytes, p.budget, what);
 }
 
 // A finished row's metrics: `in` entries with `terms` successors. `exact`:
@@ -1282,9 +1299,8 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   const size_t region_bytes = (size_t)parts_cap * pcap * cand_bytes(p);
   const size_t cursor_bytes = (size_t)parts_cap * 4 * cstride;
   const size_t table_bytes = region_bytes + (cursor_bytes + 255) / 256 * 256;
-  if (!chain_buffers(ctx, p, f, most, table_bytes)) return 0;
-  buf_reserve(ctx, ctx.table, table_bytes, p.budget, "partition regions");
-  StepScalars* d = queue_scalars(ctx, p, count);
+  if (!chain_buffers(ctx, p, f, most, table_bytes, count, "partition regions")) return 0;
+  StepScalars* d = queue_scalars(ctx, count);
   StepScalars* h = ctx.h_queue;
   const auto t0 = std::chrono::steady_clock::now();
   h[0].out_count = f.count;
@@ -1414,10 +1430,9 @@ static u64 run_queued_sites_plain(Ctx& ctx, const Plan& p, DevFrontier& f, unsig
   TableSource source;
   source.slots_cap = source.slots(most);
   const size_t table_bytes = source.slots_cap * slot_bytes(p.key_bits, p.R);
-  if (!chain_buffers(ctx, p, f, most, table_bytes)) return 0;
-  buf_reserve(ctx, ctx.table, table_bytes, p.budget, "hash table");
   const size_t sites = (size_t)count * p.n;
-  StepScalars* d = queue_scalars(ctx, p, sites);
+  if (!chain_buffers(ctx, p, f, most, table_bytes, sites, "hash table")) return 0;
+  StepScalars* d = queue_scalars(ctx, sites);
   StepScalars* h = ctx.h_queue;
   const auto t0 = std::chrono::steady_clock::now();
   h[0].out_count = f.count;
@@ -2246,10 +2261,8 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
   const size_t region_bytes = (size_t)parts_cap * pcap * cand_bytes(p);
   const size_t cursor_bytes = (size_t)parts_cap * 4 * cstride;
   const size_t table_bytes = region_bytes + (cursor_bytes + 255) / 256 * 256;
-  const size_t eb = entry_bytes(p);
-  if (count < 2 || f.count > most || !chain_buffers(ctx, p, f, most, table_bytes)) return 0;
-  buf_reserve(ctx, ctx.table, table_bytes, p.budget, "partition regions");
-  StepScalars* d = queue_scalars(ctx, p, count);
+  if (count < 2 || f.count > most || !chain_buffers(ctx, p, f, most, table_bytes, count, "partition regions")) return 0;
+  StepScalars* d = queue_scalars(ctx, count);
   StepScalars* h = ctx.h_queue;
   h[0].out_count = f.count;
   void* regions = ctx.table.ptr;
@@ -3351,9 +3364,8 @@ static unsigned serve_steps(Ctx& ctx, const Plan& p, DevFrontier& f, u64& terms,
     const size_t region_bytes = (size_t)parts_cap * pcap * cand_bytes(p);
     const size_t cursor_bytes = (size_t)parts_cap * 4 * 8;
     const size_t table_bytes = region_bytes + (cursor_bytes + 255) / 256 * 256;
-    if (chain_buffers(ctx, p, f, most, table_bytes)) {
-      buf_reserve(ctx, ctx.table, table_bytes, p.budget, "serve partitions");
-      StepScalars* d = queue_scalars(ctx, p, want);
+    if (chain_buffers(ctx, p, f, most, table_bytes, want, "serve partitions")) {
+      StepScalars* d = queue_scalars(ctx, want);
       StepScalars* h = ctx.h_queue;
       h[0].out_count = f.count;
       h[0].next_terms = terms;

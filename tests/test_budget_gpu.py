@@ -54,3 +54,15 @@ def test_held_memory_stays_within_the_budget(fresh, qp, budget):
     g = fresh.contract_rows(16, device_budget_bytes=budget)
     assert g.count == qp.known_count(16)
     assert _held(g) <= budget
+
+
+# Budgets that hold a chain's boundary and its scratch, at a quarter more than
+# the scratch needs, but not the few KB of its scalars beside them (on 152 SMs).
+@pytest.mark.parametrize("n,budget,opts", [
+    (11, 40517584, {}), (13, 45581584, {}), (11, 75892560, {"key_bits": 128}),
+    (12, 26845824, {"granularity": 1}), (12, 33565824, {"granularity": 1}),
+])
+def test_chain_scalars_fit_a_tight_budget(fresh, qp, n, budget, opts):
+    g = fresh.contract_rows(n, device_budget_bytes=budget, **opts)
+    assert g.count == qp.known_count(n)
+    assert _held(g) <= budget
