@@ -285,7 +285,7 @@ enum ErrorBits : u32 {
   kErrOverflow = 2u,    // a bounded structure overflowed its capacity
   kErrWaitLimit = 4u,   // a bounded spin-wait gave up
   kErrBounds = 8u,      // an index fell outside its buffer; the access was skipped
-  kErrSkipped = 16u,    // queued step: an earlier step of the chain failed
+  kErrSkipped = 16u,    // queued step: an earlier step of the chain failed or passed the support limit
   kErrCapacity = 32u,   // queued step: its terms do not fit the buffers
   kErrNeedWide = 64u,   // grouped row: its weights may pass 32 bits
 };
@@ -314,8 +314,9 @@ __device__ __forceinline__ bool step_sizes(const Source& q, Scalars* sc, u64 cap
   const u32 error = q.prev->error;
   const u64 terms = q.prev->next_terms, entries = q.prev->out_count;
   const u64 p = q.partitions(terms);
-  if (error || p > q.parts_cap || terms > cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->error, (u32)(error ? kErrSkipped : kErrCapacity));
+  const bool skip = error || entries > q.limit;
+  if (skip || p > q.parts_cap || terms > cap) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->error, (u32)(skip ? kErrSkipped : kErrCapacity));
     return false;
   }
   n_in = terms ? entries : 0;

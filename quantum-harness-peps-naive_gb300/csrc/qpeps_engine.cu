@@ -2242,20 +2242,36 @@ static u64 explicit_partition_step(Ctx& ctx, const Plan& p, DevFrontier& f, cons
   }
 }
 
-// Site steps [0, count) of the explicit-C frontier as a chain (run_queued_rows
-// above has the idea), from the seed boundary. Returns the steps contracted:
-// count, or the first one that did not fit the chain's buffers (or whose
-// scalars the caller stops at); their scalars are in ctx.h_queue[1 ..].
+// Steps of a chain that may stop at the support limit, at most: the launches
+// queued behind the site that passes it return at once, but take 2 us each all
+// the same (N = 20 in one chain: 10.5 ms for a limit of one entry). Fewer where
+// the boundary is near the limit: a site at most doubles it, and grows it by
+// half that in the logarithm on average.
+constexpr size_t kLimitedChain = 16;
+
+// Site steps [first, end) of the explicit-C frontier as a chain
+// (run_queued_rows above has the idea), fewer where the support limit may stop
+// it; `known_terms`: the first step's matches, kTermsUnknown to count them.
+// Returns the steps contracted, the one that passes the limit included; their
+// scalars are in ctx.h_queue[1 ..], the first step's matches in [0]. Fewer than
+// `queued` (the steps the chain had): the next one did not fit its buffers.
 static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const std::vector<FrontierStepDev>& steps,
-                               const FrontierStepDev* d_steps, const std::vector<size_t>& open_after, size_t count,
-                               ExplicitRun& out) {
+                               const FrontierStepDev* d_steps, const std::vector<size_t>& open_after, size_t first,
+                               size_t end, u64 support_limit, u64 known_terms, ExplicitRun& out, size_t& queued) {
   // Largest boundaries: 1.3 M entries at N = 12 (diamond), times about 5.8 per
-  // size; at most two matches an entry.
+  // size; at most two matches an entry, of which at most `support_limit` stand.
   const double states = 1.4e6 * std::pow(5.8, (double)p.n - 12.0);
-  const u64 most = (u64)std::min((double)kQueueTerms, std::max(65536.0, 1.8 * states));
+  const double limit = (double)support_limit;
+  const u64 most = (u64)std::min({(double)kQueueTerms, std::max(65536.0, 1.8 * states), 2.0 * limit + 1024.0});
+  size_t count = end - first;
+  if (limit < 2.0 * states) {
+    const double doublings = std::log2(limit / (double)std::max<u64>(f.count, 1));
+    count = std::min({count, kLimitedChain, (size_t)(2.0 + 2.0 * doublings)});
+  }
+  queued = count;
   const u32 pcap = wide_key_partition_capacity();
   const double mean = ctx.partition_fill * pcap;
-  StepSource source{nullptr, mean, 0, 2 * (u32)ctx.sms};
+  StepSource source{nullptr, mean, 0, 2 * (u32)ctx.sms, support_limit};
   const u32 parts_cap = source.parts_cap = (u32)source.partitions(most);
   const u32 cstride = (parts_cap <= ctx.tune.spread_cursors_below) ? 8u : 1u;
   const size_t region_bytes = (size_t)parts_cap * pcap * cand_bytes(p);
@@ -2265,6 +2281,7 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
   StepScalars* d = queue_scalars(ctx, count);
   StepScalars* h = ctx.h_queue;
   h[0].out_count = f.count;
+  if (known_terms != kTermsUnknown) h[0].next_terms = known_terms;
   void* regions = ctx.table.ptr;
   u32* cursors = reinterpret_cast<u32*>(static_cast<char*>(ctx.table.ptr) + region_bytes);
   const FrontierView view = view_of(p, ctx.front[0], f.cap);
@@ -2279,7 +2296,10 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
              "queued step scalars");
   cuda_check(cudaMemsetAsync(cursors, 0, cursor_bytes, ctx.stream), "clear partition cursors");
   cuda_check(cudaEventRecord(ctx.ev[0], ctx.stream), "event");
-  cuda_check(launch_frontier_count(view, f.count, steps[0], ctx.sms, d, ctx.stream), "frontier count kernel");
+  if (known_terms == kTermsUnknown) {
+    cuda_check(launch_frontier_count(view, f.count, steps[first], ctx.sms, d, ctx.stream), "frontier count kernel");
+    out.launches += 1;
+  }
   u64 entries = f.count;
   for (size_t i = 0; i < count; ++i) {
     const u64 fits = std::min(most, 2 * entries);  // at most two matches an entry
@@ -2288,11 +2308,13 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
     pc.parts = (u32)source.partitions(fits);
     // The merge counts the next step's matches, for the chain or the step that
     // follows it.
-    const bool next = i + 1 < steps.size() && open_after[i + 1] < 128;
-    cuda_check(launch_frontier_partition_scatter(pc, view, entries, d_steps + i, regions, cursors, d + i + 1, ctx.stream),
+    const size_t after = first + i + 1;
+    const bool next = after < steps.size() && open_after[after] < 128;
+    cuda_check(launch_frontier_partition_scatter(pc, view, entries, d_steps + first + i, regions, cursors, d + i + 1,
+                                                 ctx.stream),
                "frontier scatter kernel");
     cuda_check(launch_wide_partition_merge(pc, regions, cursors, view, 0, true, d + i + 1, ctx.stream,
-                                           next ? d_steps + i + 1 : nullptr),
+                                           next ? d_steps + after : nullptr),
                "frontier merge kernel");
     entries = fits;
   }
@@ -2302,7 +2324,7 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
   cuda_check(cudaStreamSynchronize(ctx.stream), "queued sites");
   ctx.h2d_bytes += (count + 1) * sizeof(StepScalars);
   ctx.d2h_bytes += (count + 1) * sizeof(StepScalars);
-  out.launches += 1 + 2 * count;
+  out.launches += 2 * count;
   float ms = 0;
   cudaEventElapsedTime(&ms, ctx.ev[0], ctx.ev[1]);
   out.device_ms += ms;
@@ -2484,18 +2506,22 @@ static void explicit_frontier(Ctx& ctx, unsigned n, unsigned order, u64 support_
     out.peak_states = std::max<u64>(out.peak_states, merged);
     return true;
   };
-  size_t chained = 0;  // leading steps that can be queued as a chain
+  // Leading steps that can be queued run as chains, until one does not fit.
+  size_t chainable = 0, step = 0;
   if (partitioned && d_steps)
-    while (chained < total && chained != fail_step && open_after[chained] < 128) ++chained;
-  chained = chained ? run_queued_sites(ctx, p, f, steps, d_steps, open_after, chained, out) : 0;
-  for (size_t step = 0; step < chained; ++step) {
-    const StepScalars& sc = ctx.h_queue[step + 1];
-    out.examined += (u128)f.count * 17;
-    out.accepted += ctx.h_queue[step].next_terms;
-    if (!merged_step(step, sc)) return;
-    known_terms = sc.next_terms_ok ? sc.next_terms : kTermsUnknown;
+    while (chainable < total && chainable != fail_step && open_after[chainable] < 128) ++chainable;
+  for (size_t queued = 0, done = 0; step < chainable && done == queued;) {
+    done = run_queued_sites(ctx, p, f, steps, d_steps, open_after, step, chainable, support_limit, known_terms, out,
+                            queued);
+    for (size_t i = 0; i < done; ++i, ++step) {
+      const StepScalars& sc = ctx.h_queue[i + 1];
+      out.examined += (u128)f.count * 17;
+      out.accepted += ctx.h_queue[i].next_terms;
+      if (!merged_step(step, sc)) return;
+      known_terms = sc.next_terms_ok ? sc.next_terms : kTermsUnknown;
+    }
   }
-  for (size_t step = chained; step < total; ++step) {
+  for (; step < total; ++step) {
     if (step == fail_step) fail(fail_code, fail_msg);
     const FrontierStepDev& st = steps[step];
     const size_t next_open = open_after[step];

@@ -52,6 +52,7 @@ struct StepSource {
   double mean = 0;                    // planned candidates per partition
   uint32_t parts_cap = 0;             // partitions the regions hold
   uint32_t spread = 1;                // partitions of a small step, one for each merge CTA the device holds
+  uint64_t limit = ~0ull;             // entries a boundary may have: the chain ends behind a larger one
 
   // Partitions of a step. A small step takes more of them than its candidates
   // fill: with 60 partitions for 100 K candidates the cursor atomics queue up
