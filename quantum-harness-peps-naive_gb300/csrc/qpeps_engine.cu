@@ -278,6 +278,7 @@ struct Ctx {
   CTableDev c_dev;
   bool c_uploaded = false;
   double partition_fill = 0.83;  // live target candidates per partition / slots (lowered after an overflow)
+  double chain_fill = 1.0;       // the same of queued steps, where it is lower
   uint64_t h2d_bytes = 0, d2h_bytes = 0;  // host<->device copies issued (since context creation)
   struct Tune {
     uint32_t parents_per_lane = 4;              // partition scatter: 2 or 4
@@ -1181,6 +1182,23 @@ static bool chain_buffers(Ctx& ctx, const Plan& p, DevFrontier& f, u64 most, siz
          try_reserve(ctx, ctx.table, table_bytes, p.budget, what);
 }
 
+// Planned candidates per partition of a queued step. A partition that overflows
+// ends the chain, and its row runs again by itself, so a fill meant for rows
+// that stand alone is held six standard deviations (a partition's candidates
+// are about Poisson) below the capacity: 849 of 1024 slots, where a fill of 0.9
+// plans 922 and fails nearly every row of millions of terms (N = 14: 61
+// launches instead of 27).
+static double chain_mean(const Ctx& ctx, u32 pcap) {
+  const double root = std::sqrt(9.0 + (double)pcap) - 3.0;  // mean + 6 sqrt(mean) = pcap
+  return std::min(std::min(ctx.partition_fill, ctx.chain_fill) * pcap, root * root);
+}
+
+// What a chain learns from the step that ended it: a wider margin where one of
+// its partitions overflowed all the same.
+static void chain_ended(Ctx& ctx, const StepScalars& failed, double mean, u32 pcap) {
+  if (failed.error & kErrOverflow) ctx.chain_fill = std::max(0.3, 0.8 * mean / pcap);
+}
+
 // A finished row's metrics: `in` entries with `terms` successors. `exact`:
 // plane 0 carries exact sums.
 static void add_row(const Plan& p, unsigned row, u64 in, u64 terms, const StepScalars& r, bool exact,
@@ -1292,7 +1310,7 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   // (Large rows scatter faster into half as many partitions.)
   const u32 shape = !wkeys && !large && wide_merge_supported(p.R) ? 2u : 0u;
   const u32 pcap = wkeys ? wide_key_partition_capacity() : partition_capacity(shape);
-  const double mean = ctx.partition_fill * pcap;
+  const double mean = chain_mean(ctx, pcap);
   StepSource source{nullptr, mean, 0, (shape == 2 ? 8u : 2u) * (u32)ctx.sms};
   const u32 parts_cap = source.parts_cap = (u32)source.partitions(most);
   const u32 cstride = (parts_cap <= ctx.tune.spread_cursors_below) ? 8u : 1u;
@@ -1352,6 +1370,7 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   rs.device_ms += ms;
   unsigned done = 0;
   while (done < count && !h[done + 1].error) ++done;
+  if (done < count) chain_ended(ctx, h[done + 1], mean, pcap);
   if (done < count && (h[done + 1].error & kErrBounds))
     fail(QPEPS_ERR_CUDA, row_msg("a kernel's bounds check failed (access skipped) at row", row + done + 1));
   const QueueTimes times = queue_times(h, done, ms);
@@ -2270,7 +2289,7 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
   }
   queued = count;
   const u32 pcap = wide_key_partition_capacity();
-  const double mean = ctx.partition_fill * pcap;
+  const double mean = chain_mean(ctx, pcap);
   StepSource source{nullptr, mean, 0, 2 * (u32)ctx.sms, support_limit};
   const u32 parts_cap = source.parts_cap = (u32)source.partitions(most);
   const u32 cstride = (parts_cap <= ctx.tune.spread_cursors_below) ? 8u : 1u;
@@ -2330,6 +2349,7 @@ static size_t run_queued_sites(Ctx& ctx, const Plan& p, DevFrontier& f, const st
   out.device_ms += ms;
   size_t done = 0;
   while (done < count && !h[done + 1].error) ++done;
+  if (done < count) chain_ended(ctx, h[done + 1], mean, pcap);
   if (done < count && (h[done + 1].error & kErrBounds))
     fail(QPEPS_ERR_CUDA, "explicit-C frontier: a kernel's bounds check failed (access skipped)");
   return done;
@@ -3380,7 +3400,7 @@ static unsigned serve_steps(Ctx& ctx, const Plan& p, DevFrontier& f, u64& terms,
   }
   const u32 shape = 2;  // small merge CTAs, as in run_queued_rows
   const u32 pcap = partition_capacity(shape);
-  double mean = ctx.partition_fill * pcap;
+  double mean = chain_mean(ctx, pcap);
   StepSource source{nullptr, mean, 0, 8 * (u32)ctx.sms};
   if (want > 1 && terms <= kQueueTerms) {
     // A row multiplies the terms by less than 4 on average once three rows are
@@ -3425,6 +3445,7 @@ static unsigned serve_steps(Ctx& ctx, const Plan& p, DevFrontier& f, u64& terms,
         f.count = h[done].out_count;
         terms = h[done].next_terms;
       }
+      if (done < want) chain_ended(ctx, h[done + 1], mean, pcap);
       if (done < want && (h[done + 1].error & kErrBounds)) fail(QPEPS_ERR_CUDA, "serving: a bounds check failed");
       if (done) return done;
     }
@@ -3449,6 +3470,7 @@ static unsigned serve_steps(Ctx& ctx, const Plan& p, DevFrontier& f, u64& terms,
     sync_scalars(ctx);
     if (ctx.h_sc->error & kErrOverflow) {
       if (attempt >= 4) fail(QPEPS_ERR_CAPACITY, "serving partition overflow persists");
+      chain_ended(ctx, *ctx.h_sc, mean, pcap);
       mean *= 0.6;
       continue;
     }
@@ -3794,6 +3816,7 @@ static Ctx::Tune tune_from(const qpeps_tuning& q) {
 static void apply_tune(Ctx& c, const Ctx::Tune& t) {
   c.tune = t;
   c.partition_fill = t.partition_fill;
+  c.chain_fill = 1.0;
 }
 
 // Autotuner: coordinate descent over the knobs of a contraction, starting
