@@ -362,9 +362,8 @@ def run_ours(args):
     kind = tuning.get("scatter_kind")
     # The capture behind the factor is of the u64 row path's scatter and merge.
     u64_rows = d["merge"] == 2 and args.grain == "row" and d["key_bits"] == 64
-    # Column-grouped rows report their plan kernels as the scatter: 1 % of the
-    # time, where a scatter is two thirds.
-    grouped = u64_rows and d["scatter_kernel_ms"] < 0.1 * d["merge_kernel_ms"]
+    # (A batch handed back to the partitioned rows would leave both forms' bits.)
+    grouped = d["row_forms"] == pkg.ROWS_GROUPED
     tpb = (GROUPED_TRAFFIC_PER_ALGORITHMIC_BYTE if grouped
            else TRAFFIC_PER_ALGORITHMIC_BYTE.get(kind) if u64_rows else None)
     roofline = {
@@ -421,8 +420,10 @@ def run_ours(args):
             "exact_weights": bool(d["exact_weights"]),
             "key_bits": d["key_bits"],
             "merge": {1: "hash", 2: "partition"}.get(d["merge"], d["merge"]),
-            "rows": "column-grouped" if grouped else "partitioned",
-            "cuda_graph": not args.no_graph and not grouped,
+            "rows": " + ".join(f for f, bit in (("single", pkg.ROWS_SINGLE), ("chain", pkg.ROWS_CHAIN),
+                                                ("column-grouped", pkg.ROWS_GROUPED), ("one CTA", pkg.ROWS_ONE_CTA),
+                                                ("graph replay", pkg.ROWS_REPLAY)) if d["row_forms"] & bit),
+            "cuda_graph": d["row_forms"] == pkg.ROWS_REPLAY,
             "tuning": tuning,
             "tuning_cache": tuning_note,
         },

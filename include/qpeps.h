@@ -65,6 +65,7 @@ typedef struct qpeps_layer {
  * (src/lib.rs:403-415) plus device-side facts. */
 typedef struct qpeps_result {
   uint32_t n;
+  uint32_t row_forms; /* the forms the device rows ran in: QPEPS_ROWS_* bits (a former padding word) */
   qpeps_u128 count;
   double elapsed_s;
   uint64_t peak_states;
@@ -101,6 +102,13 @@ typedef struct qpeps_result {
   uint32_t residue_primes[4];
   uint64_t count_residues[4];
 } qpeps_result;
+
+/* Forms of device rows (and of sites): what ran, whatever the times say. */
+#define QPEPS_ROWS_SINGLE 1  /* one at a time, sized by the host */
+#define QPEPS_ROWS_CHAIN 2   /* queued together, sized on the device */
+#define QPEPS_ROWS_GROUPED 4 /* a whole device batch of column-grouped rows */
+#define QPEPS_ROWS_ONE_CTA 8 /* a whole board in one CTA */
+#define QPEPS_ROWS_REPLAY 16 /* replay of a captured graph (alone) */
 
 #define QPEPS_GRAIN_ROW 0  /* compiled row operator, one fused step per row */
 #define QPEPS_GRAIN_SITE 1 /* explicit C, one plain launch per site */

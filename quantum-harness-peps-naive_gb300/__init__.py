@@ -47,6 +47,11 @@ SCATTER_CLASS = 3
 SCATTER_DIRECT = 4
 MERGEK_SCAN = 0
 MERGEK_CLAIM = 1
+ROWS_SINGLE = 1
+ROWS_CHAIN = 2
+ROWS_GROUPED = 4
+ROWS_ONE_CTA = 8
+ROWS_REPLAY = 16
 
 
 class U128(ctypes.Structure):
@@ -76,6 +81,7 @@ class Layer(ctypes.Structure):
 class Result(ctypes.Structure):
     _fields_ = [
         ("n", ctypes.c_uint32),
+        ("row_forms", ctypes.c_uint32),
         ("count", U128),
         ("elapsed_s", ctypes.c_double),
         ("peak_states", ctypes.c_uint64),
@@ -387,6 +393,7 @@ def _result_from(res: Result, layers: Sequence[Layer] | None) -> ContractionResu
                 )
             )
     device = {
+        "row_forms": res.row_forms,
         "residues": res.residues,
         "key_bits": res.key_bits,
         "slice_depth": res.slice_depth,

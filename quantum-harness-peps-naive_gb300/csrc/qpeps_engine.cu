@@ -464,6 +464,7 @@ struct RunStats {
   u64 merge_launches = 0, merge_bytes = 0;
   u64 final_res[kMaxResidues] = {0, 0, 0, 0};
   unsigned batches = 0;
+  uint32_t forms = 0;  // QPEPS_ROWS_* of the rows that ran
 };
 
 struct Plan {
@@ -896,6 +897,7 @@ static StepStatus merge_step(Ctx& ctx, const Plan& p, DevFrontier& f, bool site,
     rs.scatter_ms += ms_a;
     rs.merge_ms += ms_b;
     rs.merge_launches += 1;
+    rs.forms |= QPEPS_ROWS_SINGLE;
     rs.merge_bytes += (n_in + so.out) * eb;
     rs.entries_in += n_in;
     rs.entries_out += so.out;
@@ -1259,6 +1261,7 @@ static bool run_resident(Ctx& ctx, const Plan& p, const HostChunk& hc, std::vect
   ctx.h2d_bytes += sizeof a;
   ctx.d2h_bytes += count * sizeof(StepScalars);
   rs.batches += 1;
+  rs.forms |= QPEPS_ROWS_ONE_CTA;
   const double ms = h[count].t_merge > h[1].t_scatter ? (double)(h[count].t_merge - h[1].t_scatter) * 1e-6 : 0.0;
   rs.device_ms += ms;
   rs.merge_ms += ms;
@@ -1418,6 +1421,7 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
     }
   }
   if (done) {
+    rs.forms |= QPEPS_ROWS_CHAIN;
     const bool ended = row + done == p.n;
     f.count = ended ? 0 : h[done].out_count;
     known_terms = h[done].next_terms;
@@ -1532,6 +1536,7 @@ static u64 run_queued_sites_plain(Ctx& ctx, const Plan& p, DevFrontier& f, unsig
       rs.peak_states = std::max<u64>(rs.peak_states, r.out_count);
     }
   }
+  if (done) rs.forms |= QPEPS_ROWS_CHAIN;
   if (done) f.count = row + done / p.n == p.n ? 0 : h[done].out_count;
   return done;
 }
@@ -1843,6 +1848,7 @@ static bool run_chunk_grouped(Ctx& ctx, const Plan& p, const HostChunk& hc, std:
   ctx.h2d_bytes += h2d;
   const size_t eb = entry_bytes(p);
   rs.batches += 1;
+  rs.forms |= QPEPS_ROWS_GROUPED;
   rs.launches += launches;
   rs.device_ms += ms;
   rs.peak_states = std::max<u64>(rs.peak_states, hc.count);
@@ -2980,6 +2986,7 @@ static bool graph_replay(Ctx& ctx, unsigned n, const qpeps_options& o, const uin
     out.rs.merge_ms += b;
   }
   out.rs.launches = g->launches;
+  out.rs.forms = QPEPS_ROWS_REPLAY;
   out.elapsed = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   return true;
 }
@@ -3130,6 +3137,7 @@ static void fill_result(const Ctx& ctx, const Contraction& c, unsigned n, qpeps_
                         uint32_t cap) {
   std::memset(r, 0, sizeof *r);
   r->n = n;
+  r->row_forms = c.rs.forms;
   r->count = to_abi(c.count);
   r->elapsed_s = c.elapsed;
   r->peak_states = c.peak_states;

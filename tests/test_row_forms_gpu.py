@@ -1,0 +1,47 @@
+"""Which form the rows of a call ran in, as the result reports it."""
+from __future__ import annotations
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def fresh(qp):
+    c = qp.Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("n,opts,forms", [
+    (1, {}, ""), (4, {}, "CHAIN"), (8, {"merge": 1}, "SINGLE"), (9, {"granularity": 1}, "CHAIN"),
+    (14, {}, "CHAIN"), (14, {"symmetry": 0}, "GROUPED"), (14, {"granularity": 1}, "CHAIN SINGLE"),
+    (15, {}, "GROUPED"), (15, {"key_bits": 128}, "CHAIN"), (16, {"use_graph": 1}, "CHAIN SINGLE"),
+])
+def test_boards(fresh, qp, n, opts, forms):
+    r = fresh.contract_rows(n, **opts)
+    assert r.count == qp.known_count(n)
+    assert r.device["row_forms"] == sum(getattr(qp, f"ROWS_{f}") for f in forms.split())
+
+
+@pytest.mark.parametrize("n,prefix,forms", [
+    (14, [10, 6, 3, 0], "ONE_CTA"), (16, [4, 9, 5, 13, 15], "CHAIN"), (16, [7], "GROUPED"), (8, [0, 1], ""),
+])
+def test_partly_placed_boards(fresh, qp, n, prefix, forms):
+    assert fresh.count_with_stats(n, prefix)[1].device["row_forms"] == sum(
+        getattr(qp, f"ROWS_{f}") for f in forms.split())
+
+
+def test_a_replay_is_reported(fresh, qp):
+    seen = [fresh.contract_rows(11, use_graph=1).device["row_forms"] for _ in range(3)]
+    assert seen == [qp.ROWS_CHAIN, qp.ROWS_REPLAY, qp.ROWS_REPLAY]
+
+
+# A prefix whose boundary passes its estimate: a row of the chain does not fit,
+# and another chain goes on from its input (two kernels more than the rows take).
+def test_an_ended_chain_goes_on(fresh, qp):
+    prefix = [8, 2]
+    count, r = fresh.count_with_stats(17, prefix)
+    assert count == fresh.count(17, prefix, merge=qp.MERGE_HASH)
+    assert r.device["row_forms"] == qp.ROWS_CHAIN
+    assert r.device["gpu_launches"] > 1 + 2 * (17 - len(prefix))
