@@ -24,8 +24,9 @@ e2e    : the same entries / wall time of the C-ABI call (host seeding,
          host->device upload of the seed boundary, all row steps, device->host
          read-back of every row's metrics and of the count residues).
 roofline: the merge step (scatter + merge kernels, or plan + pull kernels of
-         column-grouped rows), algorithmic bytes E*(S_in+S_out), E = 16, summed
-         over the row steps of one contraction over those kernels' time. `traffic` is DRAM bytes per step
+         column-grouped rows), algorithmic bytes E*(S_in+S_out) summed
+         over the row steps of one contraction over those kernels' time; an entry
+         is E = 16 bytes, 8 in column-grouped rows. `traffic` is DRAM bytes per step
          scaled from a small ncu capture of peak-row launches (see
          TRAFFIC_PER_ALGORITHMIC_BYTE); null where none applies.
 cpu_baseline: the CPU oracle (threaded restatement of the reference's
@@ -70,7 +71,7 @@ PACKAGE = "quantum-harness-peps-naive_gb300"
 TRAFFIC_PER_ALGORITHMIC_BYTE: dict = {1: 171.290302464 / 56.96632816}
 # Column-grouped rows hold an entry in 8 bytes: the pulls of Q(16) rows 10-12
 # moved 5.474 GB for (51.4 + 87.8 + 87.8 + 105.5 + 105.5 + 79.5) M entries.
-GROUPED_TRAFFIC_PER_ALGORITHMIC_BYTE = 5.474 / (16 * 0.5176)
+GROUPED_TRAFFIC_PER_ALGORITHMIC_BYTE = 5.474 / (8 * 0.5176)
 METRIC = "Q(N) wall time & boundary entries/s at N=18 (bit-exact)"
 UNIT = "boundary entries/s"
 
@@ -377,7 +378,7 @@ def run_ours(args):
         "unit": "GB/s",
         "frac": achieved / peak,
         "traffic": (tpb * d["merge_kernel_bytes"]) if tpb else None,
-        "traffic_scope": ("DRAM bytes per step: the step's algorithmic bytes x 0.661, the DRAM bytes per algorithmic "
+        "traffic_scope": ("DRAM bytes per step: the step's algorithmic bytes x 1.322, the DRAM bytes per algorithmic "
                           "byte that ncu measured on the pull launches of Q(16) rows 10-12 (8-byte entries)" if grouped
                           else "DRAM bytes per step: the step's algorithmic bytes x 3.007, the DRAM bytes per algorithmic "
                           "byte that ncu measured on the scatter and merge launches of Q(17) rows 11-13 (an upper "

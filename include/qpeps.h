@@ -90,7 +90,8 @@ typedef struct qpeps_result {
   double merge_kernel_ms;     /* device time of the merge kernel (table compact or partition merge) */
   double scatter_kernel_ms;   /* device time of the expand kernel (table insert or partition scatter) */
   uint64_t merge_kernel_launches;
-  uint64_t merge_kernel_bytes; /* algorithmic bytes of the dominant kernel */
+  uint64_t merge_kernel_bytes; /* algorithmic bytes of the dominant kernel: entries read and written, in
+                                  the form's own entry size (8 bytes in column-grouped rows) */
   uint32_t tail_row;          /* first row contracted by the slice-tail kernel (N = none) */
   uint32_t exact_weights;     /* 1: the boundary's two u32 planes held each entry's exact 64-bit weight
                                  (low and high words) and the host derived the residues; 0: residue planes */

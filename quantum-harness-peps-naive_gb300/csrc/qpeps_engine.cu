@@ -1846,7 +1846,6 @@ static bool run_chunk_grouped(Ctx& ctx, const Plan& p, const HostChunk& hc, std:
   }
   if (ctx.rec) ctx.rec->ok = false;
   ctx.h2d_bytes += h2d;
-  const size_t eb = entry_bytes(p);
   rs.batches += 1;
   rs.forms |= QPEPS_ROWS_GROUPED;
   rs.launches += launches;
@@ -1875,7 +1874,7 @@ static bool run_chunk_grouped(Ctx& ctx, const Plan& p, const HostChunk& hc, std:
       rs.scatter_ms += r.t_pull > r.t_plan ? (double)(r.t_pull - r.t_plan) * 1e-6 : 0.0;
       rs.merge_ms += r.t_end > r.t_pull ? (double)(r.t_end - r.t_pull) * 1e-6 : 0.0;
       rs.merge_launches += 1;
-      rs.merge_bytes += (in + r.out_count) * eb;
+      rs.merge_bytes += (in + r.out_count) * kGroupEntryBytes;
       rs.entries_in += in;
       rs.entries_out += r.out_count;
       rs.candidates += terms;

@@ -45,3 +45,12 @@ def test_an_ended_chain_goes_on(fresh, qp):
     assert count == fresh.count(17, prefix, merge=qp.MERGE_HASH)
     assert r.device["row_forms"] == qp.ROWS_CHAIN
     assert r.device["gpu_launches"] > 1 + 2 * (17 - len(prefix))
+
+
+# Bytes are counted in the form's own entry size: key and weight in 32 bits
+# each, or a 64-bit key and a weight's two words.
+@pytest.mark.parametrize("kind,entry", [("WINDOW", 8), ("DIRECT", 16)])
+def test_bytes_are_the_entries_read_and_written(fresh, qp, kind, entry):
+    fresh.set_tuning(scatter_kind=getattr(qp, f"SCATTER_{kind}"))
+    d = fresh.contract_rows(15).device
+    assert d["merge_kernel_bytes"] == entry * (d["entries_in"] + d["entries_out"])
