@@ -1237,7 +1237,6 @@ static bool run_resident(Ctx& ctx, const Plan& p, const HostChunk& hc, std::vect
       p.merge != QPEPS_MERGE_PARTITION || p.key_bits != 64 || p.free_rows > 20 || ctx.tune.merge_kind != 1 ||
       ctx.tune.scatter_kind != 1 || ctx.tune.fold_weights != 2 || !(p.w64 || p.R == 1))
     return false;
-  const auto t0 = std::chrono::steady_clock::now();
   const unsigned count = p.n - hc.row;
   StepScalars* h = pinned_scalars(ctx, count);
   ResidentArgs a{};
@@ -1266,11 +1265,8 @@ static bool run_resident(Ctx& ctx, const Plan& p, const HostChunk& hc, std::vect
   rs.device_ms += ms;
   rs.merge_ms += ms;
   rs.peak_states = std::max<u64>(rs.peak_states, hc.count);
-  const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-  for (unsigned i = 0; i < count; ++i) {
-    rows[hc.row + i].elapsed += wall / count;
-    add_row(p, hc.row + i, h[i].out_count, h[i].next_terms, h[i + 1], true, rows, rs);
-  }
+  // (No row times: partly placed boards report none.)
+  for (unsigned i = 0; i < count; ++i) add_row(p, hc.row + i, h[i].out_count, h[i].next_terms, h[i + 1], true, rows, rs);
   return true;
 }
 
