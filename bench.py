@@ -364,7 +364,7 @@ def run_ours(args):
     # The capture behind the factor is of the u64 row path's scatter and merge.
     u64_rows = d["merge"] == 2 and args.grain == "row" and d["key_bits"] == 64
     # (A batch handed back to the partitioned rows would leave both forms' bits.)
-    grouped = d["row_forms"] == pkg.ROWS_GROUPED
+    grouped = d["row_forms"] & ~pkg.ROWS_CHECKED == pkg.ROWS_GROUPED
     tpb = (GROUPED_TRAFFIC_PER_ALGORITHMIC_BYTE if grouped
            else TRAFFIC_PER_ALGORITHMIC_BYTE.get(kind) if u64_rows else None)
     roofline = {

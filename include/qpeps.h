@@ -110,6 +110,7 @@ typedef struct qpeps_result {
 #define QPEPS_ROWS_GROUPED 4 /* a whole device batch of column-grouped rows */
 #define QPEPS_ROWS_ONE_CTA 8 /* a whole board in one CTA */
 #define QPEPS_ROWS_REPLAY 16 /* replay of a captured graph (alone) */
+#define QPEPS_ROWS_CHECKED 32 /* use_graph, not captured: every row compared with the recorded run's */
 
 #define QPEPS_GRAIN_ROW 0  /* compiled row operator, one fused step per row */
 #define QPEPS_GRAIN_SITE 1 /* explicit C, one plain launch per site */
@@ -134,7 +135,10 @@ typedef struct qpeps_options {
                                     graph; later identical contractions replay it (one launch, one
                                     synchronisation) and check every row against the recorded run.
                                     Device batches of over 200 M entries (N = 17, 18) run
-                                    column-grouped rows instead, queued at once and not captured */
+                                    column-grouped rows, and partly placed boards of up to about
+                                    2000 entries run in one CTA: both are queued at once and not
+                                    captured; later identical contractions run again and check every
+                                    row against the recorded run in the same way */
   uint64_t device_budget_bytes;  /* 0 = auto (a fraction of free device memory) */
   uint32_t tail_row;             /* rows >= tail_row run in the slice-tail kernel (a CTA contracts
                                     batches of boundary entries in shared memory); 0 = auto (never),

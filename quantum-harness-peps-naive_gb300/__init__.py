@@ -52,6 +52,7 @@ ROWS_CHAIN = 2
 ROWS_GROUPED = 4
 ROWS_ONE_CTA = 8
 ROWS_REPLAY = 16
+ROWS_CHECKED = 32
 
 
 class U128(ctypes.Structure):

@@ -566,7 +566,8 @@ struct GraphChunkRec {
 };
 
 struct GraphRecorder {
-  bool ok = true;  // false once anything outside the capturable form ran
+  bool ok = true;         // false once anything outside the capturable form ran
+  bool compared = false;  // column-grouped or one-CTA rows ran: compared with the next run instead
   std::vector<GraphChunkRec> chunks;
 };
 
@@ -1256,7 +1257,7 @@ static bool run_resident(Ctx& ctx, const Plan& p, const HostChunk& hc, std::vect
   cuda_check(cudaStreamSynchronize(ctx.stream), "resident rows");
   rs.launches += 1;
   if (h[1].error) return false;
-  if (ctx.rec) ctx.rec->ok = false;
+  if (ctx.rec) ctx.rec->ok = false, ctx.rec->compared = true;
   ctx.h2d_bytes += sizeof a;
   ctx.d2h_bytes += count * sizeof(StepScalars);
   rs.batches += 1;
@@ -1840,7 +1841,7 @@ static bool run_chunk_grouped(Ctx& ctx, const Plan& p, const HostChunk& hc, std:
       fail(QPEPS_ERR_OVERFLOW, row_msg("exact 64-bit weights are not certified at row", m));
     total = h_rows[m].weight_sum;
   }
-  if (ctx.rec) ctx.rec->ok = false;
+  if (ctx.rec) ctx.rec->ok = false, ctx.rec->compared = true;
   ctx.h2d_bytes += h2d;
   rs.batches += 1;
   rs.forms |= QPEPS_ROWS_GROUPED;
@@ -2609,7 +2610,9 @@ static void explicit_frontier(Ctx& ctx, unsigned n, unsigned order, u64 support_
 // synchronisation instead of three launches and two synchronisations per row.
 // The replay checks every row's output count, weight sums and final sums
 // against the recorded run before it answers; on any difference it drops the
-// graph and contracts eagerly.
+// graph and contracts eagerly. Column-grouped and one-CTA rows are queued
+// without the host already and are not captured: each run is compared with the
+// recorded one in the same figures.
 
 // Device batches are independent sub-contractions (their results add), so
 // the graph runs them on `batch_lanes` streams at once: each lane has its own
@@ -2678,14 +2681,43 @@ static qpeps_options graph_key_options(const qpeps_options& o) {
   return k;
 }
 
-static bool graph_matches(const Ctx& ctx, unsigned n, const qpeps_options& o, const uint32_t* prefix, unsigned k) {
+// Whether the context's record is of this call.
+static bool same_call(const Ctx& ctx, unsigned n, const qpeps_options& o, const uint32_t* prefix, unsigned k) {
   const GraphPlan* g = ctx.graph;
-  if (!g || g->n != n || g->prefix.size() != k || g->pool_gen != ctx.pool_gen) return false;
+  if (!g || g->n != n || g->prefix.size() != k) return false;
   for (unsigned i = 0; i < k; ++i)
     if (g->prefix[i] != prefix[i]) return false;
   const qpeps_options a = graph_key_options(o), b = graph_key_options(g->opt);
   if (std::memcmp(&a, &b, sizeof a) != 0) return false;
   return std::memcmp(&g->tune, &ctx.tune, sizeof g->tune) == 0;
+}
+
+// Whether a captured graph of this call can replay in the buffers as they stand.
+static bool graph_matches(const Ctx& ctx, unsigned n, const qpeps_options& o, const uint32_t* prefix, unsigned k) {
+  return same_call(ctx, n, o, prefix, k) && ctx.graph->exec && ctx.graph->pool_gen == ctx.pool_gen;
+}
+
+// A run that is not captured, as the record that the next one is compared with.
+static void record_rows(Ctx& ctx, unsigned n, const qpeps_options& o, const uint32_t* prefix, unsigned k,
+                        const Contraction& done) {
+  graph_free(ctx);
+  GraphPlan* g = ctx.graph = new GraphPlan();
+  g->n = n;
+  g->prefix.assign(prefix, prefix + k);
+  g->opt = o;
+  g->tune = ctx.tune;
+  g->base = done;
+}
+
+// The figures that a replay checks, of two whole runs.
+static bool same_rows(const Contraction& a, const Contraction& b) {
+  bool same = a.count == b.count && a.rows.size() == b.rows.size();
+  for (size_t i = 0; same && i < a.rows.size(); ++i) {
+    const RowAcc &x = a.rows[i], &y = b.rows[i];
+    same = x.input_states == y.input_states && x.output_states == y.output_states && x.matched == y.matched;
+    for (int r = 0; r < kMaxResidues; ++r) same = same && x.weight_res[r] == y.weight_res[r];
+  }
+  return same;
 }
 
 // Capture the recorded steps. Best effort: any failure leaves no graph.
@@ -3000,7 +3032,23 @@ static void contract(Ctx& ctx, unsigned n, const qpeps_options& o, const uint32_
       throw;
     }
     ctx.rec = nullptr;
-    if (o.use_graph) graph_build(ctx, n, o, prefix, k, out, rec);
+    if (rec.compared && same_call(ctx, n, o, prefix, k) && !ctx.graph->exec) {
+      if (!same_rows(ctx.graph->base, out)) {
+        // As after a replay that differs: the record goes, and a run of its own
+        // answers.
+        graph_free(ctx);
+        Contraction again;
+        contract_impl(ctx, n, o, prefix, k, again);
+        out = std::move(again);
+        record_rows(ctx, n, o, prefix, k, out);
+      } else {
+        out.rs.forms |= QPEPS_ROWS_CHECKED;
+      }
+    } else if (rec.compared) {
+      record_rows(ctx, n, o, prefix, k, out);
+    } else if (o.use_graph) {
+      graph_build(ctx, n, o, prefix, k, out, rec);
+    }
   }
   out.h2d_bytes = ctx.h2d_bytes - h0;
   out.d2h_bytes = ctx.d2h_bytes - d0;

@@ -54,3 +54,17 @@ def test_bytes_are_the_entries_read_and_written(fresh, qp, kind, entry):
     fresh.set_tuning(scatter_kind=getattr(qp, f"SCATTER_{kind}"))
     d = fresh.contract_rows(15).device
     assert d["merge_kernel_bytes"] == entry * (d["entries_in"] + d["entries_out"])
+
+
+# What use_graph does not capture (column-grouped and one-CTA rows) is compared
+# row by row with the recorded run; another call's record is not taken for it.
+def test_uncaptured_runs_are_compared(fresh, qp):
+    one, other = [10, 6, 3, 0], [10, 6, 3, 1]
+    boards = [(17, None), (14, one), (14, other)]
+    for n, prefix in boards:
+        form = qp.ROWS_ONE_CTA if prefix else qp.ROWS_GROUPED
+        runs = [fresh.count_with_stats(n, prefix, use_graph=1)[1] if prefix else fresh.contract_rows(n, use_graph=1)
+                for _ in range(3)]
+        assert [r.device["row_forms"] for r in runs] == [form] + 2 * [form | qp.ROWS_CHECKED]
+        assert runs[0].count == runs[1].count == runs[2].count
+    assert fresh.contract_rows(17).device["row_forms"] == qp.ROWS_GROUPED
