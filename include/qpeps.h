@@ -225,7 +225,15 @@ int qpeps_explicit_frontier(void* ctx, uint32_t n, uint32_t order, uint64_t supp
 /* ---- Tuning ---------------------------------------------------------------
  * No reference counterpart (the reference has one CPU code path): the knobs of
  * the partitioned merge, held per context. Every setting gives the same
- * counts and metrics; only the speed changes. */
+ * counts and metrics; only the speed changes.
+ *
+ * Settings also choose among the forms of rows (QPEPS_ROWS_*). Chains need
+ * merge_kind 1, scatter_kind 0, 1 or 4 and wide_merge 0 or 2 (64-bit keys);
+ * one-CTA boards merge_kind 1, scatter_kind 1 and fold_weights 2;
+ * column-grouped rows that and merge_compact 0. What a form does not use it
+ * ignores: parents_per_lane and scatter_block are for boundaries of over 2048
+ * entries an SM (smaller ones run one parent a lane in CTAs of 128 threads with
+ * scatter_kind 1); a server's shared batch always runs the default kinds. */
 #define QPEPS_SCATTER_SEARCH 0 /* shuffle search for each successor's parent */
 #define QPEPS_SCATTER_WINDOW 1 /* per-warp shared-memory candidate window (default) */
 #define QPEPS_SCATTER_TWO_LEVEL 2 /* coarse buckets, then partitions, each written as runs ordered in
@@ -286,7 +294,8 @@ int qpeps_ctx_set_tuning(void* ctx, const qpeps_tuning* t, char* err, size_t err
  * margin, host rows); each candidate times
  * contract_rows(n) (8 <= n <= 19) with CUDA-graph replay (device time, best
  * of `repeats` after a warm-up run; every count checked against known_count).
- * Keeps the fastest in the context and returns it. */
+ * Keeps the fastest in the context and returns it. A value that makes the
+ * same call without use_graph slower is not taken. */
 int qpeps_autotune(void* ctx, uint32_t n, uint32_t repeats, qpeps_tuning* best, double* best_device_ms, char* err,
                    size_t err_len);
 /* Name of the context's CUDA device (for keying tuning caches). */

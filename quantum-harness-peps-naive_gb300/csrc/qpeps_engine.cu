@@ -3873,10 +3873,15 @@ static void apply_tune(Ctx& c, const Ctx::Tune& t) {
 // Autotuner: coordinate descent over the knobs of a contraction, starting
 // from the context's tuning. Each pass tries, one dimension at a time, every
 // value of that dimension with the others at their best so far and keeps the
-// fastest (device time, best of `repeats` after one untimed warm-up run;
-// every count is checked against known_count); passes repeat until one
+// fastest (device time of a replay, best of `repeats` after one untimed warm-up
+// run; every count is checked against known_count); passes repeat until one
 // changes nothing (at most three). A candidate whose warm-up run takes more
-// than three times the best so far is not timed further.
+// than three times the best so far is not timed further. A value is kept only
+// if it gains half a percent and 5 us (at N = 17, where most knobs reach nothing
+// that runs, the best of two runs differs by 0.2 %, at N = 11 by 3 us) and calls without use_graph do
+// not get 2 % slower by it: some values turn chains, column-grouped rows or
+// one-CTA boards off (N = 11, replays 0.200 -> 0.188 ms by the global table, but
+// other calls 0.102 -> 0.192).
 //   scatter kind (not the class-grouped one, which is not graph-captured),
 //   parents per lane, scatter block size, merge kind, merge CTA
 //   shape (wide), partition fill, weight accumulator (fold), merge strategy
@@ -3890,12 +3895,12 @@ static double autotune(Ctx& c, unsigned n, unsigned repeats, Ctx::Tune* best) {
   qpeps_options o;
   qpeps_options_default(&o);
   o.collect_layers = 0;
-  o.use_graph = 1;  // the timed runs replay the captured contraction, as bench and serving runs do
   const Ctx::Tune saved = c.tune;
   Ctx::Tune cur = saved;
-  double best_ms = 1e300;
-  auto measure = [&](const Ctx::Tune& t, double cap_ms) {
+  double best_ms = 1e300, best_eager = 1e300;
+  auto measure = [&](const Ctx::Tune& t, double cap_ms, uint32_t use_graph) {
     apply_tune(c, t);
+    o.use_graph = use_graph;
     double ms = 1e300;
     for (unsigned r = 0; r <= repeats; ++r) {
       Contraction con;
@@ -3927,7 +3932,8 @@ static double autotune(Ctx& c, unsigned n, unsigned repeats, Ctx::Tune* best) {
       {{1, 2}, [](Ctx::Tune& t, double v) { t.batch_lanes = (uint32_t)v; }},
   };
   try {
-    best_ms = measure(cur, 1e300);
+    best_ms = measure(cur, 1e300, 1);
+    best_eager = measure(cur, 1e300, 0);
     for (int pass = 0; pass < 3; ++pass) {
       bool changed = false;
       for (const Dim& d : dims)
@@ -3935,9 +3941,12 @@ static double autotune(Ctx& c, unsigned n, unsigned repeats, Ctx::Tune* best) {
           Ctx::Tune t = cur;
           d.set(t, v);
           if (std::memcmp(&t, &cur, sizeof t) == 0) continue;
-          const double ms = measure(t, 3.0 * best_ms);
-          if (ms < best_ms) {
+          const double ms = measure(t, 3.0 * best_ms, 1);
+          if (ms >= std::min(0.995 * best_ms, best_ms - 0.005)) continue;
+          const double eager = measure(t, 3.0 * best_eager, 0);
+          if (eager <= 1.02 * best_eager) {
             best_ms = ms;
+            best_eager = std::min(best_eager, eager);
             cur = t;
             changed = true;
           }

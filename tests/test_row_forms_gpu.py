@@ -68,3 +68,14 @@ def test_uncaptured_runs_are_compared(fresh, qp):
         assert [r.device["row_forms"] for r in runs] == [form] + 2 * [form | qp.ROWS_CHECKED]
         assert runs[0].count == runs[1].count == runs[2].count
     assert fresh.contract_rows(17).device["row_forms"] == qp.ROWS_GROUPED
+
+
+# The autotuner's picks leave the forms that other calls run in: none of those
+# that it may turn off is slower than what replaces it at these sizes.
+@pytest.mark.parametrize("n", [11, 11, 11, 13, 14, 15])
+def test_autotuned_calls_keep_their_form(fresh, qp, n):
+    form = fresh.contract_rows(n).device["row_forms"]
+    fresh.autotune(n, repeats=2)
+    r = fresh.contract_rows(n)
+    assert r.count == qp.known_count(n)
+    assert r.device["row_forms"] == form
