@@ -166,7 +166,17 @@ __global__ void __launch_bounds__(BLOCK) group_plan_kernel(GroupStepArgs a) {
 
 // ---- pull: one unit per CTA at a time ---------------------------------------
 
-constexpr int kMaxSeg = 128;
+// (Both limits can be set lower when this file is compiled: no board of up to 18
+// columns passes them, and what happens beyond them has to be run somewhere.)
+#ifndef QPEPS_GROUP_MAX_SEG
+#define QPEPS_GROUP_MAX_SEG 128
+#endif
+#ifndef QPEPS_GROUP_WEIGHT_BITS
+#define QPEPS_GROUP_WEIGHT_BITS 32
+#endif
+constexpr int kMaxSeg = QPEPS_GROUP_MAX_SEG;
+constexpr int kWeightBits = QPEPS_GROUP_WEIGHT_BITS;
+static_assert(kMaxSeg <= 128 && kWeightBits <= 32, "a run's segment takes 8 bits, a weight one word");
 constexpr int kRuns = 144;  // runs of a unit besides one per segment
 constexpr u32 kBatch = 128; // matches a warp inserts at a time
 
@@ -362,10 +372,10 @@ __global__ void __launch_bounds__((W + P) * 32, CTAS) group_pull_kernel(GroupSte
   if (__syncthreads_or(*reinterpret_cast<volatile const u32*>(&row->error) != 0u)) return;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const unsigned n = a.n, m = a.m, rm = a.rm;
-  // Sums must stay within 32 bits: an output key has at most four parents a
+  // Sums must stay within a word: an output key has at most four parents a
   // column (the diagonal bits that leave the board). (The rows of 17 and 18
   // columns do.)
-  if (prev->weight_max * (4ull * m) >> 32) {
+  if (prev->weight_max * (4ull * m) >> kWeightBits) {
     if (blockIdx.x == 0 && tid == 0) atomicOr(&row->error, kErrNeedWide);
     return;
   }
