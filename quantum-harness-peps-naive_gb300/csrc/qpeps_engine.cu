@@ -1133,22 +1133,21 @@ static StepScalars* queue_scalars(Ctx& ctx, size_t steps) {
   return static_cast<StepScalars*>(ctx.queue.ptr);
 }
 
-// Device times of a finished chain's kernels from their start stamps; `total`
-// (ms, CUDA events) bounds the last one.
+// Device times of a finished chain's kernels from their stamps (the host's
+// time between two launches is in neither: a kernel's first launch in a process
+// takes 10 ms and more).
 struct QueueTimes {
   std::vector<double> scatter, merge;  // ms per step
-};
-static QueueTimes queue_times(const StepScalars* h, size_t steps, double total) {
-  QueueTimes t;
   double sum = 0;
+};
+static QueueTimes queue_times(const StepScalars* h, size_t steps) {
+  QueueTimes t;
   for (size_t i = 1; i <= steps; ++i) {
     const StepScalars& a = h[i];
-    const bool more = i < steps && h[i + 1].t_scatter > a.t_merge;
     t.scatter.push_back(a.t_merge > a.t_scatter ? (double)(a.t_merge - a.t_scatter) * 1e-6 : 0.0);
-    t.merge.push_back(more ? (double)(h[i + 1].t_scatter - a.t_merge) * 1e-6 : 0.0);
-    sum += t.scatter.back() + t.merge.back();
+    t.merge.push_back(a.t_end > a.t_merge ? (double)(a.t_end - a.t_merge) * 1e-6 : 0.0);
+    t.sum += t.scatter.back() + t.merge.back();
   }
-  if (steps) t.merge.back() += std::max(0.0, total - sum);
   return t;
 }
 
@@ -1373,7 +1372,7 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   if (done < count) chain_ended(ctx, h[done + 1], mean, pcap);
   if (done < count && (h[done + 1].error & kErrBounds))
     fail(QPEPS_ERR_CUDA, row_msg("a kernel's bounds check failed (access skipped) at row", row + done + 1));
-  const QueueTimes times = queue_times(h, done, ms);
+  const QueueTimes times = queue_times(h, done);
   const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   for (unsigned i = 0; i < done; ++i) {
     const StepScalars& r = h[i + 1];
@@ -1385,7 +1384,7 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
       if (bound >> 63) fail(QPEPS_ERR_OVERFLOW, row_msg("exact 64-bit weights are not certified at row", row + i + 1));
       f.weight_bound = r.weight_sum[0];
     }
-    rows[row + i].elapsed += ms > 0 ? wall * (times.scatter[i] + times.merge[i]) / ms : 0.0;
+    rows[row + i].elapsed += times.sum > 0 ? wall * (times.scatter[i] + times.merge[i]) / times.sum : 0.0;
     if (tm) {
       rs.scatter_ms += times.scatter[i];
       rs.merge_ms += times.merge[i];
@@ -1495,7 +1494,7 @@ static u64 run_queued_sites_plain(Ctx& ctx, const Plan& p, DevFrontier& f, unsig
   while (done < sites && !h[done + 1].error) ++done;
   if (done < sites && (h[done + 1].error & kErrProbeLimit))
     fail(QPEPS_ERR_CAPACITY, row_msg("hash probe bound exceeded at row", row + (unsigned)(done / p.n) + 1));
-  const QueueTimes times = queue_times(h, done, ms);
+  const QueueTimes times = queue_times(h, done);
   const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   if (ctx.rec) ctx.rec->ok = false;
   for (size_t i = 0; i < done; ++i) {
@@ -1520,7 +1519,7 @@ static u64 run_queued_sites_plain(Ctx& ctx, const Plan& p, DevFrontier& f, unsig
       rs.entries_in += in;
       rs.entries_out += r.out_count;
     }
-    acc.elapsed += ms > 0 ? wall * (times.scatter[i] + times.merge[i]) / ms : 0.0;
+    acc.elapsed += times.sum > 0 ? wall * (times.scatter[i] + times.merge[i]) / times.sum : 0.0;
     // (The first site's terms are a bound; what it merged is exact.)
     rs.candidates += i ? r.terms : r.out_count;
     if (site + 1 == p.n) {

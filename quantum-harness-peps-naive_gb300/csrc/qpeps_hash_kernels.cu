@@ -471,6 +471,7 @@ __global__ void __launch_bounds__(BLOCK) compact_kernel(Slot<K, R>* __restrict__
       if (sums[R + r]) atomicAdd(&sc->final_sum[r], sums[R + r]);
     }
     if (sums[2 * R]) atomicAdd(&sc->final_states, sums[2 * R]);
+    if constexpr (QUEUED) atomicMax(&sc->t_end, global_ns());
     if (sums[2 * R + 1]) atomicAdd(&sc->next_terms, sums[2 * R + 1]);
     if (sums[2 * R + 2]) atomicAdd(&sc->row_terms, sums[2 * R + 2]);
     if (sums[2 * R + 3]) atomicAdd(&sc->sitewise_examined, sums[2 * R + 3]);

@@ -39,7 +39,8 @@ struct StepScalars {
                                          // row kernel matches over the input (sitewise_entries())
   unsigned long long plan_units;         // class-grouped partitions: units of the step's plan (graph replay)
   unsigned long long next_terms;         // successor terms of the written boundary at the next row
-  unsigned long long t_scatter, t_merge; // queued steps: start of each kernel (global timer, ns)
+  unsigned long long t_scatter, t_merge, t_end; // queued steps: start of each kernel, end of the second
+                                                // (global timer, ns)
   unsigned long long row_terms;          // queued site steps that end a row: successor terms of its boundary
 };
 

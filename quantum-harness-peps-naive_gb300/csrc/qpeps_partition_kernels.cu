@@ -1026,6 +1026,7 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
       if (sums[SP + r]) atomicAdd(&sc->final_sum[r], sums[SP + r]);
     }
     if (sums[2 * SP]) atomicAdd(&sc->final_states, sums[2 * SP]);
+    if (q.prev) atomicMax(&sc->t_end, global_ns());
     if constexpr (kCountNext) {
       if (write_out && count_next) {
         if (sums[2 * SP + 1]) atomicAdd(&sc->next_terms, sums[2 * SP + 1]);

@@ -463,6 +463,7 @@ __global__ void __launch_bounds__(BLOCK, 2) wide_merge_kernel(const WCand<R>* __
       if (sums[R + r]) atomicAdd(&sc->final_sum[r], sums[R + r]);
     }
     if (sums[2 * R]) atomicAdd(&sc->final_states, sums[2 * R]);
+    if (q.prev) atomicMax(&sc->t_end, global_ns());
     if (count_next) {
       if (sums[2 * R + 1]) atomicAdd(&sc->next_terms, sums[2 * R + 1]);
       if (blockIdx.x == 0) sc->next_terms_ok = 1u;
