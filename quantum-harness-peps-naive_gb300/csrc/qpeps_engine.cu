@@ -1134,18 +1134,20 @@ static StepScalars* queue_scalars(Ctx& ctx, size_t steps) {
 }
 
 // Device times of a finished chain's kernels from their stamps (the host's
-// time between two launches is in neither: a kernel's first launch in a process
-// takes 10 ms and more).
+// time before the first launch is in neither: a kernel's first launch in a
+// process takes 10 ms and more). A site step's compaction stamps its end in the
+// last step only (242 stamps of N = 11 took 2 % of its time).
 struct QueueTimes {
   std::vector<double> scatter, merge;  // ms per step
   double sum = 0;
 };
-static QueueTimes queue_times(const StepScalars* h, size_t steps) {
+static QueueTimes queue_times(const StepScalars* h, size_t steps, size_t queued) {
   QueueTimes t;
   for (size_t i = 1; i <= steps; ++i) {
     const StepScalars& a = h[i];
     t.scatter.push_back(a.t_merge > a.t_scatter ? (double)(a.t_merge - a.t_scatter) * 1e-6 : 0.0);
-    t.merge.push_back(a.t_end > a.t_merge ? (double)(a.t_end - a.t_merge) * 1e-6 : 0.0);
+    const u64 end = a.t_end ? a.t_end : i < queued ? h[i + 1].t_scatter : 0;
+    t.merge.push_back(end > a.t_merge ? (double)(end - a.t_merge) * 1e-6 : 0.0);
     t.sum += t.scatter.back() + t.merge.back();
   }
   return t;
@@ -1372,7 +1374,7 @@ static unsigned run_queued_rows(Ctx& ctx, const Plan& p, DevFrontier& f, unsigne
   if (done < count) chain_ended(ctx, h[done + 1], mean, pcap);
   if (done < count && (h[done + 1].error & kErrBounds))
     fail(QPEPS_ERR_CUDA, row_msg("a kernel's bounds check failed (access skipped) at row", row + done + 1));
-  const QueueTimes times = queue_times(h, done);
+  const QueueTimes times = queue_times(h, done, count);
   const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   for (unsigned i = 0; i < done; ++i) {
     const StepScalars& r = h[i + 1];
@@ -1471,6 +1473,7 @@ static u64 run_queued_sites_plain(Ctx& ctx, const Plan& p, DevFrontier& f, unsig
     const unsigned r = row + (unsigned)(i / p.n), site = (unsigned)(i % p.n);
     const u64 fits = std::min<u64>(most, 2 * entries);
     source.prev = d + i;
+    source.last = i + 1 == sites;
     const bool last = r + 1 == p.n && site + 1 == p.n;
     cuda_check(launch_site_expand_insert(cfg, view, entries, p.n, site, ctx.table.ptr, source.slots(fits), d + i + 1,
                                          ctx.stream, source),
@@ -1494,7 +1497,7 @@ static u64 run_queued_sites_plain(Ctx& ctx, const Plan& p, DevFrontier& f, unsig
   while (done < sites && !h[done + 1].error) ++done;
   if (done < sites && (h[done + 1].error & kErrProbeLimit))
     fail(QPEPS_ERR_CAPACITY, row_msg("hash probe bound exceeded at row", row + (unsigned)(done / p.n) + 1));
-  const QueueTimes times = queue_times(h, done);
+  const QueueTimes times = queue_times(h, done, sites);
   const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   if (ctx.rec) ctx.rec->ok = false;
   for (size_t i = 0; i < done; ++i) {

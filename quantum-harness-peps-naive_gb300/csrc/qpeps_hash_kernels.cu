@@ -105,7 +105,10 @@ __device__ __forceinline__ bool table_sizes(const TableSource& q, StepScalars* s
   const u64 terms = q.prev->next_terms, entries = q.prev->out_count;
   const u64 want = q.slots(terms);
   if (error || want > q.slots_cap || terms > cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->error, (u32)(error ? kErrSkipped : kErrCapacity));
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      atomicOr(&sc->error, (u32)(error ? kErrSkipped : kErrCapacity));
+      if (!sc->t_scatter) sc->t_scatter = global_ns();  // the end of the step before
+    }
     return false;
   }
   n_in = terms ? entries : 0;
@@ -471,7 +474,8 @@ __global__ void __launch_bounds__(BLOCK) compact_kernel(Slot<K, R>* __restrict__
       if (sums[R + r]) atomicAdd(&sc->final_sum[r], sums[R + r]);
     }
     if (sums[2 * R]) atomicAdd(&sc->final_states, sums[2 * R]);
-    if constexpr (QUEUED) atomicMax(&sc->t_end, global_ns());
+    if constexpr (QUEUED)
+      if (q.last) atomicMax(&sc->t_end, global_ns());
     if (sums[2 * R + 1]) atomicAdd(&sc->next_terms, sums[2 * R + 1]);
     if (sums[2 * R + 2]) atomicAdd(&sc->row_terms, sums[2 * R + 2]);
     if (sums[2 * R + 3]) atomicAdd(&sc->sitewise_examined, sums[2 * R + 3]);

@@ -40,7 +40,7 @@ struct StepScalars {
   unsigned long long plan_units;         // class-grouped partitions: units of the step's plan (graph replay)
   unsigned long long next_terms;         // successor terms of the written boundary at the next row
   unsigned long long t_scatter, t_merge, t_end; // queued steps: start of each kernel, end of the second
-                                                // (global timer, ns)
+                                                // (global timer, ns; 0: the next step's start)
   unsigned long long row_terms;          // queued site steps that end a row: successor terms of its boundary
 };
 
@@ -89,6 +89,7 @@ inline cudaError_t launch_overlapped(void (*kernel)(Params...), unsigned grid, u
 struct TableSource {
   const StepScalars* prev = nullptr;  // nullptr: the host passes the sizes
   uint64_t slots_cap = 0;             // slots the table holds (a power of two)
+  bool last = false;                  // the chain's last step: its compaction stamps its end
 
   // A small step's time is its longest probe sequence, a trip to L2 each: at
   // loads up to 1/2, 30 K terms took 18 us, at up to 1/8 7 us. Larger steps
