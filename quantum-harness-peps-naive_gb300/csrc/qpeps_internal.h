@@ -372,7 +372,9 @@ cudaError_t launch_group_seed(const GroupSeedUnit* list, uint32_t count, const G
 // Serving (slotted keys, exact 64-bit weights in two planes): scatter and merge
 // of a boundary shared by requests of different board sizes. slot_mask[s] is
 // the board mask of the request in slot s; finished boards are summed into
-// slot_final[s * 4] and leave the boundary.
+// slot_final[s * 4] and leave the boundary. One pair of kernels: the window
+// scatter and the exact claim-list merge in its small shape; of `pc` only the
+// partitions, their cursors' stride and the queued sizes count.
 cudaError_t launch_serve_scatter(const PartitionCfg& pc, const FrontierView& in, uint64_t n_in,
                                  const uint64_t* slot_mask, void* regions, uint32_t* cursors, StepScalars* sc,
                                  cudaStream_t stream);

@@ -540,11 +540,8 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_kernel(const Cand<R>* _
   unsigned long long* s_acc = reinterpret_cast<unsigned long long*>(smem_raw + sizeof(u64) * H);  // [R][H]
   __shared__ u32 s_cnt[PER * WARPS];
   __shared__ unsigned long long s_base;
-  // Serving: finished boards are summed per request slot here, then flushed.
-  __shared__ unsigned long long s_slot_fin[Layout::kSlotted ? kServeMaxSlots * R : 1];
+  static_assert(!Layout::kSlotted, "the shared batch of a server merges by claim list");
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if constexpr (Layout::kSlotted)
-    for (int i = threadIdx.x; i < (int)kServeMaxSlots * R; i += BLOCK) s_slot_fin[i] = 0ull;
   // A partition overflowed in the scatter: write nothing, so the boundary
   // buffer (read by the scatter, written here in place) stays intact for the
   // host's retry with smaller partitions.
@@ -612,21 +609,7 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_kernel(const Cand<R>* _
     u32 flags = 0;
 #pragma unroll
     for (int it = 0; it < PER; ++it) {
-      bool occ = s_key[it * BLOCK + threadIdx.x] != kEmpty;
-      if constexpr (Layout::kSlotted) {
-        // A finished board leaves the boundary: sum it into its slot.
-        const u64 key = s_key[it * BLOCK + threadIdx.x];
-        if (occ && (key & L.mask_of(key)) == L.mask_of(key)) {
-          const int slot = it * BLOCK + threadIdx.x;
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            atomicAdd(&s_slot_fin[L.slot(key) * R + r], (unsigned long long)reduce_sum(s_acc[r * H + slot], r));
-            s_acc[r * H + slot] = 0ull;
-          }
-          s_key[slot] = kEmpty;
-          occ = false;
-        }
-      }
+      const bool occ = s_key[it * BLOCK + threadIdx.x] != kEmpty;
       flags |= (u32)occ << it;
       const u32 b = __ballot_sync(kFullMask, occ);
       if (lane == 0) s_cnt[it * WARPS + wid] = __popc(b);
@@ -665,8 +648,7 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_kernel(const Cand<R>* _
         const bool wr = write_out && idx < out_stride;
         bad |= write_out && !wr;
         if (wr) keys_out[idx] = key;
-        if constexpr (!Layout::kSlotted)
-          if (count_next) nterms += next_terms_of(L, key);
+        if (count_next) nterms += next_terms_of(L, key);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const u32 v = reduce_sum(s_acc[r * H + slot], r);
@@ -691,17 +673,10 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_kernel(const Cand<R>* _
   }
   const unsigned long long t = pblock_sum<BLOCK>(fstates);
   if (threadIdx.x == 0 && t) atomicAdd(&sc->final_states, t);
-  if constexpr (!Layout::kSlotted) {
-    if (write_out && count_next) {
-      const unsigned long long nt = pblock_sum<BLOCK>(nterms);
-      if (threadIdx.x == 0 && nt) atomicAdd(&sc->next_terms, nt);
-      if (blockIdx.x == 0 && threadIdx.x == 0) sc->next_terms_ok = 1u;
-    }
-  }
-  if constexpr (Layout::kSlotted) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < (int)kServeMaxSlots * R; i += BLOCK)
-      if (s_slot_fin[i]) atomicAdd(&L.slot_final[(i / R) * 4 + (i % R)], s_slot_fin[i]);
+  if (write_out && count_next) {
+    const unsigned long long nt = pblock_sum<BLOCK>(nterms);
+    if (threadIdx.x == 0 && nt) atomicAdd(&sc->next_terms, nt);
+    if (blockIdx.x == 0 && threadIdx.x == 0) sc->next_terms_ok = 1u;
   }
 }
 
@@ -760,7 +735,7 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
   static_assert(CAP % BLOCK == 0, "shape");
   constexpr bool kFold = kAcc != 0;  // one 64-bit accumulator plane
   static_assert(!kFold || R == 2, "the one-plane accumulators hold a residue pair or a weight's two words");
-  static_assert(!kRegs || !Layout::kSlotted, "register compaction is for the fixed layout");
+  static_assert(!Layout::kSlotted || (kAcc == 2 && !kRegs), "the slotted layout carries exact weights in a slot list");
   constexpr int AP = kFold ? 1 : R;  // accumulator planes
   extern __shared__ __align__(16) unsigned char smem_raw[];
   u64* s_key = reinterpret_cast<u64*>(smem_raw);
@@ -768,11 +743,10 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
   u32* s_list = reinterpret_cast<u32*>(smem_raw + sizeof(u64) * H * (1 + AP));                   // [CAP]
   __shared__ u32 s_nused, s_n;
   __shared__ unsigned long long s_base;
-  constexpr int SF = kAcc == 2 ? 1 : R;  // sums of a finished board: the exact weight, or its residues
-  __shared__ unsigned long long s_slot_fin[Layout::kSlotted ? kServeMaxSlots * SF : 1];
+  __shared__ unsigned long long s_slot_fin[Layout::kSlotted ? kServeMaxSlots : 1];
   const int lane = threadIdx.x & 31;
   if constexpr (Layout::kSlotted)
-    for (int i = threadIdx.x; i < (int)kServeMaxSlots * SF; i += BLOCK) s_slot_fin[i] = 0ull;
+    for (int i = threadIdx.x; i < (int)kServeMaxSlots; i += BLOCK) s_slot_fin[i] = 0ull;
   next_kernel_may_start();
   for (int i = threadIdx.x; i < H; i += BLOCK) s_key[i] = kEmpty;
   if (threadIdx.x == 0) s_nused = 0;
@@ -841,23 +815,12 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
           const u32 of = __shfl_sync(kFullMask, mine, leader);
           const bool in = finished && mine == of && ((left >> lane) & 1u);
           left &= ~__ballot_sync(kFullMask, in);
+          unsigned long long v = in ? one_plane<2>(buf[l].res[0], buf[l].res[1]) : 0ull;
 #pragma unroll
-          for (int r = 0; r < SF; ++r) {
-            unsigned long long v = !in ? 0ull
-                                   : kAcc == 2 ? one_plane<2>(buf[l].res[0], buf[l].res[R > 1 ? 1 : 0])
-                                               : (unsigned long long)buf[l].res[r];
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFullMask, v, d);
-            if (lane == leader) atomicAdd(&s_slot_fin[of * SF + r], v);
-          }
+          for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFullMask, v, d);
+          if (lane == leader) atomicAdd(&s_slot_fin[of], v);
         }
-        if ((left >> lane) & 1u) {
-#pragma unroll
-          for (int r = 0; r < SF; ++r)
-            atomicAdd(&s_slot_fin[mine * SF + r],
-                      kAcc == 2 ? one_plane<2>(buf[l].res[0], buf[l].res[R > 1 ? 1 : 0])
-                                : (unsigned long long)buf[l].res[r]);
-        }
+        if ((left >> lane) & 1u) atomicAdd(&s_slot_fin[mine], one_plane<2>(buf[l].res[0], buf[l].res[1]));
       }
       if (i < bcnt) {
         const Cand<R>& c = buf[l];
@@ -1036,8 +999,8 @@ __global__ void __launch_bounds__(BLOCK) partition_merge_list_kernel(const Cand<
   }
   if constexpr (Layout::kSlotted) {
     __syncthreads();
-    for (int i = threadIdx.x; i < (int)kServeMaxSlots * SF; i += BLOCK)
-      if (s_slot_fin[i]) atomicAdd(&L.slot_final[(i / SF) * 4 + (i % SF)], s_slot_fin[i]);
+    for (int i = threadIdx.x; i < (int)kServeMaxSlots; i += BLOCK)
+      if (s_slot_fin[i]) atomicAdd(&L.slot_final[i * 4], s_slot_fin[i]);
   }
 }
 
@@ -1402,26 +1365,37 @@ constexpr size_t merge_smem() {
   return (size_t)H * (8 + 8 * R);
 }
 
+template <int PPL, int BLOCK>
+unsigned scatter_grid(const PartitionCfg& pc, u64 n_in) {
+  const u64 want = (n_in + BLOCK * PPL - 1) / (BLOCK * PPL);
+  const u64 capb = (u64)pc.sms * 8 * 256 / BLOCK;  // the same resident threads per SM for every block size
+  return (unsigned)std::max<u64>(1, std::min(want, capb));
+}
+
+template <int R, int PPL, int BLOCK, typename Layout>
+cudaError_t window_scatter(const PartitionCfg& pc, const FrontierView& in, u64 n_in, Layout L, void* regions,
+                           u32* cursors, StepScalars* sc, cudaStream_t stream) {
+  return launch_overlapped(partition_scatter_list_kernel<R, BLOCK, PPL, Layout>, scatter_grid<PPL, BLOCK>(pc, n_in),
+                           BLOCK, 0, stream, pc.queued.prev != nullptr, reinterpret_cast<const u64*>(in.keys), in.res,
+                           in.cap, n_in, L, reinterpret_cast<Cand<R>*>(regions), cursors,
+                           pc.cursor_stride ? pc.cursor_stride : 1, pc.parts, pc.cap, sc, pc.queued);
+}
+
+// A boundary that leaves the chip short of warps at four parents a lane (fewer
+// than about 8 blocks an SM) takes one a lane in small blocks.
+bool few_parents(const PartitionCfg& pc, u64 n_in) { return n_in <= (u64)pc.sms * 2048; }
+
 template <int R, int PPL, int BLOCK, typename Layout>
 cudaError_t scatter_shape(const PartitionCfg& pc, const FrontierView& in, u64 n_in, Layout L, void* regions,
                           u32* cursors, StepScalars* sc, cudaStream_t stream) {
-  u64 want = (n_in + BLOCK * PPL - 1) / (BLOCK * PPL);
-  const u64 capb = (u64)pc.sms * 8 * 256 / BLOCK;  // the same resident threads per SM for every block size
-  const unsigned grid = (unsigned)std::max<u64>(1, std::min(want, capb));
-  const u32 cstride = pc.cursor_stride ? pc.cursor_stride : 1;
-  if (pc.scatter_kind == 4) {
-    partition_scatter_direct_kernel<R, BLOCK, PPL, Layout><<<grid, BLOCK, 0, stream>>>(
-        reinterpret_cast<const u64*>(in.keys), in.res, in.cap, n_in, L, reinterpret_cast<Cand<R>*>(regions), cursors,
-        cstride, pc.parts, pc.cap, sc, pc.queued);
-    return cudaGetLastError();
-  }
-  if (pc.scatter_kind != 0)  // 2 without a two-level plan, or 3 where it does not apply: the window scatter
-    return launch_overlapped(partition_scatter_list_kernel<R, BLOCK, PPL, Layout>, grid, BLOCK, 0, stream,
-                             pc.queued.prev != nullptr, reinterpret_cast<const u64*>(in.keys), in.res, in.cap, n_in, L,
-                             reinterpret_cast<Cand<R>*>(regions), cursors, cstride, pc.parts, pc.cap, sc, pc.queued);
-  partition_scatter_kernel<R, BLOCK, PPL, Layout><<<grid, BLOCK, 0, stream>>>(
+  // (2 without a two-level plan, or 3 where it does not apply: the window scatter.)
+  if (pc.scatter_kind != 0 && pc.scatter_kind != 4)
+    return window_scatter<R, PPL, BLOCK, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
+  auto kern = pc.scatter_kind == 4 ? partition_scatter_direct_kernel<R, BLOCK, PPL, Layout>
+                                   : partition_scatter_kernel<R, BLOCK, PPL, Layout>;
+  kern<<<scatter_grid<PPL, BLOCK>(pc, n_in), BLOCK, 0, stream>>>(
       reinterpret_cast<const u64*>(in.keys), in.res, in.cap, n_in, L, reinterpret_cast<Cand<R>*>(regions), cursors,
-      cstride, pc.parts, pc.cap, sc, pc.queued);
+      pc.cursor_stride ? pc.cursor_stride : 1, pc.parts, pc.cap, sc, pc.queued);
   return cudaGetLastError();
 }
 
@@ -1440,10 +1414,8 @@ cudaError_t scatter_ppl(const PartitionCfg& pc, const FrontierView& in, u64 n_in
 template <int R, typename Layout>
 cudaError_t scatter_impl(const PartitionCfg& pc, const FrontierView& in, u64 n_in, Layout L, void* regions,
                          u32* cursors, StepScalars* sc, cudaStream_t stream) {
-  // A boundary that leaves the chip short of warps at four parents a lane
-  // (fewer than about 8 blocks an SM) takes one a lane in small blocks.
-  if (pc.scatter_kind == 1 && n_in <= (u64)pc.sms * 2048)
-    return scatter_shape<R, 1, 128, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
+  if (pc.scatter_kind == 1 && few_parents(pc, n_in))
+    return window_scatter<R, 1, 128, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
   if (pc.parents_per_lane == 4) return scatter_ppl<R, 4, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
   return scatter_ppl<R, 2, Layout>(pc, in, n_in, L, regions, cursors, sc, stream);
 }
@@ -1455,15 +1427,12 @@ cudaError_t merge_shape(const PartitionCfg& pc, int blocks_per_sm, const void* r
   const bool fold = R == 2 && pc.merge_kind == 1 && pc.fold;
   const bool exact = fold && pc.fold == 2;
   if (pc.fold == 2 && !exact) return cudaErrorInvalidValue;  // exact words need the claim-list merge
-  constexpr bool kRegsOk = !Layout::kSlotted;
-  const bool regs = kRegsOk && pc.merge_regs;
-  auto kern = fold ? (exact ? (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout,
-                                                                  R == 2 ? 2 : 0, kRegsOk>
-                                    : partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout,
-                                                                  R == 2 ? 2 : 0>)
-                            : (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, R == 2 ? 1 : 0, kRegsOk>
+  const bool regs = pc.merge_regs;
+  auto kern = fold ? (exact ? (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, R == 2 ? 2 : 0, true>
+                                    : partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, R == 2 ? 2 : 0>)
+                            : (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, R == 2 ? 1 : 0, true>
                                     : partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, R == 2 ? 1 : 0>))
-                   : (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, 0, kRegsOk>
+                   : (regs ? partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout, 0, true>
                            : partition_merge_list_kernel<R, BLOCK, H, H / 2, Layout>);
   auto scan_kern = partition_merge_kernel<R, BLOCK, H, H / 2, Layout>;
   const bool scan = pc.merge_kind != 1;
@@ -1510,15 +1479,24 @@ cudaError_t launch_serve_scatter(const PartitionCfg& pc, const FrontierView& in,
                                  const uint64_t* slot_mask, void* regions, uint32_t* cursors, StepScalars* sc,
                                  cudaStream_t stream) {
   if (n_in == 0) return cudaSuccess;
-  if (pc.residues != 2) return cudaErrorInvalidValue;
-  return scatter_impl<2>(pc, in, n_in, SlotLayout{slot_mask, nullptr}, regions, cursors, sc, stream);
+  const SlotLayout L{slot_mask, nullptr};
+  if (few_parents(pc, n_in)) return window_scatter<2, 1, 128>(pc, in, n_in, L, regions, cursors, sc, stream);
+  return window_scatter<2, 4, kScatterBlock>(pc, in, n_in, L, regions, cursors, sc, stream);
 }
 
 cudaError_t launch_serve_merge(const PartitionCfg& pc, const void* regions, const uint32_t* cursors,
                                const FrontierView& out, const uint64_t* slot_mask, unsigned long long* slot_final,
                                StepScalars* sc, cudaStream_t stream) {
-  if (pc.residues != 2) return cudaErrorInvalidValue;
-  return merge_impl<2>(pc, regions, cursors, out, SlotLayout{slot_mask, slot_final}, true, sc, stream);
+  if (pc.cap != (u32)(kSmallH / 2)) return cudaErrorInvalidValue;
+  auto kern = partition_merge_list_kernel<2, kSmallBlock, kSmallH, kSmallH / 2, SlotLayout, 2>;
+  const size_t smem = merge_smem<1, kSmallH>() + (size_t)(kSmallH / 2) * 4;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const unsigned grid = (unsigned)std::max<u64>(1, std::min<u64>(pc.parts, (u64)pc.sms * 4));
+  return launch_overlapped(kern, grid, kSmallBlock, smem, stream, pc.queued.prev != nullptr,
+                           reinterpret_cast<const Cand<2>*>(regions), cursors, pc.cursor_stride ? pc.cursor_stride : 1,
+                           pc.parts, reinterpret_cast<u64*>(out.keys), out.res, out.cap,
+                           SlotLayout{slot_mask, slot_final}, 3, sc, pc.queued);
 }
 uint32_t partition_capacity(uint32_t wide) { return wide == 2 ? kSmallH / 2 : wide ? kWideH / 2 : kMergeH / 2; }
 bool wide_merge_supported(int residues) { return residues >= 1 && residues <= 2; }
