@@ -87,14 +87,15 @@ typedef struct qpeps_result {
   uint64_t gpu_launches;      /* kernels launched by this call */
   uint64_t peak_device_bytes; /* high-water mark of the context's device pool */
   double device_ms;           /* device time of all row steps (CUDA events) */
-  double merge_kernel_ms;     /* device time of the merge kernel (table compact or partition merge) */
-  double scatter_kernel_ms;   /* device time of the expand kernel (table insert or partition scatter) */
+  double merge_kernel_ms;     /* device time of the merge kernel (table compact, partition merge or pull) */
+  double scatter_kernel_ms;   /* device time of the expand kernel (table insert, partition scatter or plan) */
   uint64_t merge_kernel_launches;
   uint64_t merge_kernel_bytes; /* algorithmic bytes of the dominant kernel: entries read and written, in
                                   the form's own entry size (8 bytes in column-grouped rows) */
   uint32_t tail_row;          /* first row contracted by the slice-tail kernel (N = none) */
   uint32_t exact_weights;     /* 1: the boundary's two u32 planes held each entry's exact 64-bit weight
-                                 (low and high words) and the host derived the residues; 0: residue planes */
+                                 (low and high words; in column-grouped rows one u32, certified row by
+                                 row) and the host derived the residues; 0: residue planes */
   uint64_t tail_items;        /* boundary entries handed to the slice-tail kernel */
   uint64_t tail_overflow;     /* of those, entries redone by the row engine */
   double tail_kernel_ms;      /* device time of the slice-tail kernel */
