@@ -940,13 +940,19 @@ static void split_to_host(Ctx& ctx, const Plan& p, DevFrontier& f, unsigned row,
 
 constexpr size_t kSeedStage = 64 << 10;
 
+// Pooled buffers are dead between chunks; those of earlier calls go where they
+// exceed this call's budget.
+static void trim_pool(Ctx& ctx, const Plan& p) {
+  if (!p.budget.known()) return;
+  if (ctx.pool_bytes > p.budget) group_release(ctx);
+  if (ctx.pool_bytes > p.budget) buf_release(ctx, ctx.table);
+  if (ctx.front[0].bytes > p.budget) buf_release(ctx, ctx.front[0]);
+}
+
 static void upload_chunk(Ctx& ctx, const Plan& p, const HostChunk& hc, DevFrontier& f) {
-  // Pooled buffers are dead between chunks; drop them only if they exceed
-  // this call's budget or cannot hold the chunk.
   f.count = 0;
-  const bool bounded = p.budget.known();
-  if (bounded && ctx.pool_bytes > p.budget) buf_release(ctx, ctx.table);
-  if (f.cap < hc.count || (bounded && ctx.front[0].bytes > p.budget)) {
+  trim_pool(ctx, p);
+  if (!ctx.front[0].ptr || f.cap < hc.count) {
     buf_release(ctx, ctx.front[0]);
     f.cap = 0;
   }
@@ -1230,9 +1236,9 @@ static void add_row(const Plan& p, unsigned row, u64 in, u64 terms, const StepSc
 
 // A partly placed board whose boundary is expected to fit one CTA's shared
 // memory, from its host entries to the last row in one launch that writes its
-// scalars to pinned memory. (Whole boards run row by row: they report each
-// row's time.) False, with nothing added, where it does not apply or the
-// boundary outgrew it.
+// scalars to pinned memory. (Whole boards report each row's time and run as
+// chains.) False, with nothing added, where it does not apply or the boundary
+// outgrew it.
 static bool run_resident(Ctx& ctx, const Plan& p, const HostChunk& hc, std::vector<RowAcc>& rows, RunStats& rs) {
   if (!p.prefix || hc.count == 0 || hc.count > kResidentSeeds || hc.no_tail || hc.row >= p.n || p.tail_row < p.n ||
       p.batch_states <= 0 || p.batch_states > 0.5 * resident_capacity() || p.grain != QPEPS_GRAIN_ROW ||
@@ -1258,6 +1264,7 @@ static bool run_resident(Ctx& ctx, const Plan& p, const HostChunk& hc, std::vect
   cuda_check(cudaStreamSynchronize(ctx.stream), "resident rows");
   rs.launches += 1;
   if (h[1].error) return false;
+  trim_pool(ctx, p);
   if (ctx.rec) ctx.rec->ok = false, ctx.rec->compared = true;
   ctx.h2d_bytes += sizeof a;
   ctx.d2h_bytes += count * sizeof(StepScalars);

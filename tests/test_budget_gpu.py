@@ -66,3 +66,22 @@ def test_chain_scalars_fit_a_tight_budget(fresh, qp, n, budget, opts):
     g = fresh.contract_rows(n, device_budget_bytes=budget, **opts)
     assert g.count == qp.known_count(n)
     assert _held(g) <= budget
+
+
+# What earlier calls left goes where it exceeds the budget, also before a call
+# that needs no device memory of its own (a board in one CTA). Freed memory is
+# seen by the device: 11 GB of column-grouped rows.
+@pytest.mark.parametrize("call", [
+    lambda c, b: c.count(14, [10, 6, 3, 0], device_budget_bytes=b),
+    lambda c, b: c.contract_rows(8, device_budget_bytes=b),
+    lambda c, b: (c.contract_rows(8), c.contract_rows(8, device_budget_bytes=b)),
+    lambda c, b: c.contract_rows(8, granularity=1, device_budget_bytes=b),
+])
+def test_kept_buffers_beyond_the_budget_go(fresh, qp, call):
+    torch = pytest.importorskip("torch")
+    before = torch.cuda.mem_get_info()[0]
+    fresh.contract_rows(17)
+    kept = before - torch.cuda.mem_get_info()[0]
+    call(fresh, 64 << 20)
+    assert kept > 8 << 30
+    assert before - torch.cuda.mem_get_info()[0] < 1 << 30
