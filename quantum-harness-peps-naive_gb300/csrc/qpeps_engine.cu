@@ -388,6 +388,38 @@ static void buf_reserve(Ctx& ctx, DevBuf& b, size_t bytes, const Budget& budget,
   ++ctx.pool_gen;
 }
 
+// buf_reserve's answer instead of its exception.
+static bool try_reserve(Ctx& ctx, DevBuf& b, size_t bytes, const Budget& budget, const char* what) {
+  try {
+    buf_reserve(ctx, b, bytes, budget, what);
+    return true;
+  } catch (const Failure& e) {
+    if (e.code != QPEPS_ERR_CAPACITY) throw;
+    return false;
+  }
+}
+
+// The scalars of queued steps. No captured graph holds their buffer (a replay has
+// scalars of its own), so neither its growth nor its release ends one.
+static bool queue_reserve(Ctx& ctx, size_t bytes, const Budget& budget) {
+  const uint64_t gen = ctx.pool_gen;
+  const bool ok = try_reserve(ctx, ctx.queue, bytes, budget, "queued step scalars");
+  ctx.pool_gen = gen;
+  return ok;
+}
+
+// What a row or site that runs by itself does not use: the buffers of other
+// forms, of the slice tail and of the explicit-C frontier's steps (`plan` is
+// also the class-grouped partitions' scratch).
+static void idle_release(Ctx& ctx, bool plan) {
+  group_release(ctx);
+  const uint64_t gen = ctx.pool_gen;
+  buf_release(ctx, ctx.queue);
+  ctx.pool_gen = gen;
+  buf_release(ctx, ctx.tail);
+  if (plan) buf_release(ctx, ctx.plan);
+}
+
 static void graph_free(Ctx& ctx);
 
 static void ctx_free(Ctx* ctx) {
@@ -779,12 +811,16 @@ static StepStatus merge_step(Ctx& ctx, const Plan& p, DevFrontier& f, bool site,
       table_bytes = slots * slot_bytes(p.key_bits, p.R);
     }
     const u64 need_cap = final_step ? n_in : std::max<u64>(n_in, so.terms);
-    if (f.cap > need_cap && f.cap * eb + table_bytes > p.budget && need_cap * eb * 5 / 4 + table_bytes <= p.budget &&
-        f.count <= need_cap) {
+    // The pool's other buffers count: where they are in the way, those that this
+    // step does not use go.
+    const auto others = [&] { return ctx.pool_bytes - ctx.front[0].bytes - ctx.table.bytes; };
+    const auto fits = [&](u64 cap) { return cap * eb + table_bytes + others() <= p.budget; };
+    if (!fits(std::max<u64>(f.cap, need_cap))) idle_release(ctx, !unit);
+    if (f.cap > need_cap && !fits(f.cap) && fits(need_cap * 5 / 4) && f.count <= need_cap) {
       buf_release(ctx, ctx.table);
       shrink_front(ctx, p, f, need_cap);
     }
-    if (std::max<u64>(f.cap, need_cap) * eb + table_bytes > p.budget) {
+    if (!fits(std::max<u64>(f.cap, need_cap))) {
       if (n_in <= 1) fail(QPEPS_ERR_CAPACITY, row_msg("device budget exceeded at row", row + 1));
       return StepStatus::NeedSplit;
     }
@@ -797,7 +833,13 @@ static StepStatus merge_step(Ctx& ctx, const Plan& p, DevFrontier& f, bool site,
       }
     }
     if (ctx.pool_bytes - ctx.table.bytes + table_bytes > p.budget) buf_release(ctx, ctx.table);
-    buf_reserve(ctx, ctx.table, table_bytes, p.budget, partition ? "partition regions" : "hash table");
+    // (A boundary that grew beyond its need, for rows to come, gives way.)
+    const char* what = partition ? "partition regions" : "hash table";
+    if (!try_reserve(ctx, ctx.table, table_bytes, p.budget, what) &&
+        !(f.cap > need_cap && shrink_front(ctx, p, f, need_cap) && try_reserve(ctx, ctx.table, table_bytes, p.budget, what))) {
+      if (n_in <= 1) fail(QPEPS_ERR_CAPACITY, row_msg("device budget exceeded at row", row + 1));
+      return StepStatus::NeedSplit;
+    }
 
     LaunchCfg cfg{p.key_bits, p.R, p.threads, ctx.sms};
     FrontierView view = view_of(p, ctx.front[0], f.cap);
@@ -1159,17 +1201,6 @@ static QueueTimes queue_times(const StepScalars* h, size_t steps, size_t queued)
   return t;
 }
 
-// buf_reserve's answer instead of its exception.
-static bool try_reserve(Ctx& ctx, DevBuf& b, size_t bytes, const Budget& budget, const char* what) {
-  try {
-    buf_reserve(ctx, b, bytes, budget, what);
-    return true;
-  } catch (const Failure& e) {
-    if (e.code != QPEPS_ERR_CAPACITY) throw;
-    return false;
-  }
-}
-
 // Room for a chain of `steps` steps: their scalars, a boundary of `most`
 // entries and `table_bytes` of scratch, or false. Buffers that stand are not
 // asked about again.
@@ -1180,12 +1211,8 @@ static bool chain_buffers(Ctx& ctx, const Plan& p, DevFrontier& f, u64 most, siz
   if (!p.budget.holds(std::max<u64>(f.cap, most) * entry_bytes(p) + table_bytes + scalar_bytes)) return false;
   if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
   // The scalars come before the table, which takes what is left of the budget
-  // up to a quarter more than it needs. No captured graph holds their buffer (a
-  // replay has scalars of its own), so its growth does not end one.
-  const uint64_t gen = ctx.pool_gen;
-  const bool scalars = try_reserve(ctx, ctx.queue, scalar_bytes, p.budget, "queued step scalars");
-  ctx.pool_gen = gen;
-  if (!scalars) return false;
+  // up to a quarter more than it needs.
+  if (!queue_reserve(ctx, scalar_bytes, p.budget)) return false;
   // (A large chain's boundary is sized for its largest row.)
   if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes, most <= kQueueTerms)) return false;
   return p.budget.holds(ctx.pool_bytes - ctx.table.bytes + table_bytes) &&

@@ -85,3 +85,25 @@ def test_kept_buffers_beyond_the_budget_go(fresh, qp, call):
     call(fresh, 64 << 20)
     assert kept > 8 << 30
     assert before - torch.cuda.mem_get_info()[0] < 1 << 30
+
+
+# What a context keeps of other calls (chain scalars, site steps, the slice
+# tail's lists) takes nothing from a tight budget: calls that fit a fresh
+# context fit after any of them.
+@pytest.mark.parametrize("prep", [
+    lambda c: c.contract_rows(12), lambda c: c.contract_rows(9, granularity=1), lambda c: c.explicit_frontier(10, 1),
+    lambda c: c.contract_rows(12, tail_row=9), lambda c: c.contract_rows(15),
+], ids=["chain", "sites", "explicit", "tail", "grouped"])
+@pytest.mark.parametrize("n,opts,budgets", [
+    (11, {"granularity": 1, "symmetry": 0}, range(409600, 1740800, 56789)), (10, {"granularity": 1}, range(204800, 921600, 40961)),
+    (12, {}, range(307200, 2560000, 98765)), (11, {"merge": 1}, range(307200, 2560000, 98765)),
+    (11, {"key_bits": 128}, range(307200, 2560000, 98765)),
+])
+def test_kept_buffers_take_nothing_from_a_budget(qp, prep, n, opts, budgets):
+    for budget in budgets:
+        c = qp.Context(0)
+        try:
+            prep(c)
+            assert c.contract_rows(n, device_budget_bytes=budget, **opts).count == qp.known_count(n)
+        finally:
+            c.close()
