@@ -1202,21 +1202,33 @@ static QueueTimes queue_times(const StepScalars* h, size_t steps, size_t queued)
 }
 
 // Room for a chain of `steps` steps: their scalars, a boundary of `most`
-// entries and `table_bytes` of scratch, or false. Buffers that stand are not
-// asked about again.
+// entries and `table_bytes` of scratch, or false with the boundary and the
+// scratch as they were (the rows that run instead use them; a scratch freed
+// here and reserved there again, row by row, doubled the time of N = 16 in 280
+// batches). Buffers that stand are not asked about again.
 static bool chain_buffers(Ctx& ctx, const Plan& p, DevFrontier& f, u64 most, size_t table_bytes, size_t steps,
                           const char* what) {
-  const size_t scalar_bytes = (steps + 1) * sizeof(StepScalars);
+  const size_t scalar_bytes = (steps + 1) * sizeof(StepScalars), eb = entry_bytes(p);
   if (!p.budget.known() && f.cap >= most && ctx.table.bytes >= table_bytes && ctx.queue.bytes >= scalar_bytes) return true;
-  if (!p.budget.holds(std::max<u64>(f.cap, most) * entry_bytes(p) + table_bytes + scalar_bytes)) return false;
-  if (ctx.table.bytes < table_bytes) buf_release(ctx, ctx.table);
+  const auto others = [&] {
+    return ctx.pool_bytes - ctx.front[0].bytes - ctx.table.bytes - ctx.queue.bytes + std::max(ctx.queue.bytes, scalar_bytes);
+  };
+  const size_t table = std::max(table_bytes, ctx.table.bytes);
+  const size_t grown = f.cap < most ? most * eb : 0;  // a new boundary, beside the old one while that is copied
+  const auto fits = [&](size_t boundary, size_t scratch) { return p.budget.holds(others() + boundary + scratch); };
+  const auto room = [&] {
+    return fits(std::max(ctx.front[0].bytes, grown), table_bytes) &&
+           (!grown || fits(ctx.front[0].bytes + grown, ctx.table.bytes < table_bytes ? 0 : ctx.table.bytes));
+  };
+  if (!room() && !(group_release(ctx) && room())) return false;
   // The scalars come before the table, which takes what is left of the budget
   // up to a quarter more than it needs.
   if (!queue_reserve(ctx, scalar_bytes, p.budget)) return false;
-  // (A large chain's boundary is sized for its largest row.)
-  if (!ensure_front(ctx, p, f, most, ctx.table.ptr ? 0 : table_bytes, most <= kQueueTerms)) return false;
-  return p.budget.holds(ctx.pool_bytes - ctx.table.bytes + table_bytes) &&
-         try_reserve(ctx, ctx.table, table_bytes, p.budget, what);
+  if (ctx.table.bytes < table_bytes || !fits(std::max(ctx.front[0].bytes, grown), table)) buf_release(ctx, ctx.table);
+  // (A large chain's boundary is sized for its largest row, and one that leaves
+  // the scratch no room when it grows ahead for what it needs.)
+  const bool ahead = most <= kQueueTerms && fits(ctx.front[0].bytes + 3 * grown, table_bytes);
+  return ensure_front(ctx, p, f, most, 0, ahead) && try_reserve(ctx, ctx.table, table_bytes, p.budget, what);
 }
 
 // Planned candidates per partition of a queued step. A partition that overflows
@@ -1794,7 +1806,9 @@ static bool run_chunk_grouped(Ctx& ctx, const Plan& p, const HostChunk& hc, std:
   const u64 cap = std::max<u64>(group_capacity(p.group_states, ctx.sms), hc.count);
   if (cap > 0xfffffff0ull) return false;
   const GroupDirs d = group_dirs(n, row0, std::max<u64>(cap, ctx.grp_side[0].bytes / kGroupEntryBytes), sd.units.size());
-  if (2 * cap * kGroupEntryBytes + d.bytes > p.budget) return false;
+  size_t others = ctx.pool_bytes - ctx.front[0].bytes - ctx.table.bytes;  // what stays beside the two sides
+  for (const DevBuf* b : {&ctx.grp_side[0], &ctx.grp_side[1], &ctx.grp_dir}) others -= b->bytes;
+  if (2 * cap * kGroupEntryBytes + d.bytes + others > p.budget) return false;
   if (ctx.pool_bytes > p.budget) {
     buf_release(ctx, ctx.table);
     buf_release(ctx, ctx.front[0]);

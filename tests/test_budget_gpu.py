@@ -107,3 +107,16 @@ def test_kept_buffers_take_nothing_from_a_budget(qp, prep, n, opts, budgets):
             assert c.contract_rows(n, device_budget_bytes=budget, **opts).count == qp.known_count(n)
         finally:
             c.close()
+
+
+# A boundary kept from a smaller board, which the budget does not hold beside a
+# larger one: the chains of a board in slices find room or leave the rows'
+# buffers alone (freed and reserved again for every row, they took twice the
+# time).
+@pytest.mark.parametrize("budget", [119383412, 130862880])
+def test_chains_under_a_kept_boundary(fresh, qp, budget):
+    fresh.count(13, [1], device_budget_bytes=budget)
+    g = fresh.contract_rows(15, device_budget_bytes=budget)
+    assert g.count == qp.known_count(15) and g.device["batches"] > 1
+    assert g.device["row_forms"] & qp.ROWS_CHAIN
+    assert _held(g) <= budget
