@@ -835,8 +835,8 @@ static StepStatus merge_step(Ctx& ctx, const Plan& p, DevFrontier& f, bool site,
     if (ctx.pool_bytes - ctx.table.bytes + table_bytes > p.budget) buf_release(ctx, ctx.table);
     // (A boundary that grew beyond its need, for rows to come, gives way.)
     const char* what = partition ? "partition regions" : "hash table";
-    if (!try_reserve(ctx, ctx.table, table_bytes, p.budget, what) &&
-        !(f.cap > need_cap && shrink_front(ctx, p, f, need_cap) && try_reserve(ctx, ctx.table, table_bytes, p.budget, what))) {
+    const auto scratch = [&] { return try_reserve(ctx, ctx.table, table_bytes, p.budget, what); };
+    if (!scratch() && !(f.cap > need_cap && shrink_front(ctx, p, f, need_cap) && scratch())) {
       if (n_in <= 1) fail(QPEPS_ERR_CAPACITY, row_msg("device budget exceeded at row", row + 1));
       return StepStatus::NeedSplit;
     }
@@ -1211,7 +1211,8 @@ static bool chain_buffers(Ctx& ctx, const Plan& p, DevFrontier& f, u64 most, siz
   const size_t scalar_bytes = (steps + 1) * sizeof(StepScalars), eb = entry_bytes(p);
   if (!p.budget.known() && f.cap >= most && ctx.table.bytes >= table_bytes && ctx.queue.bytes >= scalar_bytes) return true;
   const auto others = [&] {
-    return ctx.pool_bytes - ctx.front[0].bytes - ctx.table.bytes - ctx.queue.bytes + std::max(ctx.queue.bytes, scalar_bytes);
+    const size_t scalars = std::max(ctx.queue.bytes, scalar_bytes);
+    return ctx.pool_bytes - ctx.front[0].bytes - ctx.table.bytes - ctx.queue.bytes + scalars;
   };
   const size_t table = std::max(table_bytes, ctx.table.bytes);
   const size_t grown = f.cap < most ? most * eb : 0;  // a new boundary, beside the old one while that is copied

@@ -95,7 +95,8 @@ def test_kept_buffers_beyond_the_budget_go(fresh, qp, call):
     lambda c: c.contract_rows(12, tail_row=9), lambda c: c.contract_rows(15),
 ], ids=["chain", "sites", "explicit", "tail", "grouped"])
 @pytest.mark.parametrize("n,opts,budgets", [
-    (11, {"granularity": 1, "symmetry": 0}, range(409600, 1740800, 56789)), (10, {"granularity": 1}, range(204800, 921600, 40961)),
+    (11, {"granularity": 1, "symmetry": 0}, range(409600, 1740800, 56789)),
+    (10, {"granularity": 1}, range(204800, 921600, 40961)),
     (12, {}, range(307200, 2560000, 98765)), (11, {"merge": 1}, range(307200, 2560000, 98765)),
     (11, {"key_bits": 128}, range(307200, 2560000, 98765)),
 ])
